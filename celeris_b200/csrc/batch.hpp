@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "celeris_internal.hpp"
@@ -24,8 +25,9 @@ namespace cel {
 constexpr size_t COLS_STATIC_SMEM = 16384;
 
 // ---- one lane (fused.cu) ----------------------------------------------------------------------
+// batch_sizes: (nx, ny) of every member of the batch, whichever lane holds it
 cel_lane* lane_create(int n, const cel_params* const* params, const float* const* bathy, const int* bnx,
-                      const int* bny, int form, std::string& err);
+                      const int* bny, int form, const std::vector<std::pair<int, int>>& batch_sizes, std::string& err);
 void lane_destroy(cel_lane* b);
 int lane_set_stream(cel_lane* b, cudaStream_t s, std::string& err);
 cudaStream_t lane_stream(const cel_lane* b);

@@ -106,6 +106,7 @@ struct PassArgs {
     int stats;          // accumulate GetStats of the input state (first pass of a physical step)
     int friction;       // some member has a nonzero friction coefficient
     double* late_flag;  // set when a bounded TMA wait gave up
+    double* spart;      // STATS_N totals of each strip of the stencil (statistics pass)
 };
 
 __device__ __forceinline__ void two_sum_add(float& hi, float& lo, float d) {
@@ -687,7 +688,7 @@ __global__ void __launch_bounds__(MW, MARCH_MIN_CTAS) k_march(const MemberDev* _
                 }
             }
         }
-        // ---- strip statistics -> member accumulators (statistics pass only) ----
+        // ---- strip statistics (statistics pass only) ----
         if (stats) {
             double sv[STATS_N];
             for (int k = 0; k < 5; ++k) sv[k] = acc[k].value();
@@ -711,8 +712,7 @@ __global__ void __launch_bounds__(MW, MARCH_MIN_CTAS) k_march(const MemberDev* _
             if (tid < STATS_N - 1) {
                 double a = red[0][tid];
                 for (int w = 1; w < MW / 32; ++w) a = (tid >= 6) ? fmax(a, red[w][tid]) : a + red[w][tid];
-                if (tid < 6) { if (a != 0.0) atomicAdd(M.stats + tid, a); }
-                else atomic_max_nonneg(M.stats + tid, a);
+                pa.spart[size_t(it) * STATS_N + tid] = a;   // k_advance_time adds the strips up
             }
         }
     }
@@ -1312,8 +1312,7 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
             if (tid < STATS_N - 1) {
                 double a = red[0][tid];
                 for (int w = 1; w < TW / 32; ++w) a = (tid >= 6) ? fmax(a, red[w][tid]) : a + red[w][tid];
-                if (tid < 6) { if (a != 0.0) atomicAdd(M.stats + tid, a); }
-                else atomic_max_nonneg(M.stats + tid, a);
+                pa.spart[size_t(it) * STATS_N + tid] = a;   // k_advance_time adds the strips up
             }
         }
     }
@@ -2621,8 +2620,6 @@ __global__ void k_choose_dt(DtCtl* __restrict__ ctl, float* __restrict__ dt_tabl
     dt_table[i] = C.dt;
 }
 
-// End of a physical step: advance the clocks by the dt of the step's last pass and, in adaptive
-// batches, shift the controller's dt queue (engine.cpp:1507-1518).
 // The band-major copy of a member's y factors for band width cw (k_cols reads it).
 __global__ void k_band_major(const MemberDev* __restrict__ mems, int mi, int cw) {
     const MemberDev& M = mems[mi];
@@ -2641,10 +2638,31 @@ __global__ void k_rcp_selftest(const float* __restrict__ x, float* __restrict__ 
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = rcp_newton(x[i]);
 }
 
-__global__ void k_advance_time(const MemberDev* __restrict__ mems, DtCtl* __restrict__ ctl, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// End of a physical step: advance the clocks by the dt of the step's last pass and, in adaptive
+// batches, shift the controller's dt queue (engine.cpp:1507-1518).
+// One warp per member: the totals of the step's first pass from its strips' partials, added in the
+// order of the strips, so that they depend neither on scheduling nor on the lanes of the batch; then
+// the clock.
+__global__ void k_advance_time(const MemberDev* __restrict__ mems, DtCtl* __restrict__ ctl, int n,
+                               const int2* __restrict__ strips, const double* __restrict__ spart) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= n) return;
     const MemberDev& M = mems[i];
+    const int2 r = strips[i];   // first strip, number of strips
+    double v[STATS_N - 1];
+    for (int k = 0; k < STATS_N - 1; ++k) v[k] = 0.0;
+    for (int t = lane; t < r.y; t += 32)
+        for (int k = 0; k < STATS_N - 1; ++k) {
+            const double a = spart[size_t(r.x + t) * STATS_N + k];
+            v[k] = (k >= 6) ? fmax(v[k], a) : v[k] + a;
+        }
+    for (int off = 16; off; off >>= 1)
+        for (int k = 0; k < STATS_N - 1; ++k) {
+            const double o = __shfl_down_sync(0xffffffffu, v[k], off);
+            v[k] = (k >= 6) ? fmax(v[k], o) : v[k] + o;
+        }
+    if (lane != 0) return;
+    for (int k = 0; k < STATS_N - 1; ++k) M.stats[k] = v[k];
     *M.time64 += double(*M.dtp);
     *M.time32 += *M.dtp;
     if (ctl) {
@@ -2694,6 +2712,8 @@ struct cel_lane {
     cel::Idx ix;
     int4* tiles = nullptr; int ntiles = 0;      // 32x16 tiles (statistics on demand)
     int4* mtiles = nullptr; int nmtiles = 0;    // marching strips of the fused stencil
+    int2* mrange = nullptr;                     // each member's strips: first, number
+    double* spart = nullptr;                    // their statistics
     int2* rows = nullptr; int nrows = 0;
     int2* bands = nullptr; int nbands = 0;
     int2* bitems[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -2732,8 +2752,10 @@ struct cel_lane {
     int col_cl = 0;                     // cluster column solver: CTAs per cluster (0: not in use)
     bool col_tt = false;                // tile-transposed column solver (band width 16, "1 chunk")
     int mh = cel::MH_DEFAULT;           // stencil strip height (rows per CTA work item)
-    int rows_per_step = 1;              // stencil rows per thread step: 1 (k_march) or 2 (k_march2)
-    int mw = 128;                       // stencil CTA width in threads (k_march2: 128 or 96)
+    int rows_per_step = 2;              // stencil rows per thread step: 1 (k_march) or 2 (k_march2)
+    int mw = 96;                        // stencil CTA width in threads (k_march2: 128 or 96)
+    bool rows_chosen = false;           // the caller selected the stencil variant (lane_set_stencil_rows)
+    std::vector<std::pair<int, int>> batch_sizes;   // (nx, ny) of every member of the batch, all lanes
     int max_nx = 0, max_ny = 0;
     bool any_log = false;               // some member has <logData> doLog set
     const float* elapsed_src = nullptr; // engine handles: the elapsed time of their latest resetTimestep
@@ -2857,8 +2879,6 @@ int launch_pass(cel_lane* b, const PassArgs& pa, std::string& err) {
     // the launch checks below read the runtime's last-error state: drop what calls outside this pass
     // left there (they reported it, or ignored it, where they happened)
     (void)cudaGetLastError();
-    const size_t nm = b->mem.size();
-    if (pa.stats) B_TRY(cudaMemsetAsync(b->stats_all, 0, nm * STATS_N * sizeof(double), b->stream));
     {
         TimedLaunch t(&b->tm, b->stream, "fused_stencil");
         const bool ad = pa.scheme == CEL_SCHEME_PREDICTOR_ADAPTIVE;
@@ -3005,6 +3025,7 @@ int run_pass(cel_lane* b, bool first_of_step, std::string& err) {
     pa.stats = first_of_step ? 1 : 0;
     pa.friction = b->any_friction ? 1 : 0;
     pa.late_flag = b->late_flag;
+    pa.spart = b->spart;
     if (int e = launch_pass(b, pa, err)) return e;
     if (first_of_step) {
         b->step_stats_valid = true;
@@ -3015,7 +3036,8 @@ int run_pass(cel_lane* b, bool first_of_step, std::string& err) {
     if (book) {
         const int o = ix.og, oo = ix.oog, sc = ix.scr;
         ix.og = sc; ix.oog = o; ix.scr = oo;
-        k_advance_time<<<(int(b->mem.size()) + 127) / 128, 128, 0, b->stream>>>(b->ddev, b->ctl, int(b->mem.size()));
+        k_advance_time<<<(int(b->mem.size()) + 3) / 4, 128, 0, b->stream>>>(b->ddev, b->ctl, int(b->mem.size()), b->mrange,
+                                                                            b->spart);
         B_TRY(cudaGetLastError());
     } else if (was_pred) {
         ix.pred = ix.scr;
@@ -3109,6 +3131,41 @@ cudaError_t allow_max_dynamic_smem(const void* kernel) {
     return e;
 }
 
+// The strip height of a batch's stencil: at most mh_max rows, fewer where taller strips would leave
+// SMs idle.  A strip is a serial chain of row steps, so a batch with fewer strips than CTA slots takes
+// as long as one strip, and one with a few strips more than a whole number of waves takes a wave
+// more.  The cost of a height h is modelled as
+//   sum over waves of (row steps of a strip + PRO) x step(CTAs per SM in that wave),
+// where a step takes STEP_US alone on its SM (latency) and n x RATE_US with n CTAs beside it
+// (issue), and PRO steps stand for the prologue (filling the ring, the first faces).  Measured with
+// the paired-row stencil at 96 threads: 2.06 us a step on an idle GPU (512 x 64 cells, heights 8 to
+// 64) and 4.2 us at four CTAs an SM (16 M cells); the one-row stencil 1.5 and 3.6 (at five).
+// Against 64-row strips, ms per step: 512 x 64 cells 0.185 -> 0.068 (8 rows), 1024 x 1024 0.261 ->
+// 0.181 (24), 40 members of 128..512 a side 0.553 -> 0.522 (48); 16 M cells keep 64 rows (1.497;
+// 32 rows 1.515).  Heights change the split of the work, never a cell's arithmetic; every lane of a
+// batch takes the height of the whole batch, so the statistics do not depend on the lanes either.
+int strip_height(const cel_lane* b, int mo, int rps, int mw, int mh_max) {
+    constexpr int H_MIN = 8;
+    constexpr double PRO = 2.5;
+    const int slots = rps == 1 ? MARCH_MIN_CTAS : march2_min_ctas(mw);
+    const double step_us = rps == 1 ? 1.5 : 2.1;
+    const double rate_us = (rps == 1 ? 3.6 : 4.2) / slots;
+    auto step = [&](double n) { return std::max(step_us, n * rate_us); };
+    const double sms = b->sms;
+    int best = mh_max;
+    double best_t = 1e300;
+    for (int h = std::min(H_MIN, mh_max);; h = std::min(h + 2, mh_max)) {
+        long long strips = 0;
+        for (const auto& m : b->batch_sizes) strips += (long long)((m.first + mo - 1) / mo) * ((m.second + h - 1) / h);
+        const double per_sm = std::ceil(strips / sms);
+        const double whole = std::floor(per_sm / slots), rest = per_sm - whole * slots;
+        const double t = ((h + rps - 1) / rps + PRO) * (whole * step(slots) + (rest > 0 ? step(rest) : 0.0));
+        if (t <= best_t) { best_t = t; best = h; }   // the taller of two equals: fewer prologues
+        if (h == mh_max) break;
+    }
+    return best;
+}
+
 int configure_work(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::string& err) {
     // 32-column bands with 32, 64 or 128 chunks per column (nt = chunks x 32 = 1024, 2048, 4096):
     // the cluster solver, 8 chunks per CTA and nt / 256 CTAs per cluster
@@ -3154,11 +3211,16 @@ int configure_work(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::st
                              : (cw == 1 || cl > 0) ? 0 : sizeof(float) * size_t(b->max_ny) * cw;
     if (smem_cols + COLS_STATIC_SMEM > 227 * 1024) { err = "column band too wide for the tallest member (shared memory)"; return CEL_ERR_ARG; }
     std::vector<int4> mt;
-    std::vector<int2> bd;
+    std::vector<int2> bd, mr;
+    const int sh = strip_height(b, mo, rps, mw, mh);
     for (int i = 0; i < int(b->mem.size()); ++i) {
         const HostSetup& hs = b->mem[i].hs;
-        for (int y0 = 2; y0 < hs.ny + 2; y0 += mh)
-            for (int x0 = 2; x0 < hs.nx + 2; x0 += mo) mt.push_back(make_int4(i, x0, y0, mh));
+        // a member's strips as equal as whole steps allow
+        const int nb = (hs.ny + sh - 1) / sh, hm = std::min(sh, ((hs.ny + nb - 1) / nb + rps - 1) / rps * rps);
+        const int first = int(mt.size());
+        for (int y0 = 2; y0 < hs.ny + 2; y0 += hm)
+            for (int x0 = 2; x0 < hs.nx + 2; x0 += mo) mt.push_back(make_int4(i, x0, y0, hm));
+        mr.push_back(make_int2(first, int(mt.size()) - first));
         if (cw == 1) {
             // one entry per column; columns 0, 1 and past nx+1 are padding (-1) so that each warp
             // covers 32 columns starting on a 128-byte boundary
@@ -3172,20 +3234,28 @@ int configure_work(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::st
     free_graphs(b);
     B_TRY(cudaStreamSynchronize(b->stream));
     B_TRY(cudaStreamSynchronize(b->side));
-    for (void* p : {static_cast<void*>(b->mtiles), static_cast<void*>(b->bands)})
+    for (void* p : {static_cast<void*>(b->mtiles), static_cast<void*>(b->bands), static_cast<void*>(b->mrange),
+                    static_cast<void*>(b->spart)})
         if (p) { cudaFree(p); b->allocs.erase(std::remove(b->allocs.begin(), b->allocs.end(), p), b->allocs.end()); }
     b->mtiles = nullptr;
     b->bands = nullptr;
+    b->mrange = nullptr;
+    b->spart = nullptr;
     void* p = nullptr;
     if (dalloc(b, &p, mt.size() * sizeof(int4), err)) return CEL_ERR_CUDA;
     b->mtiles = static_cast<int4*>(p);
     if (dalloc(b, &p, bd.size() * sizeof(int2), err)) return CEL_ERR_CUDA;
     b->bands = static_cast<int2*>(p);
+    if (dalloc(b, &p, mr.size() * sizeof(int2), err)) return CEL_ERR_CUDA;
+    b->mrange = static_cast<int2*>(p);
+    if (dalloc(b, &p, mt.size() * STATS_N * sizeof(double), err)) return CEL_ERR_CUDA;
+    b->spart = static_cast<double*>(p);
     // the allocations' zeroing ran on the legacy stream: finish it before the batch stream writes
     B_TRY(cudaDeviceSynchronize());
     // on the batch stream (non-blocking: it would not wait for legacy-stream copies)
     B_TRY(cudaMemcpyAsync(b->mtiles, mt.data(), mt.size() * sizeof(int4), cudaMemcpyHostToDevice, b->stream));
     B_TRY(cudaMemcpyAsync(b->bands, bd.data(), bd.size() * sizeof(int2), cudaMemcpyHostToDevice, b->stream));
+    B_TRY(cudaMemcpyAsync(b->mrange, mr.data(), mr.size() * sizeof(int2), cudaMemcpyHostToDevice, b->stream));
     B_TRY(cudaStreamSynchronize(b->stream));
     b->nmtiles = int(mt.size());
     b->nbands = int(bd.size());
@@ -3241,8 +3311,9 @@ int configure_work(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::st
 }
 
 cel_lane* lane_create(int n, const cel_params* const* params, const float* const* bathy, const int* bnx,
-                        const int* bny, int form, std::string& err) {
+                        const int* bny, int form, const std::vector<std::pair<int, int>>& batch_sizes, std::string& err) {
     std::unique_ptr<cel_lane> b(new cel_lane());
+    b->batch_sizes = batch_sizes;
     b->form = form;
     b->mixed = (form == CEL_FORM_MIXED);
     const int N0 = params[0]->correction_steps;
@@ -3512,7 +3583,7 @@ cel_lane* lane_create(int n, const cel_params* const* params, const float* const
     }
     {   // column bands of 16 columns (8 for tall domains: shared-memory capacity), strips of 64 rows
         const int cw = (size_t(max_ny) * 16 * sizeof(float) + COLS_STATIC_SMEM <= 227 * 1024) ? 16 : 8;
-        if (configure_work(b.get(), cw, MH_DEFAULT, 1, MW, NTC_DEFAULT, err)) return nullptr;
+        if (configure_work(b.get(), cw, MH_DEFAULT, b->rows_per_step, b->mw, NTC_DEFAULT, err)) return nullptr;
     }
     b->sch.reset(*params[0]);
     cudaMemcpy(b->dt_table, b->dt_host, sizeof(float) * n, cudaMemcpyHostToDevice);
@@ -3861,11 +3932,14 @@ int lane_get_tuning(const cel_lane* b, int* tx, int* ty, int* rps) {
 int lane_col_chunks(const cel_lane* b) { return b->cw > 1 ? b->cnt / b->cw : 1; }
 
 int lane_set_stencil_rows(cel_lane* b, int rps, std::string& err) {
-    return configure_work(b, b->cw, b->mh, rps, rps == 2 ? b->mw : MW, b->cnt, err);
+    // two rows per step start from 128-thread strips until a width is chosen (lane_set_stencil_width)
+    if (int e = configure_work(b, b->cw, b->mh, rps, rps == 2 && b->rows_chosen ? b->mw : MW, b->cnt, err)) return e;
+    b->rows_chosen = true;
+    return CEL_OK;
 }
 
 int lane_set_stencil_width(cel_lane* b, int threads, std::string& err) {
-    if (b->rows_per_step != 2 && threads != MW) {
+    if ((b->rows_per_step != 2 || !b->rows_chosen) && threads != MW) {
         err = "the one-row stencil runs 128-thread strips; select two rows per step first";
         return CEL_ERR_ARG;
     }
@@ -3878,7 +3952,9 @@ cudaStream_t lane_stream(const cel_lane* b) { return b->stream; }
 int lane_members(const cel_lane* b) { return int(b->mem.size()); }
 int lane_max_ny(const cel_lane* b) { return b->max_ny; }
 int lane_configure(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::string& err) {
-    return configure_work(b, cw, mh, rps, mw, nt, err);
+    if (int e = configure_work(b, cw, mh, rps, mw, nt, err)) return e;
+    b->rows_chosen = true;
+    return CEL_OK;
 }
 int lane_col_threads(const cel_lane* b) { return b->cnt; }
 
@@ -3911,7 +3987,7 @@ public:
             if (int st = read_cbf(p.bathymetry_path, &tmp, bnx, bny, err)) return st;
             bz = tmp.data();
         }
-        b = lane_create(1, &pp, &bz, &bnx, &bny, form, err);
+        b = lane_create(1, &pp, &bz, &bnx, &bny, form, {{p.nx, p.ny}}, err);
         if (b) b->elapsed_src = &log_elapsed;
         return b ? CEL_OK : CEL_ERR_ARG;
     }

@@ -113,6 +113,8 @@ cel_batch* batch_create(int n, const cel_params* const* params, const float* con
     L = std::min(L, n);
     auto g = std::make_unique<cel_batch>();
     // largest members first, each onto the lane with the fewest cells so far
+    std::vector<std::pair<int, int>> sizes(n);
+    for (int i = 0; i < n; ++i) sizes[i] = {params[i]->nx, params[i]->ny};
     std::vector<long long> cells(n);
     for (int i = 0; i < n; ++i) cells[i] = (long long)params[i]->nx * params[i]->ny;
     std::vector<int> order(n);
@@ -141,7 +143,7 @@ cel_batch* batch_create(int n, const cel_params* const* params, const float* con
             bx.push_back(bnx[ms[k]]);
             by.push_back(bny[ms[k]]);
         }
-        cel_lane* ln = lane_create(int(ms.size()), p.data(), z.data(), bx.data(), by.data(), form, err);
+        cel_lane* ln = lane_create(int(ms.size()), p.data(), z.data(), bx.data(), by.data(), form, sizes, err);
         if (!ln) return nullptr;   // the lanes made so far go with g
         g->lanes.push_back(ln);
     }

@@ -275,7 +275,8 @@ int cel_batch_launches_per_step(const cel_batch* b);
 /* ---- tuning and measurement ------------------------------------------------------------- */
 /* Fused forms.  tile_x: column-solver band width (8, 16 or 32 columns per CTA, chunked scans; or 1:
  * one thread per column, serial sweeps, forward values kept in the right-hand-side plane); tile_y: stencil
- * strip height (rows a CTA marches, 8..1024); 0 keeps the current value.  pcr_switch: chunks per
+ * strip height (the most rows a CTA marches, 8..1024; strips are split shorter where the batch has too few
+ * of them to fill the GPU); 0 keeps the current value.  pcr_switch: chunks per
  * column of the column solver, i.e. where it switches from the parallel stage to serial sweeps.  The
  * solves factor each system once (M = LU, engine.cpp:2612-2887 coefficients); the L and U sweeps of
  * a column are split into that many chunks, each swept serially by one thread (Thomas), and the
@@ -292,7 +293,7 @@ int cel_batch_get_tuning(const cel_batch* b, int* tile_x, int* tile_y, int* rows
 /* The column solver's chunks per column (the pcr_switch above; 1 with tile_x = 1: one thread per column). */
 int cel_batch_col_chunks(const cel_batch* b);
 /* Stencil variant: 1 = one row per thread step; 2 = two rows per step as pairs, with the paired
- * single-precision instructions of sm_100 (f32x2). */
+ * single-precision instructions of sm_100 (f32x2).  Until it is selected, two rows at 96 threads. */
 int cel_batch_set_stencil_rows(cel_batch* b, int rows_per_step);
 /* Threads per stencil CTA, i.e. strip width + 2 halo columns: 128 or 96 (96 with two rows per step
  * only).  Narrower strips waste fewer lanes on members whose width is not a multiple of 126. */
