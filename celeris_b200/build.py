@@ -31,7 +31,7 @@ UNITS = [
     ("plain.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
     ("fused.cu", ["-prec-div=false", "-prec-sqrt=false", "-ftz=true"]),
 ]
-HEADERS = ["celeris_internal.hpp", "engine_iface.hpp", "scheme.hpp", "device_math.cuh", "batch.hpp"]
+HEADERS = ["celeris_internal.hpp", "engine_iface.hpp", "scheme.hpp", "device_math.cuh", "batch.hpp", "boundary_plan.hpp"]
 
 
 def nvcc() -> str:

@@ -15,6 +15,7 @@
 #include <string>
 #include <vector>
 
+#include "boundary_plan.hpp"
 #include "device_math.cuh"
 #include "engine_iface.hpp"
 #include "scheme.hpp"
@@ -64,47 +65,34 @@ __global__ void k_pass1(const float4* __restrict__ st, const float4* __restrict_
     aux2[i] = make_float4(mid, 0.f, msd, bw);
 }
 
-// ---- Pass2 (compute.hlsl:470-542): KP fluxes at east / north faces; region [1,nx+2)x[1,ny+2) --
-__global__ void k_pass2(const float4* __restrict__ H, const float4* __restrict__ U, const float4* __restrict__ V,
-                        const float4* __restrict__ aux2, float4* __restrict__ XF, float4* __restrict__ YF,
-                        float4* __restrict__ aux1, SimConsts c, float dt) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    if (x >= c.nx + 2 || y >= c.ny + 2) return;
-    const int NX = c.NX;
-    const size_t i = size_t(y) * NX + x;
-    const float4 hc = H[i], uc = U[i], vc = V[i];
-    const float hN = hc.x, hE = hc.y, uN = uc.x, uE = uc.y, vN = vc.x, vE = vc.y;
-    const float hWe = H[i + 1].w, hSn = H[i + NX].z;
-    const float uWe = U[i + 1].w, uSn = U[i + NX].z;
-    const float vWe = V[i + 1].w, vSn = V[i + NX].z;
-    const float g = c.g, hg = c.half_g;
-    const float cN = sqrtf(g * hN), cE = sqrtf(g * hE), cW = sqrtf(g * hWe), cS = sqrtf(g * hSn);
+// ---- Pass2 (compute.hlsl:470-542): KP flux between the cell on a face's low side (m) and the one on
+// its high side (p); x: the east face of m, y: its north face ----
+__device__ __forceinline__ float3 x_flux(float hE, float uE, float vE, float hWe, float uWe, float vWe, float g, float hg) {
+    const float cE = sqrtf(g * hE), cW = sqrtf(g * hWe);
     const float ap = fmaxf(fmaxf(uE + cE, uWe + cW), 0.f);
     const float am = fminf(fminf(uE - cE, uWe - cW), 0.f);
+    return make_float3(numflux(ap, am, hWe * uWe, hE * uE, hWe - hE),
+                       numflux(ap, am, hWe * (uWe * uWe + hg * hWe), hE * (uE * uE + hg * hE), hWe * uWe - hE * uE),
+                       numflux(ap, am, hWe * uWe * vWe, hE * uE * vE, hWe * vWe - hE * vE));
+}
+__device__ __forceinline__ float3 y_flux(float hN, float uN, float vN, float hSn, float uSn, float vSn, float g, float hg) {
+    const float cN = sqrtf(g * hN), cS = sqrtf(g * hSn);
     const float bp = fmaxf(fmaxf(vN + cN, vSn + cS), 0.f);
     const float bm = fminf(fminf(vN - cN, vSn - cS), 0.f);
-    float4 xf, yf;
-    xf.x = numflux(ap, am, hWe * uWe, hE * uE, hWe - hE);
-    xf.y = numflux(ap, am, hWe * (uWe * uWe + hg * hWe), hE * (uE * uE + hg * hE), hWe * uWe - hE * uE);
-    xf.z = numflux(ap, am, hWe * uWe * vWe, hE * uE * vE, hWe * vWe - hE * vE);
-    xf.w = 0.f;
-    yf.x = numflux(bp, bm, hSn * vSn, hN * vN, hSn - hN);
-    yf.y = numflux(bp, bm, hSn * uSn * vSn, hN * uN * vN, hSn * uSn - hN * uN);
-    yf.z = numflux(bp, bm, hSn * (vSn * vSn + hg * hSn), hN * (vN * vN + hg * hN), hSn * vSn - hN * vN);
-    yf.w = 0.f;
-    XF[i] = xf; YF[i] = yf;
-    const float4 a2 = aux2[i];
-    aux1[i] = make_float4(a2.x, 0.f, a2.z, a2.w * t_pow(fabsf(c.whitewater_decay_rate), dt));
+    return make_float3(numflux(bp, bm, hSn * vSn, hN * vN, hSn - hN),
+                       numflux(bp, bm, hSn * uSn * vSn, hN * uN * vN, hSn * uSn - hN * uN),
+                       numflux(bp, bm, hSn * (vSn * vSn + hg * hSn), hN * (vN * vN + hg * hN), hSn * vSn - hN * vN));
 }
 
 struct Pass3Args {
-    const float4* st; const float4* bot; const float4* XF; const float4* YF;
+    const float4* st; const float4* bot; const float4* H; const float4* U; const float4* V;
+    const float4* aux2; float4* aux1;
     const float4* ABCx; const float4* ABCy;
     const float4* og; const float4* oog; const float4* ofg; const float4* oofg;
     const float4* cur; const float4* pred; const float4* fgpred;
     float4* out; float4* sgrad; float4* sfg;
     float dt, dt_old, dt_old_old;
+    float decay;   // pow(|white-water decay rate|, dt)
     int scheme;
 };
 
@@ -124,13 +112,35 @@ __device__ __forceinline__ void second_order(float yn, float y1, float y2, float
     o[2] = r * yn + g * y1 + bb * y2;
 }
 
-// ---- Pass3Predictor (compute.hlsl:616-812): RHS, time scheme; interior [2,nx+2)x[2,ny+2) -----
-__global__ void k_pass3(Pass3Args a, SimConsts c) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x + 2;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y + 2;
-    if (x >= c.nx + 2 || y >= c.ny + 2) return;
+// ---- Pass2 and Pass3Predictor (compute.hlsl:470-542, 616-812) in one kernel, every texel of the new
+// state written once: zero on the ghost frame (engine.cpp:1007), the right-hand sides inside.  A cell
+// takes the fluxes of its four faces from the stored face states (each flux is computed by the two
+// cells that share the face, from the same values), so the flux textures, their clears and their
+// round trip through memory are gone.  It is bound by the flux arithmetic (IEEE divisions and square
+// roots) once the textures are in L2: 12.5 us on 512 x 64 cells and 76 us on 1001 x 777 by event timing,
+// where Pass2 and Pass3 took 8.5 + 8.6 and 24 + 51 us beside three clears.  The white-water decay of Pass2
+// runs on its own region [1,nx+2)x[1,ny+2). ----
+__global__ void k_pass23(Pass3Args a, SimConsts c) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    const int y = blockIdx.y * blockDim.y + threadIdx.y;
+    if (x >= c.NX || y >= c.NY) return;
     const int NX = c.NX;
     const size_t i = size_t(y) * NX + x;
+    if (x >= 1 && y >= 1 && x < c.nx + 2 && y < c.ny + 2) {
+        const float4 a2 = a.aux2[i];
+        a.aux1[i] = make_float4(a2.x, 0.f, a2.z, a2.w * a.decay);
+    }
+    if (x < 2 || y < 2 || x >= c.nx + 2 || y >= c.ny + 2) {
+        a.out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        return;
+    }
+    const float4 hc = a.H[i], uc = a.U[i], vc = a.V[i];
+    const float4 hw = a.H[i - 1], uw = a.U[i - 1], vw = a.V[i - 1], he = a.H[i + 1], ue = a.U[i + 1], ve = a.V[i + 1];
+    const float4 hs = a.H[i - NX], us = a.U[i - NX], vs = a.V[i - NX], hn = a.H[i + NX], un = a.U[i + NX], vn = a.V[i + NX];
+    const float3 xh = x_flux(hc.y, uc.y, vc.y, he.w, ue.w, ve.w, c.g, c.half_g);
+    const float3 xw = x_flux(hw.y, uw.y, vw.y, hc.w, uc.w, vc.w, c.g, c.half_g);
+    const float3 yh = y_flux(hc.x, uc.x, vc.x, hn.z, un.z, vn.z, c.g, c.half_g);
+    const float3 ys = y_flux(hs.x, us.x, vs.x, hc.z, uc.z, vc.z, c.g, c.half_g);
     const float4* st = a.st;
     const float4* bot = a.bot;
     const float BYh = bot[i].x, BXh = bot[i].y, BAh = bot[i].z;
@@ -150,7 +160,6 @@ __global__ void k_pass3(Pass3Args a, SimConsts c) {
     const float edd = st[i - 2 * NX].x - sl, euu = st[i + 2 * NX].x - sl;
     const float eul = st[i + NX - 1].x - sl, eur = st[i + NX + 1].x - sl;
     const float edl = st[i - NX - 1].x - sl, edr = st[i - NX + 1].x - sl;
-    const float4 xh = a.XF[i], xw = a.XF[i - 1], yh = a.YF[i], ys = a.YF[i - NX];
     const float odx = c.one_over_dx, ody = c.one_over_dy;
     const float od2x = odx * odx, od3x = od2x * odx, od2y = ody * ody, od3y = od2y * ody;
     const float ddx = (-drr + 8 * dr - 8 * dl + dll) * odx / 12.0f;
@@ -213,80 +222,143 @@ __global__ void k_pass3(Pass3Args a, SimConsts c) {
     a.sfg[i] = make_float4(Fs, Gs, 0.f, 0.f);
 }
 
-// ---- Cyclic reduction, one level per launch (compute.hlsl:835-947) ------------------------
-// D arrays: element (x, y) at base[y*pitch + x*stride] (the level-0 RHS is a channel of the
-// float4 state; reduced levels are plain float planes).
-__global__ void k_cr_reduce_x(const float* __restrict__ Dp, int dps, int dpp, const float4* __restrict__ Ap, int app,
-                              float* __restrict__ Dk, int dkp, int len_k, int ny) {
-    const int x2 = blockIdx.x * blockDim.x + threadIdx.x + 2;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y + 2;
-    if (x2 >= len_k + 2 || y >= ny + 2) return;
-    const int x1 = (x2 - 2) * 2 + 3;
-    const float* row = Dp + size_t(y) * dpp;
-    const float4* ar = Ap + size_t(y) * app;
-    const float k1 = ar[x1].x / ar[x1 - 1].y, k2 = ar[x1].z / ar[x1 + 1].y;
-    Dk[size_t(y) * dkp + x2] = row[x1 * dps] - row[(x1 - 1) * dps] * k1 - row[(x1 + 1) * dps] * k2;
-}
+// ---- Cyclic reduction (compute.hlsl:835-947), every level of a system in one CTA -----------
+// The levels of one direction, level k's elements i = 0 .. len_k - 1 (texel i + 2):
+//   reduce      D_k[i] = D_{k-1}[2i+1] - D_{k-1}[2i] k1 - D_{k-1}[2i+2] k2
+//   substitute  X_k[2j] = (D_k[2j] - a X_{k+1}[j-1] - c X_{k+1}[j]) / b,  X_k[2j+1] = X_{k+1}[j]
+// with zeros where an index leaves the level.  k1 and k2 are the shader's quotients of coefficient
+// texels: they depend on the bottom only, so the host forms them once (the same IEEE divisions); the
+// division by b stays a division.  Operation by operation this is the shader's arithmetic, so the
+// results do not change a bit.
+//
+// A draw per level, the shader's way, costs 2 log2(n) launches a direction, most of which touch a
+// few elements.  Here a CTA keeps a system's levels in shared memory: CTAs [0, ny) take one row each,
+// the others CR_COLS adjacent columns (whose level 0 they read from the state when they need it instead
+// of keeping it).  What bounds it is latency, since the levels are a serial chain: the coefficients of
+// a level are loaded before the barrier that ends the level before it, and levels of at most 32
+// elements run in one warp.  hu and hv go back into the state in place (CopyFromXxAndXy,
+// compute.hlsl:814-823, is folded in).  Measured by event timing, a pass's solves: 512 x 64 cells 32
+// launches and 210 us -> 14.7 us, 1001 x 777 cells 38 launches and 295 us -> 53 us.
+constexpr int CR_MAX_LEVELS = 16;
+constexpr int CR_THREADS = 256;
+constexpr int CR_COLS = 4;              // columns of a column CTA: 64-byte pieces of a state row
+constexpr size_t CR_SMEM_MAX = 200 * 1024;
+struct CrLevels {
+    int K;                              // levels
+    int tail;                           // first level (>= 1) that one warp handles
+    int len[CR_MAX_LEVELS];
+    int off[CR_MAX_LEVELS];             // start of a level's values in a system's scratch
+    size_t koff[CR_MAX_LEVELS];         // start of a level's {k1, k2} (levels >= 1)
+    size_t soff[CR_MAX_LEVELS];         // start of a level's {a, c, b}, even elements only
+    int total;                          // scratch values of a system
+    const float2* k12;                  // rows: [y][i], columns: [i][x]
+    const float4* acb;
+};
+struct SolveArgs {
+    float4* st;
+    CrLevels x, y;
+    float* scratch;                     // the levels in global memory where shared memory does not hold them
+};
 
-__global__ void k_cr_subst_x(const float* __restrict__ Dk, int dks, int dkp, const float4* __restrict__ Ak, int akp,
-                             const float* __restrict__ Xn, int xnp, float* __restrict__ Xk, int xkp, int len_k, int ny) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x + 2;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y + 2;
-    if (x >= len_k + 2 || y >= ny + 2) return;
-    float o;
-    const float* xn = Xn ? Xn + size_t(y) * xnp : nullptr;
-    if (x % 2 == 1) {
-        o = xn ? xn[x / 2 + 1] : 0.f;
-    } else {
-        const float4 a = Ak[size_t(y) * akp + x];
-        const float x1 = xn ? xn[x / 2] : 0.f, x2 = xn ? xn[x / 2 + 1] : 0.f;
-        o = (Dk[size_t(y) * dkp + size_t(x) * dks] - a.x * x1 - a.z * x2) / a.y;
+// ROW: one row (level 0 kept with the levels); else CR_COLS columns.  lv: the levels, element i of
+// column c of level k at lv[(off_k + i) * W + c]; st0: the level-0 values in the state, d0 floats apart;
+// sys: the row, or this thread's column; ns: the number of columns (the columns' coefficient stride).
+template <bool ROW>
+__device__ __forceinline__ void cr_solve(const CrLevels& L, float* __restrict__ lv, float* st0, size_t d0, int sys, int ns,
+                                         bool live) {
+    constexpr int W = ROW ? 1 : CR_COLS, T = CR_THREADS / W;
+    const int c = int(threadIdx.x) % W, t = int(threadIdx.x) / W;
+    const int n = L.len[0];
+    lv += c;
+    auto k12 = [&](int k, int i) -> float2 {
+        if (!live || i >= L.len[k]) return make_float2(0.f, 0.f);
+        return __ldg(L.k12 + L.koff[k] + (ROW ? size_t(sys) * L.len[k] + i : size_t(i) * ns + sys));
+    };
+    auto acb = [&](int k, int j) -> float4 {
+        const int half = (L.len[k] + 1) / 2;
+        if (!live || j >= half) return make_float4(0.f, 0.f, 1.f, 0.f);
+        return __ldg(L.acb + L.soff[k] + (ROW ? size_t(sys) * half + j : size_t(j) * ns + sys));
+    };
+    auto d0_at = [&](int i) -> float {
+        if (ROW) return lv[L.off[0] + i];
+        return (live && i < n) ? st0[size_t(i) * d0] : 0.f;
+    };
+    auto reduce = [&](int k, int i, float2 q) {
+        const float* p = lv + size_t(L.off[k - 1]) * W;
+        const float mid = k == 1 ? d0_at(2 * i + 1) : p[(2 * i + 1) * W];
+        const float lo = k == 1 ? d0_at(2 * i) : p[(2 * i) * W];
+        const float hi = k == 1 ? d0_at(2 * i + 2) : p[(2 * i + 2) * W];
+        lv[size_t(L.off[k] + i) * W] = mid - lo * q.x - hi * q.y;
+    };
+    auto substitute = [&](int k, int j, float4 q) {
+        const bool last = k + 1 == L.K;
+        const float* xn = last ? nullptr : lv + size_t(L.off[k + 1]) * W;
+        const float x1 = (!last && j > 0) ? xn[(j - 1) * W] : 0.f;
+        const float x2 = (!last && j < L.len[k + 1]) ? xn[j * W] : 0.f;
+        const float d = k == 0 ? d0_at(2 * j) : lv[size_t(L.off[k] + 2 * j) * W];
+        const float o = (d - q.x * x1 - q.y * x2) / q.z;
+        if (k == 0) {
+            if (live) {
+                st0[size_t(2 * j) * d0] = o;
+                if (2 * j + 1 < n) st0[size_t(2 * j + 1) * d0] = x2;
+            }
+        } else {
+            lv[size_t(L.off[k] + 2 * j) * W] = o;
+            if (2 * j + 1 < L.len[k]) lv[size_t(L.off[k] + 2 * j + 1) * W] = x2;
+        }
+    };
+    float2 q = L.K > 1 ? k12(1, t) : make_float2(0.f, 0.f);
+    if (ROW) {
+        for (int i = t; i < n; i += T) lv[L.off[0] + i] = st0[size_t(i) * d0];
+        if (t == 0) lv[L.off[0] + n] = 0.f;
+        __syncthreads();
     }
-    Xk[size_t(y) * xkp + x] = o;
-}
-
-__global__ void k_cr_reduce_y(const float* __restrict__ Dp, int dps, int dpp, const float4* __restrict__ Ap, int NX,
-                              float* __restrict__ Dk, int len_k, int nx) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x + 2;
-    const int y2 = blockIdx.y * blockDim.y + threadIdx.y + 2;
-    if (x >= nx + 2 || y2 >= len_k + 2) return;
-    const int y1 = (y2 - 2) * 2 + 3;
-    const float4 a0 = Ap[size_t(y1) * NX + x];
-    const float k1 = a0.x / Ap[size_t(y1 - 1) * NX + x].y, k2 = a0.z / Ap[size_t(y1 + 1) * NX + x].y;
-    const float dIn = Dp[size_t(y1) * dpp + size_t(x) * dps];
-    const float dL = Dp[size_t(y1 - 1) * dpp + size_t(x) * dps];
-    const float dR = Dp[size_t(y1 + 1) * dpp + size_t(x) * dps];
-    Dk[size_t(y2) * NX + x] = dIn - dL * k1 - dR * k2;
-}
-
-__global__ void k_cr_subst_y(const float* __restrict__ Dk, int dks, int dkp, const float4* __restrict__ Ak, int NX,
-                             const float* __restrict__ Xn, float* __restrict__ Xk, int len_k, int nx) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x + 2;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y + 2;
-    if (x >= nx + 2 || y >= len_k + 2) return;
-    float o;
-    if (y % 2 == 1) {
-        o = Xn ? Xn[size_t(y / 2 + 1) * NX + x] : 0.f;
-    } else {
-        const float4 a = Ak[size_t(y) * NX + x];
-        const float x1 = Xn ? Xn[size_t(y / 2) * NX + x] : 0.f, x2 = Xn ? Xn[size_t(y / 2 + 1) * NX + x] : 0.f;
-        o = (Dk[size_t(y) * dkp + size_t(x) * dks] - a.x * x1 - a.z * x2) / a.y;
+    for (int k = 1; k < L.tail; ++k) {
+        for (int i = t; i < L.len[k]; i += T) reduce(k, i, i == t ? q : k12(k, i));
+        if (t == 0) lv[size_t(L.off[k] + L.len[k]) * W] = 0.f;
+        if (k + 1 < L.K) q = k12(k + 1, t);
+        __syncthreads();
     }
-    Xk[size_t(y) * NX + x] = o;
+    float4 s = make_float4(0.f, 0.f, 1.f, 0.f);
+    if (threadIdx.x < 32) {   // levels of at most 32 elements, all columns together
+        for (int k = L.tail; k < L.K; ++k) {
+            if (t < L.len[k]) reduce(k, t, q);
+            if (t == 0) lv[size_t(L.off[k] + L.len[k]) * W] = 0.f;
+            if (k + 1 < L.K) q = k12(k + 1, t);
+            __syncwarp();
+        }
+        for (int k = L.K - 1; k >= L.tail; --k) {
+            s = acb(k, t);
+            if (2 * t < L.len[k]) substitute(k, t, s);
+            __syncwarp();
+        }
+    }
+    s = acb(L.tail - 1, t);
+    __syncthreads();
+    for (int k = L.tail - 1; k >= 0; --k) {
+        for (int j = t; 2 * j < L.len[k]; j += T) substitute(k, j, j == t ? s : acb(k, j));
+        if (k > 0) {
+            s = acb(k - 1, t);
+            __syncthreads();
+        }
+    }
 }
 
-// CopyFromXxAndXy (compute.hlsl:814-823) over the interior
-__global__ void k_copy_from(float4* __restrict__ st, const float* __restrict__ Xx, const float* __restrict__ Xy,
-                            SimConsts c) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x + 2;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y + 2;
-    if (x >= c.nx + 2 || y >= c.ny + 2) return;
-    const size_t i = size_t(y) * c.NX + x;
-    float4 s = st[i];
-    s.y = Xx[i];
-    s.z = Xy[i];
-    s.w = 0.f;
-    st[i] = s;
+// SMEM_X / SMEM_Y: the rows' / the columns' levels fit in shared memory.
+template <bool SMEM_X, bool SMEM_Y>
+__global__ void __launch_bounds__(CR_THREADS) k_cr(SolveArgs a, SimConsts c) {
+    extern __shared__ float cr_sm[];
+    const int rows = c.ny, b = blockIdx.x;
+    if (b < rows) {
+        float* lv = SMEM_X ? cr_sm : a.scratch + size_t(b) * a.x.total;
+        cr_solve<true>(a.x, lv, reinterpret_cast<float*>(a.st + size_t(b + 2) * c.NX + 2) + 1, 4, b, 0, true);
+    } else {
+        const int band = b - rows, col = band * CR_COLS + int(threadIdx.x) % CR_COLS;
+        float* lv = SMEM_Y ? cr_sm
+                           : a.scratch + (SMEM_X ? 0 : size_t(rows) * a.x.total) + size_t(band) * a.y.total * CR_COLS;
+        cr_solve<false>(a.y, lv, reinterpret_cast<float*>(a.st + size_t(2) * c.NX + 2 + col) + 2, size_t(4) * c.NX, col, c.nx,
+                        col < c.nx);
+    }
 }
 
 // ---- Boundaries (compute.hlsl:985-1309) --------------------------------------------------
@@ -340,12 +412,9 @@ __device__ float3 irregular_sum(const BArgs& b, float xx, float yy, float dh, fl
     return stk[0];
 }
 
-__global__ void k_boundary(const float4* __restrict__ st, const float4* __restrict__ bot, float4* __restrict__ strip,
-                           BArgs b, SimConsts c) {
-    const int sx = blockIdx.x * blockDim.x + threadIdx.x;
-    const int sy = blockIdx.y * blockDim.y + threadIdx.y;
-    if (sx >= b.sw || sy >= b.sh) return;
-    const int x = b.x0 + sx, y = b.y0 + sy;
+// The value one side's shader writes at texel (x, y)
+__device__ float4 boundary_value(const float4* st, const float4* __restrict__ bot, const BArgs& b, const SimConsts& c, int x,
+                                 int y) {
     const int NX = c.NX, NY = c.NY;
     const size_t i = size_t(y) * NX + x;
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -391,7 +460,15 @@ __global__ void k_boundary(const float4* __restrict__ st, const float4* __restri
             o.x = r.x; o.y = r.y; o.z = r.z;
         }
     }
-    strip[size_t(sy) * b.sw + sx] = o;
+    return o;
+}
+
+__global__ void k_boundary(const float4* __restrict__ st, const float4* __restrict__ bot, float4* __restrict__ strip,
+                           BArgs b, SimConsts c) {
+    const int sx = blockIdx.x * blockDim.x + threadIdx.x;
+    const int sy = blockIdx.y * blockDim.y + threadIdx.y;
+    if (sx >= b.sw || sy >= b.sh) return;
+    strip[size_t(sy) * b.sw + sx] = boundary_value(st, bot, b, c, b.x0 + sx, b.y0 + sy);
 }
 
 __global__ void k_strip_copy(float4* __restrict__ st, const float4* __restrict__ strip, int x0, int y0, int sw, int sh,
@@ -402,80 +479,120 @@ __global__ void k_strip_copy(float4* __restrict__ st, const float4* __restrict__
     st[size_t(y0 + sy) * NX + x0 + sx] = strip[size_t(sy) * sw + sx];
 }
 
-// ---- GetStats (compute.hlsl:1319-1378) per 4x4 block, then an FP64 reduction -------------
-__global__ void k_getstats(const float4* __restrict__ st, const float4* __restrict__ bot, float* __restrict__ blocks,
-                           SimConsts c) {
-    const int bx = blockIdx.x * blockDim.x + threadIdx.x;
-    const int by = blockIdx.y * blockDim.y + threadIdx.y;
-    const int nbx = c.nx / 4, nby = c.ny / 4;
-    if (bx >= nbx || by >= nby) return;
-    float sh = 0, sb = 0, shu = 0, shv = 0, sk = 0, mu = 0, mh = 0, mc = 0, mf = 0;
-    for (int j = 2; j < 6; ++j)
-        for (int ii = 2; ii < 6; ++ii) {
-            const size_t i = size_t(by * 4 + j) * c.NX + bx * 4 + ii;
-            const float4 s = st[i];
-            const float B = bot[i].z;
-            const float h = fmaxf(0.f, s.x - B);
-            const float cc = sqrtf(c.g * h);
-            const float q = div_by_h(h, c.epsilon);
-            const float u = q * s.y, v = q * s.z;
-            sh += h; sb += h * (B + 0.5f * h); shu += s.y; shv += s.z;
-            sk += (s.y * u + s.z * v);
-            const float u2v2 = u * u + v * v;
-            mu = fmaxf(mu, u2v2); mh = fmaxf(mh, h);
-            mc = fmaxf(mc, (fabsf(u) + cc) * c.one_over_dx);
-            mc = fmaxf(mc, (fabsf(v) + cc) * c.one_over_dy);
-            mf = fmaxf(mf, u2v2 * q);
+// All four sides in one launch (boundary_plan.hpp): a work item is 256 texels of a segment, written in
+// place by one thread each, or a whole corner, whose two sides one CTA takes in drawing order.  The
+// sides' own launches, each followed by a copy out of the strip texture, are 8 launches of a few
+// hundred texels each; domains that the plan refuses still take them.
+struct BoundaryArgs {
+    BArgs side[4];
+    Rect region[BND_REGIONS];
+};
+__global__ void __launch_bounds__(256) k_boundary_all(float4* st, const float4* __restrict__ bot, const int2* __restrict__ items,
+                                                      BoundaryArgs a, SimConsts c) {
+    const int2 it = items[blockIdx.x];
+    const Rect r = a.region[it.x];
+    if (it.x < 4) {
+        const int w = r.x1 - r.x0, k = it.y + int(threadIdx.x);
+        if (k >= w * (r.y1 - r.y0)) return;
+        const int x = r.x0 + k % w, y = r.y0 + k / w;
+        st[size_t(y) * c.NX + x] = boundary_value(st, bot, a.side[it.x], c, x, y);
+        return;
+    }
+    for (int q = 0; q < 2; ++q) {
+        const BArgs& b = a.side[corner_side(it.x - 4, q)];
+        const int x0 = max(r.x0, b.x0), x1 = min(r.x1, b.x0 + b.sw), y0 = max(r.y0, b.y0), y1 = min(r.y1, b.y0 + b.sh);
+        const int w = x1 - x0, n = w > 0 ? w * (y1 - y0) : 0;
+        for (int k = threadIdx.x; k < n; k += blockDim.x) {
+            const int x = x0 + k % w, y = y0 + k / w;
+            st[size_t(y) * c.NX + x] = boundary_value(st, bot, b, c, x, y);
         }
-    float* o = blocks + (size_t(by) * nbx + bx) * 9;
-    o[0] = sh; o[1] = sb; o[2] = shu; o[3] = shv; o[4] = sk; o[5] = mu; o[6] = mh; o[7] = mc; o[8] = mf;
+        __syncthreads();
+    }
 }
 
-// One CTA: FP64 sums / maxima of the block partials, plus the FP64 sum of h over every interior
-// cell (out[9]).  out[10] = 1 if any state value is non-finite (health flag).
-__global__ void k_reduce_stats(const float* __restrict__ blocks, int nb, const float4* __restrict__ st,
-                               const float4* __restrict__ bot, SimConsts c, double* __restrict__ out) {
-    __shared__ double sm[10][32];
-    __shared__ int bad_s;
-    double v[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    int bad = 0;
-    for (int k = threadIdx.x; k < nb; k += blockDim.x) {
-        const float* b = blocks + size_t(k) * 9;
-        for (int q = 0; q < 5; ++q) v[q] += double(b[q]);
-        for (int q = 5; q < 9; ++q) v[q] = fmax(v[q], double(b[q]));
-    }
-    const int n = c.nx * c.ny;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const int x = k % c.nx + 2, y = k / c.nx + 2;
-        const size_t i = size_t(y) * c.NX + x;
-        const float4 s = st[i];
-        if (!isfinite(s.x) || !isfinite(s.y) || !isfinite(s.z)) bad = 1;
-        v[9] += fmax(0.0, double(s.x) - double(bot[i].z));
-    }
-    if (threadIdx.x == 0) bad_s = 0;
-    __syncthreads();
-    if (bad) bad_s = 1;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int q = 0; q < 10; ++q) {
-        double x = v[q];
-        for (int off = 16; off; off >>= 1) {
-            const double y = __shfl_down_sync(0xffffffffu, x, off);
-            x = (q >= 5 && q < 9) ? fmax(x, y) : x + y;
+// ---- GetStats (compute.hlsl:1319-1378) and its FP64 reduction in one launch -------------
+// One thread per 4x4 block (the texture's partial sums, kept for getWaterHeight) with the FP64 volume
+// and the non-finite flag of its cells; blocks cut off by the far edges count for those two only.  Each
+// CTA leaves one set of FP64 partials, and the last one to finish adds them up in CTA order, so the
+// totals do not depend on scheduling.  (The reduction by one CTA over every cell took 313 us on
+// 1001 x 777 cells, one SM of 148 reading everything.)
+// out: [0..4] sums, [5..8] maxima, [9] the volume, [10] 1 if a state value is not finite
+constexpr int STATS_THREADS = 64;
+__global__ void __launch_bounds__(STATS_THREADS) k_stats(const float4* __restrict__ st, const float4* __restrict__ bot,
+                                                         float* __restrict__ blocks, SimConsts c, double* __restrict__ part,
+                                                         unsigned int* __restrict__ done, double* __restrict__ out) {
+    __shared__ double sm[STATS_THREADS / 32][11];
+    __shared__ bool last;
+    const int nbx = c.nx / 4, nby = c.ny / 4, tbx = (c.nx + 3) / 4, tby = (c.ny + 3) / 4;
+    const int k = blockIdx.x * STATS_THREADS + threadIdx.x;
+    double v[11] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (k < tbx * tby) {
+        const int bx = k % tbx, by = k / tbx;
+        const bool whole = bx < nbx && by < nby;
+        const int jn = min(4, c.ny - 4 * by), in = min(4, c.nx - 4 * bx);
+        float sh = 0, sb = 0, shu = 0, shv = 0, sk = 0, mu = 0, mh = 0, mc = 0, mf = 0;
+        for (int j = 0; j < jn; ++j)
+            for (int ii = 0; ii < in; ++ii) {
+                const size_t i = size_t(by * 4 + j + 2) * c.NX + bx * 4 + ii + 2;
+                const float4 s = st[i];
+                const float B = bot[i].z;
+                if (!isfinite(s.x) || !isfinite(s.y) || !isfinite(s.z)) v[10] = 1.0;
+                v[9] += fmax(0.0, double(s.x) - double(B));
+                const float h = fmaxf(0.f, s.x - B);
+                const float cc = sqrtf(c.g * h);
+                const float q = div_by_h(h, c.epsilon);
+                const float u = q * s.y, w = q * s.z;
+                sh += h; sb += h * (B + 0.5f * h); shu += s.y; shv += s.z;
+                sk += (s.y * u + s.z * w);
+                const float u2v2 = u * u + w * w;
+                mu = fmaxf(mu, u2v2); mh = fmaxf(mh, h);
+                mc = fmaxf(mc, (fabsf(u) + cc) * c.one_over_dx);
+                mc = fmaxf(mc, (fabsf(w) + cc) * c.one_over_dy);
+                mf = fmaxf(mf, u2v2 * q);
+            }
+        if (whole) {
+            float* o = blocks + (size_t(by) * nbx + bx) * 9;
+            o[0] = sh; o[1] = sb; o[2] = shu; o[3] = shv; o[4] = sk; o[5] = mu; o[6] = mh; o[7] = mc; o[8] = mf;
+            v[0] = sh; v[1] = sb; v[2] = shu; v[3] = shv; v[4] = sk;
+            v[5] = mu; v[6] = mh; v[7] = mc; v[8] = mf;
         }
-        if (lane == 0) sm[q][wid] = x;
     }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const int nw = blockDim.x >> 5;
-        for (int q = 0; q < 10; ++q) {
-            double x = lane < nw ? sm[q][lane] : 0.0;
+    auto is_max = [](int q) { return (q >= 5 && q < 9) || q == 10; };
+    auto cta_reduce = [&]() {   // thread 0 ends with the CTA's totals
+        for (int q = 0; q < 11; ++q) {
+            double x = v[q];
             for (int off = 16; off; off >>= 1) {
                 const double y = __shfl_down_sync(0xffffffffu, x, off);
-                x = (q >= 5 && q < 9) ? fmax(x, y) : x + y;
+                x = is_max(q) ? fmax(x, y) : x + y;
             }
-            if (lane == 0) out[q] = x;
+            if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5][q] = x;
         }
-        if (lane == 0) out[10] = bad_s ? 1.0 : 0.0;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int q = 0; q < 11; ++q) {
+                v[q] = sm[0][q];
+                for (int w = 1; w < STATS_THREADS / 32; ++w) v[q] = is_max(q) ? fmax(v[q], sm[w][q]) : v[q] + sm[w][q];
+            }
+    };
+    cta_reduce();
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < 11; ++q) part[size_t(blockIdx.x) * 11 + q] = v[q];
+        __threadfence();
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int q = 0; q < 11; ++q) v[q] = 0.0;
+    for (int b = threadIdx.x; b < int(gridDim.x); b += STATS_THREADS)
+        for (int q = 0; q < 11; ++q) {
+            const double y = __ldcg(part + size_t(b) * 11 + q);
+            v[q] = is_max(q) ? fmax(v[q], y) : v[q] + y;
+        }
+    cta_reduce();
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < 11; ++q) out[q] = v[q];
+        *done = 0u;
     }
 }
 
@@ -507,17 +624,31 @@ public:
     KernelTimer tm;
     size_t ntex = 0;
     // device textures
-    float4 *st[2] = {nullptr, nullptr}, *H = nullptr, *U = nullptr, *V = nullptr, *XF = nullptr, *YF = nullptr;
-    float4 *AUX1 = nullptr, *AUX2 = nullptr, *CUR = nullptr, *PRED = nullptr, *FGPRED = nullptr, *BOT = nullptr;
-    float4 *GRAD[3] = {nullptr, nullptr, nullptr}, *FG[3] = {nullptr, nullptr, nullptr}, *STRIP = nullptr;
+    // The state rotates through three textures and the derivatives through four, by index: a corrector
+    // finds the state that it corrects and the predictor's derivatives where their passes left them
+    // (the reference copies them aside, engine.cpp:1050-1058: 48 bytes a cell and predictor).
+    float4 *st[3] = {nullptr, nullptr, nullptr}, *H = nullptr, *U = nullptr, *V = nullptr;
+    float4 *AUX1 = nullptr, *AUX2 = nullptr, *BOT = nullptr;
+    float4 *GRAD[4] = {nullptr, nullptr, nullptr, nullptr}, *FG[4] = {nullptr, nullptr, nullptr, nullptr}, *STRIP = nullptr;
     float4* WAVES = nullptr;
-    std::vector<float4*> ABCx, ABCy;
-    std::vector<float*> Dx, Xx, Dy, Xy;
+    float4 *ABCx = nullptr, *ABCy = nullptr;                        // level-0 systems (the right-hand sides' products)
+    float2 *K12x = nullptr, *K12y = nullptr;                        // reduction multipliers of every level
+    float4 *ACBx = nullptr, *ACBy = nullptr;                        // substitution coefficients of every level
+    SolveArgs solve{};
+    bool smem_x = true, smem_y = true;
+    size_t smem_cr = 0;
+    bool planned = false;                                           // the four sides run as one launch
+    Rect regions[BND_REGIONS] = {};
+    int2* bitems = nullptr;
+    int nbitems = 0;
     float* blocks = nullptr;
     double* dstats = nullptr;
+    double* spart = nullptr;
+    unsigned int* sdone = nullptr;
+    int stats_ctas = 1;
     std::vector<void*> allocs;
     int wave_off[4] = {0, 0, 0, 0};
-    int sim_idx = 0, old_i = 0, oldold_i = 1, scratch_i = 2;
+    int sim_idx = 0, cur_i = 0, old_i = 0, oldold_i = 1, scratch_i = 2, spare_i = 3, pred_i = 3;
     int uts_iter[4] = {1, 1, 1, 1};
     bool bootstrap_needed = true;
     std::vector<float> terrain;   // bathymetry grid given by set_bathymetry (used by remesh)
@@ -557,28 +688,13 @@ public:
         own_stream = true;
         c = make_consts(p, hs, hs.NX);
         ntex = size_t(hs.NX) * hs.NY;
-        for (float4** t : {&st[0], &st[1], &H, &U, &V, &XF, &YF, &AUX1, &AUX2, &CUR, &PRED, &FGPRED, &BOT, &STRIP})
+        for (float4** t : {&st[0], &st[1], &st[2], &H, &U, &V, &AUX1, &AUX2, &BOT, &STRIP, &ABCx, &ABCy})
             if (int e = dalloc(*t, ntex)) return e;
-        for (int k = 0; k < 3; ++k) {
+        for (int k = 0; k < 4; ++k) {
             if (int e = dalloc(GRAD[k], ntex)) return e;
             if (int e = dalloc(FG[k], ntex)) return e;
         }
-        ABCx.assign(hs.Kx, nullptr); Dx.assign(hs.Kx, nullptr); Xx.assign(hs.Kx, nullptr);
-        ABCy.assign(hs.Ky, nullptr); Dy.assign(hs.Ky, nullptr); Xy.assign(hs.Ky, nullptr);
-        for (int k = 0; k < hs.Kx; ++k) {
-            const size_t n = size_t(hs.lenx[k] + 4) * hs.NY;
-            if (int e = dalloc(ABCx[k], n)) return e;
-            if (int e = dalloc(Dx[k], n)) return e;
-            if (int e = dalloc(Xx[k], k == 0 ? ntex : n)) return e;
-            CEL_CUDA_TRY(cudaMemcpy(ABCx[k], hs.ABCx[k].data(), n * sizeof(float4), cudaMemcpyHostToDevice));
-        }
-        for (int k = 0; k < hs.Ky; ++k) {
-            const size_t n = size_t(hs.NX) * (hs.leny[k] + 4);
-            if (int e = dalloc(ABCy[k], n)) return e;
-            if (int e = dalloc(Dy[k], n)) return e;
-            if (int e = dalloc(Xy[k], k == 0 ? ntex : n)) return e;
-            CEL_CUDA_TRY(cudaMemcpy(ABCy[k], hs.ABCy[k].data(), n * sizeof(float4), cudaMemcpyHostToDevice));
-        }
+        if (int e = init_solve()) return e;
         {
             std::vector<float4> b(ntex);
             for (size_t i = 0; i < ntex; ++i) b[i] = make_float4(hs.BY[i], hs.BX[i], hs.BA[i], 0.f);
@@ -609,10 +725,128 @@ public:
         const int nb = std::max(1, (hs.nx / 4) * (hs.ny / 4));
         if (int e = dalloc(blocks, size_t(nb) * 9)) return e;
         if (int e = dalloc(dstats, 16)) return e;
+        stats_ctas = (((hs.nx + 3) / 4) * ((hs.ny + 3) / 4) + STATS_THREADS - 1) / STATS_THREADS;
+        if (int e = dalloc(spart, size_t(stats_ctas) * 11)) return e;
+        if (int e = dalloc(sdone, 1)) return e;
+        if (int e = init_boundary()) return e;
         // the set-up copies and memsets above ran on the legacy stream, which the engine's
         // non-blocking stream does not wait for: finish them
         CEL_CUDA_TRY(cudaDeviceSynchronize());
         return remesh();
+    }
+
+    // Work items of the one-launch boundary, where the domain's sides allow it.
+    int init_boundary() {
+        const cel_boundary* sides[4] = {&p.north, &p.east, &p.south, &p.west};
+        int type[4], width[4];
+        for (int s = 0; s < 4; ++s) { type[s] = sides[s]->type; width[s] = sides[s]->width; }
+        planned = plan_boundary(hs.nx, hs.ny, type, width, regions);
+        if (!planned) return CEL_OK;
+        std::vector<int2> items;
+        for (int k = 4; k < BND_REGIONS; ++k)
+            if (regions[k].x1 > regions[k].x0 && regions[k].y1 > regions[k].y0) items.push_back(make_int2(k, 0));
+        for (int k = 0; k < 4; ++k) {
+            const int n = std::max(0, regions[k].x1 - regions[k].x0) * std::max(0, regions[k].y1 - regions[k].y0);
+            for (int t = 0; t < n; t += 256) items.push_back(make_int2(k, t));
+        }
+        nbitems = int(items.size());
+        if (int e = dalloc(bitems, std::max<size_t>(items.size(), 1))) return e;
+        if (nbitems) CEL_CUDA_TRY(cudaMemcpy(bitems, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice));
+        return CEL_OK;
+    }
+
+    // Level tables of the cyclic reduction and, once, the room for them.
+    int init_solve() {
+        auto levels = [](const std::vector<int>& len, bool rows, int systems) {
+            CrLevels L{};
+            L.K = int(len.size());
+            L.tail = L.K;
+            size_t ko = 0, so = 0;
+            for (int k = 0; k < L.K; ++k) {
+                L.len[k] = len[k];
+                L.off[k] = L.total;
+                if (k > 0 || rows) L.total += len[k] + 1;   // one zero past a level's end
+                L.koff[k] = ko;
+                L.soff[k] = so;
+                if (k > 0) ko += size_t(len[k]) * systems;
+                so += size_t((len[k] + 1) / 2) * systems;
+                if (k > 0 && L.tail == L.K && len[k] * (rows ? 1 : CR_COLS) <= 32) L.tail = k;
+            }
+            return std::make_pair(L, std::make_pair(ko, so));
+        };
+        const auto lx = levels(hs.lenx, true, hs.ny), ly = levels(hs.leny, false, hs.nx);
+        solve.x = lx.first;
+        solve.y = ly.first;
+        if (int e = dalloc(K12x, lx.second.first)) return e;
+        if (int e = dalloc(ACBx, lx.second.second)) return e;
+        if (int e = dalloc(K12y, ly.second.first)) return e;
+        if (int e = dalloc(ACBy, ly.second.second)) return e;
+        solve.x.k12 = K12x; solve.x.acb = ACBx;
+        solve.y.k12 = K12y; solve.y.acb = ACBy;
+        const size_t bx = sizeof(float) * size_t(solve.x.total), by = sizeof(float) * size_t(solve.y.total) * CR_COLS;
+        smem_x = bx <= CR_SMEM_MAX;
+        smem_y = by <= CR_SMEM_MAX;
+        smem_cr = std::max(smem_x ? bx : 0, smem_y ? by : 0);
+        const size_t scratch = (smem_x ? 0 : size_t(hs.ny) * solve.x.total) +
+                               (smem_y ? 0 : size_t((hs.nx + CR_COLS - 1) / CR_COLS) * CR_COLS * solve.y.total);
+        if (scratch)
+            if (int e = dalloc(solve.scratch, scratch)) return e;
+        // the limit is the function's, not this engine's: set once to the most any engine asks for
+        for (auto* k : {k_cr<true, true>, k_cr<true, false>, k_cr<false, true>, k_cr<false, false>})
+            CEL_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(CR_SMEM_MAX)));
+        // the allocations' clears ran on the legacy stream, which the engine's stream does not wait for
+        CEL_CUDA_TRY(cudaDeviceSynchronize());
+        return upload_solve();
+    }
+
+    // The solve's coefficients from the host's levels, on the engine's stream.
+    int upload_solve() {
+        // texel (i + 2) of system s (from 0) of a level
+        auto pack = [](const std::vector<std::vector<Float4>>& abc, const CrLevels& L, bool rows, int n, int NX,
+                       std::vector<float2>& k12, std::vector<float4>& acb) {
+            for (int k = 0; k < L.K; ++k) {
+                const size_t ss = rows ? size_t(L.len[k] + 4) : 1, si = rows ? 1 : size_t(NX);
+                const size_t ps = k > 0 && rows ? size_t(L.len[k - 1] + 4) : 1;
+                const int half = (L.len[k] + 1) / 2;
+                auto equation = [&](int s, int i, size_t to) {
+                    const Float4* p = &abc[k - 1][size_t(s + 2) * ps + size_t(2 * i + 2) * si];
+                    k12[L.koff[k] + to] = make_float2(p[si].x / p[0].y, p[si].z / p[2 * si].y);
+                };
+                auto even = [&](int s, int j, size_t to) {
+                    const Float4& q = abc[k][size_t(s + 2) * ss + size_t(2 * j + 2) * si];
+                    acb[L.soff[k] + to] = make_float4(q.x, q.z, q.y, 0.f);
+                };
+                if (rows) {
+                    for (int s = 0; s < n; ++s) {
+                        for (int i = 0; k > 0 && i < L.len[k]; ++i) equation(s, i, size_t(s) * L.len[k] + i);
+                        for (int j = 0; j < half; ++j) even(s, j, size_t(s) * half + j);
+                    }
+                } else {
+                    for (int i = 0; k > 0 && i < L.len[k]; ++i)
+                        for (int s = 0; s < n; ++s) equation(s, i, size_t(i) * n + s);
+                    for (int j = 0; j < half; ++j)
+                        for (int s = 0; s < n; ++s) even(s, j, size_t(j) * n + s);
+                }
+            }
+        };
+        for (const bool rows : {true, false}) {
+            const CrLevels& L = rows ? solve.x : solve.y;
+            const int n = rows ? hs.ny : hs.nx;
+            size_t equations = 0, evens = 0;
+            for (int k = 0; k < L.K; ++k) {
+                if (k > 0) equations += size_t(L.len[k]) * n;
+                evens += size_t((L.len[k] + 1) / 2) * n;
+            }
+            std::vector<float2> k12(equations);
+            std::vector<float4> acb(evens);
+            const auto& abc = rows ? hs.ABCx : hs.ABCy;
+            pack(abc, L, rows, n, hs.NX, k12, acb);
+            CEL_CUDA_TRY(cudaMemcpyAsync(rows ? ABCx : ABCy, abc[0].data(), ntex * sizeof(float4), cudaMemcpyHostToDevice, stream));
+            CEL_CUDA_TRY(cudaMemcpyAsync(rows ? K12x : K12y, k12.data(), k12.size() * sizeof(float2), cudaMemcpyHostToDevice, stream));
+            CEL_CUDA_TRY(cudaMemcpyAsync(rows ? ACBx : ACBy, acb.data(), acb.size() * sizeof(float4), cudaMemcpyHostToDevice, stream));
+            CEL_CUDA_TRY(cudaStreamSynchronize(stream));   // before the host copies go out of scope
+        }
+        return CEL_OK;
     }
 
     int remesh() override {
@@ -620,13 +854,8 @@ public:
             HostSetup fresh;
             if (int st0 = make_setup(p, terrain.data(), terrain_nx, terrain_ny, fresh, err)) return st0;
             hs = fresh;
-            // on the engine's stream, finished before the host copies go out of scope
-            for (int k = 0; k < hs.Kx; ++k)
-                CEL_CUDA_TRY(cudaMemcpyAsync(ABCx[k], hs.ABCx[k].data(), size_t(hs.lenx[k] + 4) * hs.NY * sizeof(float4),
-                                             cudaMemcpyHostToDevice, stream));
-            for (int k = 0; k < hs.Ky; ++k)
-                CEL_CUDA_TRY(cudaMemcpyAsync(ABCy[k], hs.ABCy[k].data(), size_t(hs.NX) * (hs.leny[k] + 4) * sizeof(float4),
-                                             cudaMemcpyHostToDevice, stream));
+            if (int st0 = upload_solve()) return st0;
+            // on the engine's stream, finished before the host copy goes out of scope
             std::vector<float4> b(ntex);
             for (size_t i = 0; i < ntex; ++i) b[i] = make_float4(hs.BY[i], hs.BX[i], hs.BA[i], 0.f);
             CEL_CUDA_TRY(cudaMemcpyAsync(BOT, b.data(), ntex * sizeof(float4), cudaMemcpyHostToDevice, stream));
@@ -636,11 +865,11 @@ public:
         for (size_t i = 0; i < ntex; ++i) s[i] = make_float4(hs.ic[3 * i], hs.ic[3 * i + 1], hs.ic[3 * i + 2], 0.f);
         CEL_CUDA_TRY(cudaMemcpyAsync(st[0], s.data(), ntex * sizeof(float4), cudaMemcpyHostToDevice, stream));
         CEL_CUDA_TRY(cudaMemcpyAsync(st[1], s.data(), ntex * sizeof(float4), cudaMemcpyHostToDevice, stream));
-        for (float4* t : {H, U, V, XF, YF, AUX1, AUX2, CUR, PRED, FGPRED, GRAD[0], GRAD[1], GRAD[2], FG[0], FG[1], FG[2]})
+        for (float4* t : {H, U, V, AUX1, AUX2, GRAD[0], GRAD[1], GRAD[2], GRAD[3], FG[0], FG[1], FG[2], FG[3]})
             CEL_CUDA_TRY(cudaMemsetAsync(t, 0, ntex * sizeof(float4), stream));
         CEL_CUDA_TRY(cudaStreamSynchronize(stream));
         sch.reset(p);
-        sim_idx = 0; old_i = 0; oldold_i = 1; scratch_i = 2;
+        sim_idx = 0; cur_i = 0; old_i = 0; oldold_i = 1; scratch_i = 2; spare_i = 3; pred_i = 3;
         for (int& u : uts_iter) u = 1;
         bootstrap_needed = true;
         return CEL_OK;
@@ -661,7 +890,8 @@ public:
         }
     }
 
-    int boundary_side(float4* stt, int side) {
+    // One side's settings at this pass; false if it has no texels.
+    bool boundary_args(int side, BArgs& a) {
         const cel_boundary& b = side == 0 ? p.north : side == 1 ? p.east : side == 2 ? p.south : p.west;
         const int NX = hs.NX, NY = hs.NY;
         int x0, x1, y0, y1;
@@ -670,8 +900,8 @@ public:
         else if (side == 2) { x0 = 0; x1 = NX; y0 = 0; y1 = b.width; }
         else { x0 = 0; x1 = b.width; y0 = 0; y1 = NY; }
         x0 = std::max(x0, 0); y0 = std::max(y0, 0); x1 = std::min(x1, NX); y1 = std::min(y1, NY);
-        if (x1 <= x0 || y1 <= y0) return CEL_OK;
-        BArgs a{};
+        a = BArgs{};
+        if (x1 <= x0 || y1 <= y0) return false;
         a.side = side; a.type = b.type; a.width = b.width;
         a.sea_level = float(b.sea_level); a.amp = float(b.amplitude); a.period = float(b.period);
         a.theta = float(b.theta);
@@ -687,28 +917,37 @@ public:
             a.uts_eta = v[0]; a.uts_hu = v[1]; a.uts_hv = v[2];
         }
         a.x0 = x0; a.y0 = y0; a.sw = x1 - x0; a.sh = y1 - y0;
-        {
+        return true;
+    }
+
+    // boundaries East, North, West, South (engine.cpp:1342-1438)
+    void boundaries(float4* stt) {
+        if (planned) {
+            BoundaryArgs a{};
+            for (int side : {1, 0, 3, 2}) boundary_args(side, a.side[side]);
+            std::copy(regions, regions + BND_REGIONS, a.region);
+            if (nbitems == 0) return;
             TimedLaunch tl(&tm, stream, "plain_boundary");
-            k_boundary<<<grid2(a.sw, a.sh), dim3(BX2, BY2), 0, stream>>>(stt, BOT, STRIP, a, c);
+            k_boundary_all<<<nbitems, 256, 0, stream>>>(stt, BOT, bitems, a, c);
+            return;
         }
-        {
+        for (int side : {1, 0, 3, 2}) {
+            BArgs a;
+            if (!boundary_args(side, a)) continue;
+            {
+                TimedLaunch tl(&tm, stream, "plain_boundary");
+                k_boundary<<<grid2(a.sw, a.sh), dim3(BX2, BY2), 0, stream>>>(stt, BOT, STRIP, a, c);
+            }
             TimedLaunch tl(&tm, stream, "plain_strip_copy");
-            k_strip_copy<<<grid2(a.sw, a.sh), dim3(BX2, BY2), 0, stream>>>(stt, STRIP, x0, y0, a.sw, a.sh, NX);
+            k_strip_copy<<<grid2(a.sw, a.sh), dim3(BX2, BY2), 0, stream>>>(stt, STRIP, a.x0, a.y0, a.sw, a.sh, hs.NX);
         }
-        return CEL_OK;
     }
 
     int run_stats_kernels() {
         (void)cudaGetLastError();
-        const float4* s = st[sim_idx];
-        const int nbx = hs.nx / 4, nby = hs.ny / 4;
-        if (nbx > 0 && nby > 0) {
-            TimedLaunch tl(&tm, stream, "plain_getstats");
-            k_getstats<<<grid2(nbx, nby), dim3(BX2, BY2), 0, stream>>>(s, BOT, blocks, c);
-        }
         {
-            TimedLaunch tl(&tm, stream, "plain_reduce_stats");
-            k_reduce_stats<<<1, 1024, 0, stream>>>(blocks, nbx * nby, s, BOT, c, dstats);
+            TimedLaunch tl(&tm, stream, "plain_stats");
+            k_stats<<<stats_ctas, STATS_THREADS, 0, stream>>>(st[sim_idx], BOT, blocks, c, spart, sdone, dstats);
         }
         CEL_CUDA_TRY(cudaGetLastError());
         return CEL_OK;
@@ -780,74 +1019,42 @@ public:
         (void)cudaGetLastError();   // the launch checks below must see only this pass's launches
         if (!sch.initialized) { if (int e = reset_timestep(0.f, 0.f, nullptr)) return e; }
         const dim3 blk(BX2, BY2);
+        int out_i;
+        if (sch.time_scheme == CEL_SCHEME_CORRECTOR) {
+            out_i = 3 - sim_idx - cur_i;
+        } else {
+            cur_i = sim_idx;
+            out_i = (sim_idx + 1) % 3;
+        }
         float4* old_state = st[sim_idx];
-        float4* new_state = st[1 - sim_idx];
+        float4* new_state = st[out_i];
         if (bootstrap_needed) {
             TimedLaunch tl(&tm, stream, "plain_pass1");
             k_pass1<<<grid2(hs.nx + 2, hs.ny + 2), blk, 0, stream>>>(old_state, BOT, AUX1, H, U, V, AUX2, c);
             bootstrap_needed = false;
         }
-        CEL_CUDA_TRY(cudaMemsetAsync(XF, 0, ntex * sizeof(float4), stream));
-        CEL_CUDA_TRY(cudaMemsetAsync(YF, 0, ntex * sizeof(float4), stream));
-        {
-            TimedLaunch tl(&tm, stream, "plain_pass2");
-            k_pass2<<<grid2(hs.nx + 1, hs.ny + 1), blk, 0, stream>>>(H, U, V, AUX2, XF, YF, AUX1, c, sch.dt);
-        }
-        CEL_CUDA_TRY(cudaMemsetAsync(new_state, 0, ntex * sizeof(float4), stream));
         Pass3Args a{};
-        a.st = old_state; a.bot = BOT; a.XF = XF; a.YF = YF; a.ABCx = ABCx[0]; a.ABCy = ABCy[0];
+        a.st = old_state; a.bot = BOT; a.H = H; a.U = U; a.V = V; a.aux2 = AUX2; a.aux1 = AUX1;
+        a.ABCx = ABCx; a.ABCy = ABCy;
         a.og = GRAD[old_i]; a.oog = GRAD[oldold_i]; a.ofg = FG[old_i]; a.oofg = FG[oldold_i];
-        a.cur = CUR; a.pred = PRED; a.fgpred = FGPRED;
+        a.cur = st[cur_i]; a.pred = GRAD[pred_i]; a.fgpred = FG[pred_i];
         a.out = new_state; a.sgrad = GRAD[scratch_i]; a.sfg = FG[scratch_i];
         a.dt = sch.dt; a.dt_old = sch.dt_old; a.dt_old_old = sch.dt_old_old;
+        a.decay = float(std::pow(double(std::fabs(c.whitewater_decay_rate)), double(sch.dt)));
         a.scheme = sch.time_scheme;
         {
-            TimedLaunch tl(&tm, stream, "plain_pass3");
-            k_pass3<<<grid2(hs.nx, hs.ny), blk, 0, stream>>>(a, c);
+            TimedLaunch tl(&tm, stream, "plain_pass23");
+            k_pass23<<<grid2(hs.NX, hs.NY), blk, 0, stream>>>(a, c);
         }
-        if (sch.is_predictor()) {  // engine.cpp:1050-1058
-            CEL_CUDA_TRY(cudaMemcpyAsync(PRED, GRAD[scratch_i], ntex * sizeof(float4), cudaMemcpyDeviceToDevice, stream));
-            CEL_CUDA_TRY(cudaMemcpyAsync(FGPRED, FG[scratch_i], ntex * sizeof(float4), cudaMemcpyDeviceToDevice, stream));
-            CEL_CUDA_TRY(cudaMemcpyAsync(CUR, old_state, ntex * sizeof(float4), cudaMemcpyDeviceToDevice, stream));
-        }
-        // cyclic reduction in x then y, then back substitution (engine.cpp:1060-1217)
-        const float* rhs_x = reinterpret_cast<const float*>(new_state) + 1;
-        const float* rhs_y = reinterpret_cast<const float*>(new_state) + 2;
-        for (int k = 1; k < hs.Kx; ++k) {
-            const bool l0 = (k == 1);
-            TimedLaunch tl(&tm, stream, "plain_cr_reduce_x");
-            k_cr_reduce_x<<<grid2(hs.lenx[k], hs.ny), blk, 0, stream>>>(
-                l0 ? rhs_x : Dx[k - 1], l0 ? 4 : 1, l0 ? hs.NX * 4 : hs.lenx[k - 1] + 4, ABCx[k - 1],
-                l0 ? hs.NX : hs.lenx[k - 1] + 4, Dx[k], hs.lenx[k] + 4, hs.lenx[k], hs.ny);
-        }
-        for (int k = 1; k < hs.Ky; ++k) {
-            const bool l0 = (k == 1);
-            TimedLaunch tl(&tm, stream, "plain_cr_reduce_y");
-            k_cr_reduce_y<<<grid2(hs.nx, hs.leny[k]), blk, 0, stream>>>(
-                l0 ? rhs_y : Dy[k - 1], l0 ? 4 : 1, l0 ? hs.NX * 4 : hs.NX, ABCy[k - 1], hs.NX, Dy[k], hs.leny[k], hs.nx);
-        }
-        for (int k = hs.Kx - 1; k >= 0; --k) {
-            const bool l0 = (k == 0);
-            TimedLaunch tl(&tm, stream, "plain_cr_subst_x");
-            k_cr_subst_x<<<grid2(hs.lenx[k], hs.ny), blk, 0, stream>>>(
-                l0 ? rhs_x : Dx[k], l0 ? 4 : 1, l0 ? hs.NX * 4 : hs.lenx[k] + 4, ABCx[k], l0 ? hs.NX : hs.lenx[k] + 4,
-                k + 1 < hs.Kx ? Xx[k + 1] : nullptr, k + 1 < hs.Kx ? hs.lenx[k + 1] + 4 : 0, Xx[k],
-                l0 ? hs.NX : hs.lenx[k] + 4, hs.lenx[k], hs.ny);
-        }
-        for (int k = hs.Ky - 1; k >= 0; --k) {
-            const bool l0 = (k == 0);
-            TimedLaunch tl(&tm, stream, "plain_cr_subst_y");
-            k_cr_subst_y<<<grid2(hs.nx, hs.leny[k]), blk, 0, stream>>>(
-                l0 ? rhs_y : Dy[k], l0 ? 4 : 1, l0 ? hs.NX * 4 : hs.NX, ABCy[k], hs.NX,
-                k + 1 < hs.Ky ? Xy[k + 1] : nullptr, Xy[k], hs.leny[k], hs.nx);
-        }
+        const bool was_predictor = sch.is_predictor();
+        // the implicit systems along x and y, in place (engine.cpp:1060-1217)
         {
-            TimedLaunch tl(&tm, stream, "plain_copy_from");
-            k_copy_from<<<grid2(hs.nx, hs.ny), blk, 0, stream>>>(new_state, Xx[0], Xy[0], c);
+            TimedLaunch tl(&tm, stream, "plain_cr");
+            auto* k = smem_x ? (smem_y ? k_cr<true, true> : k_cr<true, false>) : (smem_y ? k_cr<false, true> : k_cr<false, false>);
+            solve.st = new_state;
+            k<<<hs.ny + (hs.nx + CR_COLS - 1) / CR_COLS, CR_THREADS, smem_cr, stream>>>(solve, c);
         }
-        // boundaries East, North, West, South (engine.cpp:1342-1438)
-        for (int side : {1, 0, 3, 2})
-            if (int e = boundary_side(new_state, side)) return e;
+        boundaries(new_state);
         {
             TimedLaunch tl(&tm, stream, "plain_pass1");
             k_pass1<<<grid2(hs.nx + 2, hs.ny + 2), blk, 0, stream>>>(new_state, BOT, AUX1, H, U, V, AUX2, c);
@@ -857,8 +1064,11 @@ public:
         if (book) {
             const int o = old_i, oo = oldold_i, s = scratch_i;
             old_i = s; oldold_i = o; scratch_i = oo;
+        } else if (was_predictor) {   // the correctors read its derivatives and write elsewhere
+            pred_i = scratch_i;
+            std::swap(scratch_i, spare_i);
         }
-        sim_idx = 1 - sim_idx;
+        sim_idx = out_i;
         if (book && p.log.do_log && sch.last_count % p.log.log_step == 0) {
             // st_DumpToFile of the new state, with the time at the start of the step (engine.cpp:1488-1493)
             std::vector<float> host(ntex * 4);
