@@ -29,9 +29,11 @@ UNITS = [
     ("capi.cpp", []),
     ("lanes.cpp", []),
     ("plain.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
+    ("readback.cu", []),
     ("fused.cu", ["-prec-div=false", "-prec-sqrt=false", "-ftz=true"]),
 ]
-HEADERS = ["celeris_internal.hpp", "engine_iface.hpp", "scheme.hpp", "device_math.cuh", "batch.hpp", "boundary_plan.hpp"]
+HEADERS = ["celeris_internal.hpp", "engine_iface.hpp", "scheme.hpp", "device_math.cuh", "batch.hpp", "boundary_plan.hpp",
+           "readback.hpp"]
 
 
 def nvcc() -> str:

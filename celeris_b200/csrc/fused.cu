@@ -36,6 +36,7 @@
 #include "batch.hpp"
 #include "device_math.cuh"
 #include "engine_iface.hpp"
+#include "readback.hpp"
 #include "scheme.hpp"
 
 namespace cel {
@@ -2708,6 +2709,7 @@ struct cel_lane {
     cudaStream_t side = nullptr;       // second stream: the column solve runs beside the row solve
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cel::KernelTimer tm;
+    cel::Readback rb;                  // staging of state and aux reads
     cel::Scheme sch;      // shared pass sequence (all members use the same correction count)
     cel::Idx ix;
     int4* tiles = nullptr; int ntiles = 0;      // 32x16 tiles (statistics on demand)
@@ -3752,59 +3754,51 @@ int lane_stats_finish(cel_lane* b, cel_stats* out, bool current, std::string& er
     return CEL_OK;
 }
 
+// Member i's texels in the public layout (readback.hpp)
+static int read_texels(cel_lane* b, int i, PackMode mode, float* rgba, std::string& err) {
+    if (i < 0 || i >= int(b->mem.size())) { err = "member index out of range"; return CEL_ERR_ARG; }
+    const Member& m = b->mem[i];
+    const MemberDev& d = b->hdev[i];
+    PackArgs a{};
+    for (int q = 0; q < 3; ++q) {
+        a.hi[q] = d.S[b->ix.sin][q];
+        a.lo[q] = b->mixed ? d.L[b->ix.sin][q] : nullptr;
+    }
+    a.aux = reinterpret_cast<const float2*>(d.AUX[0]);
+    a.NX = m.hs.NX;
+    a.P = m.P;
+    a.mode = mode;
+    (void)cudaGetLastError();
+    const size_t bytes = size_t(m.hs.NX) * m.hs.NY * sizeof(float4);
+    if (bytes <= READBACK_DIRECT) {
+        // small: formed in the history slot that the next pass overwrites (4 planes of at least NX columns),
+        // then one copy
+        float4* scratch = d.HA[b->ix.scr];
+        B_TRY(launch_pack(a, 0, bytes / sizeof(float4), scratch, b->stream));
+        B_TRY(cudaMemcpyAsync(rgba, scratch, bytes, cudaMemcpyDeviceToHost, b->stream));
+        B_TRY(cudaStreamSynchronize(b->stream));
+        return CEL_OK;
+    }
+    return b->rb.read(rgba, bytes, b->stream,
+                      [&](size_t off, size_t n, char* slot) {
+                          return launch_pack(a, off / sizeof(float4), n / sizeof(float4), reinterpret_cast<float4*>(slot),
+                                             b->stream);
+                      },
+                      err);
+}
+
 // The state as two float textures whose sum is the compensated value: hi = the stored state, lo =
 // its low words (zero in the FP32 forms).  Either pointer may be null.
 int lane_get_state_parts(cel_lane* b, int i, float* hi_rgba, float* lo_rgba, std::string& err) {
     if (i < 0 || i >= int(b->mem.size())) { err = "member index out of range"; return CEL_ERR_ARG; }
-    Member& m = b->mem[i];
-    const MemberDev& d = b->hdev[i];
-    const int NX = m.hs.NX, NY = m.hs.NY;
-    std::vector<float> pl[3], lo[3];
-    for (int q = 0; q < 3; ++q) {
-        pl[q].resize(m.plane);
-        lo[q].assign(m.plane, 0.f);
-        B_TRY(cudaMemcpyAsync(pl[q].data(), d.S[b->ix.sin][q], m.plane * sizeof(float), cudaMemcpyDeviceToHost, b->stream));
-        if (b->mixed)
-            B_TRY(cudaMemcpyAsync(lo[q].data(), d.L[b->ix.sin][q], m.plane * sizeof(float), cudaMemcpyDeviceToHost, b->stream));
-    }
-    B_TRY(cudaStreamSynchronize(b->stream));
-    for (int y = 0; y < NY; ++y)
-        for (int x = 0; x < NX; ++x) {
-            const size_t k = size_t(y) * m.P + x, o = (size_t(y) * NX + x) * 4;
-            for (int q = 0; q < 3; ++q) {
-                if (hi_rgba) hi_rgba[o + q] = pl[q][k];
-                if (lo_rgba) lo_rgba[o + q] = lo[q][k];
-            }
-            if (hi_rgba) hi_rgba[o + 3] = 0.f;
-            if (lo_rgba) lo_rgba[o + 3] = 0.f;
-        }
+    if (hi_rgba)
+        if (int e = read_texels(b, i, PACK_HI, hi_rgba, err)) return e;
+    if (lo_rgba)
+        if (int e = read_texels(b, i, PACK_LO, lo_rgba, err)) return e;
     return CEL_OK;
 }
 
-int lane_get_state(cel_lane* b, int i, float* rgba, std::string& err) {
-    if (i < 0 || i >= int(b->mem.size())) { err = "member index out of range"; return CEL_ERR_ARG; }
-    Member& m = b->mem[i];
-    const MemberDev& d = b->hdev[i];
-    const int NX = m.hs.NX, NY = m.hs.NY;
-    std::vector<float> pl[3], lo[3];
-    for (int q = 0; q < 3; ++q) {
-        pl[q].resize(m.plane);
-        B_TRY(cudaMemcpyAsync(pl[q].data(), d.S[b->ix.sin][q], m.plane * sizeof(float), cudaMemcpyDeviceToHost, b->stream));
-        if (b->mixed) {
-            lo[q].resize(m.plane);
-            B_TRY(cudaMemcpyAsync(lo[q].data(), d.L[b->ix.sin][q], m.plane * sizeof(float), cudaMemcpyDeviceToHost, b->stream));
-        }
-    }
-    B_TRY(cudaStreamSynchronize(b->stream));
-    for (int y = 0; y < NY; ++y)
-        for (int x = 0; x < NX; ++x) {
-            const size_t k = size_t(y) * m.P + x;
-            float* o = rgba + (size_t(y) * NX + x) * 4;
-            for (int q = 0; q < 3; ++q) o[q] = b->mixed ? float(double(pl[q][k]) + double(lo[q][k])) : pl[q][k];
-            o[3] = 0.f;
-        }
-    return CEL_OK;
-}
+int lane_get_state(cel_lane* b, int i, float* rgba, std::string& err) { return read_texels(b, i, PACK_SUM, rgba, err); }
 
 int lane_set_state(cel_lane* b, int i, const float* rgba, std::string& err) {
     if (i < 0 || i >= int(b->mem.size())) { err = "member index out of range"; return CEL_ERR_ARG; }
@@ -3872,23 +3866,7 @@ int lane_add_solitary_wave(cel_lane* b, int i, double H, double theta_deg, doubl
     return CEL_OK;
 }
 
-int lane_get_aux(cel_lane* b, int i, float* rgba, std::string& err) {
-    if (i < 0 || i >= int(b->mem.size())) { err = "member index out of range"; return CEL_ERR_ARG; }
-    Member& m = b->mem[i];
-    const MemberDev& d = b->hdev[i];
-    // AUX is one float2 plane pair: {max inundated depth, breaking indicator} per texel
-    std::vector<float> a(2 * m.plane);
-    B_TRY(cudaMemcpyAsync(a.data(), d.AUX[0], 2 * m.plane * sizeof(float), cudaMemcpyDeviceToHost, b->stream));
-    B_TRY(cudaStreamSynchronize(b->stream));
-    const int NX = m.hs.NX, NY = m.hs.NY;
-    for (int y = 0; y < NY; ++y)
-        for (int x = 0; x < NX; ++x) {
-            float* o = rgba + (size_t(y) * NX + x) * 4;
-            const size_t k = 2 * (size_t(y) * m.P + x);
-            o[0] = a[k]; o[1] = 0.f; o[2] = 0.f; o[3] = a[k + 1];
-        }
-    return CEL_OK;
-}
+int lane_get_aux(cel_lane* b, int i, float* rgba, std::string& err) { return read_texels(b, i, PACK_AUX, rgba, err); }
 
 int lane_use_graph(cel_lane* b, bool enable, std::string& err) {
     (void)err;

@@ -18,6 +18,7 @@
 #include "boundary_plan.hpp"
 #include "device_math.cuh"
 #include "engine_iface.hpp"
+#include "readback.hpp"
 #include "scheme.hpp"
 
 namespace cel {
@@ -622,6 +623,7 @@ public:
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     KernelTimer tm;
+    Readback rb;
     size_t ntex = 0;
     // device textures
     // The state rotates through three textures and the derivatives through four, by index: a corrector
@@ -1104,19 +1106,27 @@ public:
         bootstrap_needed = true;
         return CEL_OK;
     }
+    int read_texture(const float4* t, float* rgba) {
+        if (ntex * sizeof(float4) <= READBACK_DIRECT) {
+            CEL_CUDA_TRY(cudaMemcpyAsync(rgba, t, ntex * sizeof(float4), cudaMemcpyDeviceToHost, stream));
+            CEL_CUDA_TRY(cudaStreamSynchronize(stream));
+            return CEL_OK;
+        }
+        return rb.read(rgba, ntex * sizeof(float4), stream,
+                       [&](size_t off, size_t n, char* slot) {
+                           return cudaMemcpyAsync(slot, reinterpret_cast<const char*>(t) + off, n, cudaMemcpyDeviceToHost, stream);
+                       },
+                       err);
+    }
     int get_state(float* rgba) override {
-        CEL_CUDA_TRY(cudaMemcpyAsync(rgba, st[sim_idx], ntex * sizeof(float4), cudaMemcpyDeviceToHost, stream));
-        CEL_CUDA_TRY(cudaStreamSynchronize(stream));
-        return CEL_OK;
+        return read_texture(st[sim_idx], rgba);
     }
     int get_bottom(float* b3) override {
         for (size_t i = 0; i < ntex; ++i) { b3[3 * i] = hs.BY[i]; b3[3 * i + 1] = hs.BX[i]; b3[3 * i + 2] = hs.BA[i]; }
         return CEL_OK;
     }
     int get_aux(float* rgba) override {
-        CEL_CUDA_TRY(cudaMemcpyAsync(rgba, AUX1, ntex * sizeof(float4), cudaMemcpyDeviceToHost, stream));
-        CEL_CUDA_TRY(cudaStreamSynchronize(stream));
-        return CEL_OK;
+        return read_texture(AUX1, rgba);
     }
     // newTerrainSettings -> fillTerrainTexture (engine.cpp:3313-3379): keep every texel's water depth
     // (w - BA_old + BA_new, in float as there), resample the bottom, clear both aux textures and
