@@ -67,9 +67,11 @@ struct MemberDev {
     int P;                  // plane pitch in floats
     float* base;            // first plane; plane k starts at base + k * plane
     unsigned long long plane;
-    const CUtensorMap* tmaps;  // 2D row maps: state [buffer*3 + field], then BA, BX, BY
+    const CUtensorMap* tmaps;  // 2D row maps: state [buffer*3 + field], then BA, BX, BY (k_march); from 13 on the
+                               // row-pair maps of k_march2: 3 state buffers and the corners for each width
     float tan_thr;          // tan(dissipation threshold): atan(x) > thr  <=>  x > tan(thr)
     const float* dtp;       // this member's time step (device table, host-updatable)
+    float dt_base;          // the uniform time step that an adaptive batch's correctors take
     const float* ab;        // adaptive AB3 predictor: {k, A0, A1, A2, K0, K1, K2} (see k_choose_dt)
     float* S[3][3];         // state buffers [buffer][w, hu, hv]
     float* L[3][3];         // compensation words (mixed form)
@@ -108,6 +110,7 @@ struct PassArgs {
     int friction;       // some member has a nonzero friction coefficient
     double* late_flag;  // set when a bounded TMA wait gave up
     double* spart;      // STATS_N totals of each strip of the stencil (statistics pass)
+    int handoff;        // a predictor with correctors to follow: it leaves them its combinations, not its rates
 };
 
 __device__ __forceinline__ void two_sum_add(float& hi, float& lo, float d) {
@@ -183,7 +186,6 @@ constexpr int MH_DEFAULT = 64;   // rows per strip unless tuned (each work item 
 constexpr int RING = 7;          // state / bottom rows resident in shared memory (PREFETCH + 5)
 constexpr int RBOX = 136;        // TMA box width in floats (covers columns x0-2 .. x0+127)
 constexpr int RSTR = 160;        // ring row stride in floats (640 B, a multiple of 128 B)
-constexpr int CBOX = RBOX + 4;   // corner-grid box: the RBOX cells' corners (one more), rounded to 16 B
 constexpr unsigned ROW_BYTES = 6u * RBOX * 4u;
 constexpr int PREFETCH = 2;      // rows requested ahead of the row being consumed
 
@@ -435,11 +437,11 @@ __global__ void __launch_bounds__(MW, MARCH_MIN_CTAS) k_march(const MemberDev* _
         // per-plane bases of this pass
         const float4* __restrict__ HAo = reinterpret_cast<const float4*>(B + (iH0 + 5 * pa.og) * PL);
         const float4* __restrict__ HAoo = reinterpret_cast<const float4*>(B + (iH0 + 5 * pa.oog) * PL);
-        const float4* __restrict__ HAp = reinterpret_cast<const float4*>(B + (iH0 + 5 * pa.pred) * PL);
+        const float* __restrict__ HCp = B + (iH0 + 5 * pa.pred) * PL;   // the predictor's combinations (3 planes)
         float4* __restrict__ HAs = reinterpret_cast<float4*>(B + (iH0 + 5 * pa.scr) * PL);
+        float* __restrict__ HCs = B + (iH0 + 5 * pa.scr) * PL;
         const float* __restrict__ HBo = B + (iH0 + 5 * pa.og + 4) * PL;
         const float* __restrict__ HBoo = B + (iH0 + 5 * pa.oog + 4) * PL;
-        const float* __restrict__ HBp = B + (iH0 + 5 * pa.pred + 4) * PL;
         float* __restrict__ HBs = B + (iH0 + 5 * pa.scr + 4) * PL;
         float* __restrict__ Wout = B + (3 * pa.out) * PL;
         const float* __restrict__ Wcur = B + (3 * pa.cur) * PL;
@@ -513,8 +515,8 @@ __global__ void __launch_bounds__(MW, MARCH_MIN_CTAS) k_march(const MemberDev* _
             // neighbour it never stores to)
             const size_t el = erow + size_t(xl);
             // per-cell inputs of Pass3 at (xc, t), requested before the face work
-            float4 ho = make_float4(0.f, 0.f, 0.f, 0.f), hoo = ho, hp = ho;
-            float go = 0.f, goo = 0.f, gp = 0.f, wcur = 0.f, wlo = 0.f;
+            float4 ho = make_float4(0.f, 0.f, 0.f, 0.f), hoo = ho;
+            float go = 0.f, goo = 0.f, cw = 0.f, cu = 0.f, cv = 0.f, wcur = 0.f, wlo = 0.f;
             // aux texel of row t+1 owned by this strip (ghost texels x = 1 / y = 1 go with column /
             // row 2), read-modify-written after the faces of row t+1
             const int gy = t + 1;
@@ -525,10 +527,11 @@ __global__ void __launch_bounds__(MW, MARCH_MIN_CTAS) k_march(const MemberDev* _
             float2 aux_old = make_float2(0.f, 0.f);
             if (aux_ok) aux_old = *a0;
             if (p3) {
-                if (!euler) {
+                if (corr) {
+                    cw = __ldg(HCp + el); cu = __ldg(HCp + PL + el); cv = __ldg(HCp + 2 * PL + el); wcur = __ldg(Wcur + el);
+                } else if (!euler) {
                     ho = __ldg(HAo + el); hoo = __ldg(HAoo + el);
                     go = __ldg(HBo + el); goo = __ldg(HBoo + el);
-                    if (corr) { hp = __ldg(HAp + el); gp = __ldg(HBp + el); wcur = __ldg(Wcur + el); }
                 }
                 if (MIXED) wlo = __ldg(Lbase + el);
             }
@@ -625,10 +628,11 @@ __global__ void __launch_bounds__(MW, MARCH_MIN_CTAS) k_march(const MemberDev* _
                     rhu = k12 * (23.0f * f1 - 16.0f * ho.y + 5.0f * hoo.y) + (2.0f * Fs - 3.0f * ho.w + hoo.w);
                     rhv = k12 * (23.0f * f2 - 16.0f * ho.z + 5.0f * hoo.z) + (2.0f * Gs - 3.0f * go + goo);
                 } else {
-                    const float k24 = dt * (1.0f / 24.0f);
-                    dw = k24 * (9 * f0 + 19 * hp.x - 5 * ho.x + 1 * hoo.x);
-                    rhu = k24 * (9 * f1 + 19 * hp.y - 5 * ho.y + 1 * hoo.y) + Fs - hp.w;
-                    rhv = k24 * (9 * f2 + 19 * hp.z - 5 * ho.z + 1 * hoo.z) + Gs - gp;
+                    // the predictor's combinations with this pass's rates (k_march2 has the layout)
+                    const float k9 = dt * 0.375f;
+                    dw = dt * (1.0f / 24.0f) * (9 * f0 + cw);
+                    rhu = k9 * f1 + (Fs + cu);
+                    rhv = k9 * f2 + (Gs + cv);
                     wbase = wcur;
                 }
                 float wn = wbase, wl = wlo;
@@ -639,8 +643,15 @@ __global__ void __launch_bounds__(MW, MARCH_MIN_CTAS) k_march(const MemberDev* _
                     if (MIXED) Lout[e] = wl;
                     R0[e] = rhu;
                     R0[e + PL] = rhv;
-                    HAs[e] = make_float4(f0, f1, f2, Fs);
-                    HBs[e] = Gs;
+                    if (pa.handoff) {
+                        const float k24 = (ADAPT ? M.dt_base : dt) * (1.0f / 24.0f);
+                        HCs[e] = 19 * f0 - 5 * ho.x + hoo.x;
+                        HCs[e + PL] = k24 * (19 * f1 - 5 * ho.y + hoo.y) - Fs;
+                        HCs[e + 2 * PL] = k24 * (19 * f2 - 5 * ho.z + hoo.z) - Gs;
+                    } else {
+                        HAs[e] = make_float4(f0, f1, f2, Fs);
+                        HBs[e] = Gs;
+                    }
                 }
                 if (stats) {   // GetStats (compute.hlsl:1319-1378) of the input state
                     const float q = div_by_h_fast(h, c.epsilon);
@@ -729,22 +740,47 @@ __global__ void __launch_bounds__(MW, MARCH_MIN_CTAS) k_march(const MemberDev* _
 // k_march2: the passes of k_march on two rows per step.  Every per-cell quantity is a pair
 // (row t, row t+1) held in a float2, and arithmetic on pairs uses the paired single-precision
 // instructions of sm_100 (__fadd2_rn, __fmul2_rn, __ffma2_rn): one instruction does the work of
-// two cells.  The per-step bookkeeping (barriers, TMA requests, ring rotation, addressing) is paid
-// once per two rows.  The faces run one step ahead of Pass3: step j computes the faces of rows
-// t+2 and t+3 and uses those of rows t and t+1 from step j-1.  Ring: RING2 = 9 rows, the window
-// t-2 .. t+4 plus the two rows requested one step ahead.
+// two cells.  The faces run one step ahead of Pass3: step j computes the faces of rows t+2 and t+3
+// and uses those of rows t and t+1 from step j-1.
+//
+// The ring holds row pairs: one 3-D TMA box brings w, hu and hv of rows t, t+1, a second one the two
+// corner-grid rows above them (the bottom BA, BX, BY is rebuilt from the corners), onto one mbarrier.
+// A step's window is the pairs t-2 .. t+4, and the pair t+6 is requested a step ahead: PRING = 5 slots.
+// Every shared-memory operand is one of four slot addresses plus a compile-time offset (the 9-row ring
+// before it took a remainder per row and 8 copies a step: without a corrector, 6.6 M cells at 123 -> 117 us
+// a launch).
+//
+// Bytes.  A corrector combines its rates with 19 f - 5 f_old + f_oldold of its predictor's step (AM4), and
+// F*, G* with the predictor's.  The predictor, which holds all three levels, leaves that combination in its
+// history slot (3 planes, 12 bytes a cell) instead of its rates (20), and every corrector of the step
+// reads it instead of three levels (60): compensated form 112 -> 104 bytes a cell in the predictor,
+// 136 -> 88 in the corrector.  28 members, 16 M cells: 286 -> 253 us a launch on average, ms per step
+// 1.482 -> 1.374.  What the correctors add up is rounded once more than before (the combination, relative
+// 2^-24), as the rates themselves were; the states' distance from 64 bits is unchanged.
 // ---------------------------------------------------------------------------------------------
 // CTAs per SM the paired-row stencil is built for: 3 of 128 threads or 4 of 96 (12 warps either
 // way, within the register file at up to 168 registers per thread)
 constexpr int march2_min_ctas(int w) { return w == 128 ? MARCH2_MIN_CTAS : 4; }
-constexpr int RING2 = 9;
-constexpr int FSTR2 = RING2 * RSTR;
-// the 9-row TMA ring of the paired-row stencil: fields w, hu, hv and the corner grid row above
-// each cell row (the bottom BA, BX, BY is rebuilt from the corners)
-constexpr size_t MARCH2_DYN_SMEM = sizeof(float) * 4 * FSTR2;
-constexpr unsigned ROW_BYTES2 = (3u * RBOX + unsigned(CBOX)) * 4u;
+constexpr int PRING = 5;
+template <int TW>
+struct PairRing {
+    static constexpr int BOX = TW + 8;                          // floats of a row: columns x0-2 .. x0+TW, from a
+                                                                // 16-byte boundary up to 2 columns before
+    static constexpr int CORNER = (6 * BOX + 31) / 32 * 32;     // slot: 3 fields x 2 rows, then (128-byte aligned)
+    static constexpr int SLOT = (CORNER + 2 * BOX + 31) / 32 * 32;   // the 2 corner rows
+    static constexpr size_t SMEM = sizeof(float) * size_t(PRING) * SLOT;
+};
 
+__device__ __forceinline__ void tma_pair3(float* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+            smem_u32(dst)),
+        "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(0), "r"(smem_u32(bar))
+        : "memory");
+}
 
+// kinds of pass a stencil kernel is built for
+enum { PASS_FIXED = 0, PASS_ADAPTIVE = 1, PASS_CORRECTOR = 2 };   // Euler or AB3; variable-step AB3; AM4
 
 typedef float2 f2;
 __device__ __forceinline__ f2 P2(float a, float b) { return make_float2(a, b); }
@@ -809,30 +845,30 @@ struct Carry2 {
     }
 };
 
-// Pass1 on rows r and r+1 of one column: ring-row offsets of rows r-1, r, r+1, r+2 and the column.
-__device__ __forceinline__ void faces_at2(const float* __restrict__ ring, int om1, int o0, int o1, int o2, int col,
-                                          const SimConsts& c, Face2& f) {
-    const float* W = ring;
-    const float* HU = ring + FSTR2;
-    const float* HV = ring + 2 * FSTR2;
-    const float* Cr = ring + 3 * FSTR2;   // slot of row q holds corner row q+1
-    const int a0 = o0 + col, a1 = o1 + col;
+// Pass1 on rows r and r+1 of one column: p0, p1, p2 point to this column in the slots of the pairs
+// (r-2, r-1), (r, r+1), (r+2, r+3).
+template <int TW>
+__device__ __forceinline__ void faces_at2(const float* __restrict__ p0, const float* __restrict__ p1,
+                                          const float* __restrict__ p2, const SimConsts& c, Face2& f) {
+    constexpr int RW = PairRing<TW>::BOX, HUo = 2 * RW, HVo = 4 * RW, Co = PairRing<TW>::CORNER;
     const f2 tt = S2(c.two_theta);
-    const f2 wc = P2(W[a0], W[a1]), wl = P2(W[a0 - 1], W[a1 - 1]), wr = P2(W[a0 + 1], W[a1 + 1]);
-    const f2 wd = P2(W[om1 + col], W[a0]), wu = P2(W[a1], W[o2 + col]);
-    // corners of cells (r, r+1): south edges in the slots of rows r-1, r; north edges in r, r+1
-    const f2 L0 = P2(Cr[om1 + col], Cr[a0]), L1 = P2(Cr[a0], Cr[a1]);
-    const f2 R0 = P2(Cr[om1 + col + 1], Cr[a0 + 1]), R1 = P2(Cr[a0 + 1], Cr[a1 + 1]);
+    const f2 wc = P2(p1[0], p1[RW]), wl = P2(p1[-1], p1[RW - 1]), wr = P2(p1[1], p1[RW + 1]);
+    const f2 wd = P2(p0[RW], p1[0]), wu = P2(p1[RW], p2[0]);
+    // corners of cells (r, r+1): a row's slot holds the corner row above it
+    const f2 L0 = P2(p0[Co + RW], p1[Co]), L1 = P2(p1[Co], p1[Co + RW]);
+    const f2 R0 = P2(p0[Co + RW + 1], p1[Co + 1]), R1 = P2(p1[Co + 1], p1[Co + RW + 1]);
     const f2 BN = corner_mean2(L1, R1), BE = corner_mean2(R0, R1);
     const f2 BS = corner_mean2(L0, R0), BW = corner_mean2(L0, L1);
     f2 wN, wE, wS, wW, huN, huE, huS, huW, hvN, hvE, hvS, hvW, sd1, sd2;
     recon_sd2(tt, wl, wc, wr, wW, wE, sd1);
     recon_sd2(tt, wd, wc, wu, wS, wN, sd2);
-    const f2 huc = P2(HU[a0], HU[a1]), hvc = P2(HV[a0], HV[a1]);
-    recon2(tt, P2(HU[a0 - 1], HU[a1 - 1]), huc, P2(HU[a0 + 1], HU[a1 + 1]), huW, huE);
-    recon2(tt, P2(HU[om1 + col], HU[a0]), huc, P2(HU[a1], HU[o2 + col]), huS, huN);
-    recon2(tt, P2(HV[a0 - 1], HV[a1 - 1]), hvc, P2(HV[a0 + 1], HV[a1 + 1]), hvW, hvE);
-    recon2(tt, P2(HV[om1 + col], HV[a0]), hvc, P2(HV[a1], HV[o2 + col]), hvS, hvN);
+    auto momentum = [&](int o, f2& vW, f2& vE, f2& vS, f2& vN) {
+        const f2 vc = P2(p1[o], p1[o + RW]);
+        recon2(tt, P2(p1[o - 1], p1[o + RW - 1]), vc, P2(p1[o + 1], p1[o + RW + 1]), vW, vE);
+        recon2(tt, P2(p0[o + RW], p1[o]), vc, P2(p1[o + RW], p2[o]), vS, vN);
+    };
+    momentum(HUo, huW, huE, huS, huN);
+    momentum(HVo, hvW, hvE, hvS, hvN);
     correct_w2(BW, BE, wc, wW, wE);
     correct_w2(BS, BN, wc, wS, wN);
     f.hN = sub2(wN, BN); f.hE = sub2(wE, BE); f.hS = sub2(wS, BS); f.hW = sub2(wW, BW);
@@ -885,32 +921,30 @@ struct Kahan2 {
     __device__ __forceinline__ double value() const { return (double(s.x) - double(c.x)) + (double(s.y) - double(c.y)); }
 };
 
-template <bool MIXED, bool ADAPT, int TW>
+template <bool MIXED, int KIND, int TW>
 __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const MemberDev* __restrict__ mems,
                                                                const int4* __restrict__ tiles, int ntiles, PassArgs pa) {
-    extern __shared__ __align__(128) float ring[];   // 4 * FSTR2 floats: w, hu, hv, corner rows
-    __shared__ float dring[RING2 * RSTR];   // still-water depth of each ring row (same stride as the ring)
-    __shared__ __align__(8) unsigned long long bars[RING2];
+    constexpr int RW = PairRing<TW>::BOX, SLOT = PairRing<TW>::SLOT, CO = PairRing<TW>::CORNER, HUo = 2 * RW, HVo = 4 * RW;
+    constexpr int DSLOT = 2 * RW;
+    constexpr bool CORR = KIND == PASS_CORRECTOR, ADAPT = KIND == PASS_ADAPTIVE;
+    extern __shared__ __align__(128) float ring[];   // PRING slots: w, hu, hv (2 rows each), corner rows
+    __shared__ float dring[PRING * DSLOT];  // still-water depth of the ring's rows
+    __shared__ __align__(8) unsigned long long bars[PRING];
     __shared__ float fW[2][2][4][TW];       // [step parity][row of the pair][hW, uW, vW, wW][thread]
     __shared__ float xb[2][3][TW];          // [row of the pair][component][thread]
     constexpr int OFF = MIXED ? 18 : 9;
     constexpr int iR0 = OFF + 3, iH0 = OFF + 5, iAUX = OFF + 25;
     const int tid = threadIdx.x;
     if (tid == 0) {
-        for (int k = 0; k < RING2; ++k) mbar_init(&bars[k], 1);
+        for (int k = 0; k < PRING; ++k) mbar_init(&bars[k], 1);
         mbar_fence_init();
     }
     __syncthreads();
-    unsigned seq = 0;          // rows requested by this CTA so far (the same value in every thread)
-    unsigned requested = 0;    // thread 0: sequence number of the last row it requested, plus one
+    unsigned seq = 0;          // pairs requested by this CTA so far (the same value in every thread)
+    unsigned requested = 0;    // thread 0: sequence number of the last pair it requested, plus one
     bool tma_late = false;
-    const float* W = ring;
-    const float* HU = ring + FSTR2;
-    const float* HV = ring + 2 * FSTR2;
-    const float* Cr = ring + 3 * FSTR2;   // slot of row q: corner row q+1
-    const bool stats = pa.stats != 0;
-    const bool corr = pa.scheme == CEL_SCHEME_CORRECTOR;
-    const bool euler = pa.scheme == CEL_SCHEME_EULER;
+    const bool stats = !CORR && pa.stats != 0;
+    const bool euler = !CORR && pa.scheme == CEL_SCHEME_EULER;
 
     for (int it = blockIdx.x; it < ntiles; it += gridDim.x) {
         const int4 tl = tiles[it];
@@ -919,15 +953,14 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
         const int P = M.P, nx = c.nx, ny = c.ny, NYm1 = c.NY - 1;
         float* __restrict__ B = M.base;
         const size_t PL = M.plane;
-        const CUtensorMap* tm = M.tmaps;
+        const CUtensorMap* tms = M.tmaps + (TW == 128 ? 13 : 17);   // pair maps: state buffers, corners
         const int x0 = tl.y, y0 = tl.z, MH = tl.w;
         const int xs = (x0 - 2) & ~3;          // TMA box start, 16-byte aligned
         const int xc = x0 - 1 + tid;           // this thread's column
-        const int rc0 = xc - xs;               // its ring column (1 .. 131)
+        const int rc0 = xc - xs;               // its ring column (1 .. TW + 2)
         const int rc = max(rc0, 2);            // Pass3 column (clamped for the halo thread 0)
         const int yend = min(y0 + MH, ny + 2);
         const int nsteps = (yend - y0 + 1) / 2;             // output row pairs of this strip
-        const int last_row = y0 + 2 * (nsteps - 1) + 4;     // last row any step reads
         const bool out_col = tid >= 1 && tid <= (TW - 2) && xc < nx + 2;
         const int xl = min(xc, c.NX - 1);
         const float dtm = *M.dtp;
@@ -935,102 +968,106 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
         const float sl = c.sea_level;
         const float4* __restrict__ HAo = reinterpret_cast<const float4*>(B + (iH0 + 5 * pa.og) * PL);
         const float4* __restrict__ HAoo = reinterpret_cast<const float4*>(B + (iH0 + 5 * pa.oog) * PL);
-        const float4* __restrict__ HAp = reinterpret_cast<const float4*>(B + (iH0 + 5 * pa.pred) * PL);
+        const float* __restrict__ HCp = B + (iH0 + 5 * pa.pred) * PL;   // the predictor's combinations (3 planes)
         float4* __restrict__ HAs = reinterpret_cast<float4*>(B + (iH0 + 5 * pa.scr) * PL);
+        float* __restrict__ HCs = B + (iH0 + 5 * pa.scr) * PL;
         const float* __restrict__ HBo = B + (iH0 + 5 * pa.og + 4) * PL;
         const float* __restrict__ HBoo = B + (iH0 + 5 * pa.oog + 4) * PL;
-        const float* __restrict__ HBp = B + (iH0 + 5 * pa.pred + 4) * PL;
         float* __restrict__ HBs = B + (iH0 + 5 * pa.scr + 4) * PL;
         float* __restrict__ Wout = B + (3 * pa.out) * PL;
         const float* __restrict__ Wcur = B + (3 * pa.cur) * PL;
         float* __restrict__ R0 = B + iR0 * PL;
         float2* __restrict__ AUX = reinterpret_cast<float2*>(B + iAUX * PL);
-        const float* __restrict__ Lbase = B + (9 + 3 * (corr ? pa.cur : pa.in)) * PL;
+        const float* __restrict__ Lbase = B + (9 + 3 * (CORR ? pa.cur : pa.in)) * PL;
         float* __restrict__ Lout = B + (9 + 3 * pa.out) * PL;
 
-        // row r of the strip has sequence number seq0 + (r - (y0 - 2)): slot seq % RING2, mbarrier
-        // phase parity (seq / RING2) & 1
+        // pair k of the strip holds rows y0 - 2 + 2k and the next; it has sequence number seq0 + k: slot
+        // seq % PRING, mbarrier phase parity (seq / PRING) & 1
         const unsigned seq0 = seq;
-        auto slot_of = [&](int r) { return int((seq0 + unsigned(r - (y0 - 2))) % RING2); };
-        auto par_of = [&](int r) { return ((seq0 + unsigned(r - (y0 - 2))) / RING2) & 1u; };
-        auto issue = [&](int row) {   // one thread: request a row's w, hu, hv and the corner row above it
-            if (tma_late) return;       // a wait gave up: request nothing more
-            requested = seq0 + unsigned(row - (y0 - 2)) + 1u;
-            const int sl_ = slot_of(row);
-            const int ry = min(row, NYm1);          // rows past the domain are never used; load the last
-            mbar_expect_tx(&bars[sl_], ROW_BYTES2);
-            float* dst = ring + sl_ * RSTR;
-            tma_row(dst, tm + pa.in * 3 + 0, xs, ry, &bars[sl_]);
-            tma_row(dst + FSTR2, tm + pa.in * 3 + 1, xs, ry, &bars[sl_]);
-            tma_row(dst + 2 * FSTR2, tm + pa.in * 3 + 2, xs, ry, &bars[sl_]);
-            tma_row(dst + 3 * FSTR2, tm + 12, xs, ry + 1, &bars[sl_]);   // corner rows 0 .. NY
+        const int npairs = nsteps + 3;
+        auto issue = [&](int k) {   // one thread: request pair k
+            if (tma_late) return;     // a wait gave up: request nothing more
+            requested = seq0 + unsigned(k) + 1u;
+            const int sl_ = int((seq0 + unsigned(k)) % PRING);
+            mbar_expect_tx(&bars[sl_], unsigned(8 * RW * sizeof(float)));
+            float* dst = ring + sl_ * SLOT;
+            tma_pair3(dst, tms + pa.in, xs, y0 - 2 + 2 * k, &bars[sl_]);
+            tma_row(dst + CO, tms + 3, xs, y0 - 1 + 2 * k, &bars[sl_]);   // the corner rows above them
         };
-        auto wait_row = [&](int row) {
-            if (!mbar_wait_bounded(&bars[slot_of(row)], par_of(row), tma_late ? 1 : (1 << 22))) tma_late = true;
+        auto wait_pair = [&](int k) {
+            const unsigned q = seq0 + unsigned(k);
+            if (!mbar_wait_bounded(&bars[q % PRING], (q / PRING) & 1u, tma_late ? 1 : (1 << 22))) tma_late = true;
         };
-        // still-water depth of a ring row: thread k covers ring column rc0(thread 0) - 1 + k, and
-        // threads 0 and 1 also the two columns past the last thread.  BA is rebuilt from the corner
-        // rows in the slots of rows row-1 and row; the strip's first row (whose lower corner row is
-        // not in the ring) reads BA from its plane (zero past the row, as the TMA fill would give).
+        // still-water depth of a pair's rows: thread k covers ring column rc0(thread 0) - 1 + k, and
+        // threads 0 and 1 also the two columns past the last thread.  below: the slot of the pair below;
+        // the strip's first row has no corner row below it in the ring, so its depth comes from BA's plane
+        // (zero past the row, as the TMA fill would give).
         const int dcol = rc0 - 1;
-        const int d2c = min(dcol + TW, RBOX - 1);
-        auto depth_at = [&](int row, int k) {
-            float ba;
-            if (row == y0 - 2) {
-                const int gx = xs + k;
-                ba = gx < c.NX ? M.BA[size_t(row) * P + gx] : 0.f;
-            } else {
-                const float* lo = Cr + slot_of(row - 1) * RSTR;
-                const float* up = Cr + slot_of(row) * RSTR;
-                ba = fmaf(0.25f, up[k + 1], fmaf(0.25f, up[k], fmaf(0.25f, lo[k + 1], 0.25f * lo[k])));
-            }
-            return fmaxf(0.f, sl - ba);
-        };
-        auto depth_row = [&](int row) {
-            float* dr = dring + slot_of(row) * RSTR;
-            dr[dcol] = depth_at(row, dcol);
-            if (tid < 2) dr[d2c] = depth_at(row, d2c);
+        const int d2c = min(dcol + TW, RW - 2);
+        auto depth_pair = [&](int below, int slot, bool first) {
+            auto at = [&](int k) {
+                const float* up = ring + slot * SLOT + CO + k;
+                float* d = dring + slot * DSLOT + k;
+                f2 ba;
+                if (first) {
+                    const int gx = xs + k;
+                    ba.x = gx < c.NX ? M.BA[size_t(y0 - 2) * P + gx] : 0.f;
+                    ba.y = corner_mean4(S2(up[0]), S2(up[1]), S2(up[RW]), S2(up[RW + 1])).x;
+                } else {
+                    const float* lo = ring + below * SLOT + CO + RW + k;
+                    ba = corner_mean4(P2(lo[0], up[0]), P2(lo[1], up[1]), P2(up[0], up[RW]), P2(up[1], up[RW + 1]));
+                }
+                d[0] = fmaxf(0.f, sl - ba.x);
+                d[RW] = fmaxf(0.f, sl - ba.y);
+            };
+            at(dcol);
+            if (tid < 2) at(d2c);
         };
 
         Kahan2 acc[5];
         double mfull = 0.0;
         f2 mx[4] = {S2(0.f), S2(0.f), S2(0.f), S2(0.f)};
         bool bad = false;
+        // aux texels this thread owns: the ghost texels x = 1 / y = 1 go with column / row 2
+        const int cxa = max(xc, 2);
+        const bool aux_col = xc >= 1 && xc < nx + 2 && cxa >= x0 && cxa < x0 + (TW - 2);
+        const int aux_last = min(y0 + MH, ny + 2);   // rows [y0, aux_last), and row 1 with the first strip
+        auto aux_step = [&](float2* p, float2 old, float md, float msd) {
+            const float bw = (msd > M.tan_thr) ? 1.0f : old.y;   // atan(msd) > threshold
+            *p = make_float2(fmaxf(md, old.x), bw * decay);
+        };
 
         __syncthreads();  // the previous strip is done with shared memory
         if (tid == 0) {
             fence_proxy_async();
-            for (int r = y0 - 2; r <= min(y0 + 2, last_row); ++r) issue(r);   // rows of the prologue and step -1
+            for (int k = 0; k < 3; ++k) issue(k);   // pairs of the prologue and step -1
         }
-        // prologue: faces of rows y0-2 and y0-1 (row y0-3's slot holds stale data: only row y0-2's
+        auto next_slot = [](int k) { return k + 1 == PRING ? 0 : k + 1; };
+        const int sA = int(seq0 % PRING), sB = next_slot(sA), sC = next_slot(sB);
+        const int sZ = sA == 0 ? PRING - 1 : sA - 1;   // a slot with no copy in flight
+        wait_pair(0);
+        wait_pair(1);
+        depth_pair(sZ, sA, true);
+        depth_pair(sA, sB, false);
+        // prologue: faces of rows y0-2 and y0-1 (the place of row y0-3 holds stale data: only row y0-2's
         // faces read it, and those are never used)
-        wait_row(y0 - 2); wait_row(y0 - 1); wait_row(y0);
-        depth_row(y0 - 2); depth_row(y0 - 1); depth_row(y0);
         Carry2 fp;   // faces of the previous step's rows (t, t+1 of the coming step)
         float ypv[3] = {0.f, 0.f, 0.f};   // y flux through the south face of row t (per component)
         {
-        Face2 fq;
-        faces_at2(ring, slot_of(y0 - 3) * RSTR, slot_of(y0 - 2) * RSTR, slot_of(y0 - 1) * RSTR, slot_of(y0) * RSTR,
-                  rc0, c, fq);
-        {
+            Face2 fq;
+            faces_at2<TW>(ring + sZ * SLOT + rc0, ring + sA * SLOT + rc0, ring + sB * SLOT + rc0, c, fq);
             const int pp = 1;   // parity of step -1
             fW[pp][0][0][tid] = fq.hW.x; fW[pp][0][1][tid] = fq.uW.x; fW[pp][0][2][tid] = fq.vW.x;
             fW[pp][1][0][tid] = fq.hW.y; fW[pp][1][1][tid] = fq.uW.y; fW[pp][1][2][tid] = fq.vW.y;
             fW[pp][0][3][tid] = fq.wW.x; fW[pp][1][3][tid] = fq.wW.y;
-        }
-        {   // aux of row y0-1 (the ghost row y = 1 belongs to the first strip)
-            const int gy = y0 - 1;
-            const int cxa = xc < 2 ? 2 : xc, cya = gy < 2 ? 2 : gy;
-            if (xc >= 1 && xc < nx + 2 && gy >= 1 && cxa >= x0 && cxa < x0 + (TW - 2) && cya >= y0 && cya < y0 + MH) {
-                float2* a = AUX + (size_t(gy) * P + xc);
-                const float2 old = *a;
-                const float md = (((fq.hN.y + fq.hE.y) + (fq.hS.y + fq.hW.y)) * 0.25f);
-                const float bw = (fq.msd.y > M.tan_thr) ? 1.0f : old.y;
-                *a = make_float2(fmaxf(md, old.x), bw * decay);
+            if (aux_col && y0 == 2) {   // the ghost row y = 1 belongs to the first strip
+                float2* a = AUX + (size_t(1) * P + xc);
+                aux_step(a, *a, ((fq.hN.y + fq.hE.y) + (fq.hS.y + fq.hW.y)) * 0.25f, fq.msd.y);
             }
+            fp.set(fq);
         }
-        fp.set(fq);
-        }
+        // slots of the pairs t-2, t, t+2, t+4; at step -1 (t = y0 - 2) the pair t-2 is not used
+        int sm = sZ, s0 = sA, s2 = sB, s4 = sC;
 
         for (int j = -1; j < nsteps; ++j) {
             const int t = y0 + 2 * j;
@@ -1039,65 +1076,47 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
             const size_t e0 = size_t(t) * P + xc, e1 = e0 + P;
             const size_t l0 = size_t(t) * P + xl, l1 = l0 + P;
             // Pass3 inputs of rows t and t+1
-            float4 ho0 = make_float4(0.f, 0.f, 0.f, 0.f), ho1 = ho0, hoo0 = ho0, hoo1 = ho0, hp0 = ho0, hp1 = ho0;
-            f2 go = S2(0.f), goo = go, gp = go, wcur = go, wlo = go;
+            float4 ho0 = make_float4(0.f, 0.f, 0.f, 0.f), ho1 = ho0, hoo0 = ho0, hoo1 = ho0;
+            f2 go = S2(0.f), goo = go, cw = go, cu = go, cv = go, wcur = go, wlo = go;
             if (p3) {
-                if (!euler) {
+                if (CORR) {
+                    cw = P2(__ldg(HCp + l0), __ldg(HCp + l1));
+                    cu = P2(__ldg(HCp + PL + l0), __ldg(HCp + PL + l1));
+                    cv = P2(__ldg(HCp + 2 * PL + l0), __ldg(HCp + 2 * PL + l1));
+                    wcur = P2(__ldg(Wcur + l0), __ldg(Wcur + l1));
+                } else if (!euler) {
                     ho0 = __ldg(HAo + l0); ho1 = __ldg(HAo + l1);
                     hoo0 = __ldg(HAoo + l0); hoo1 = __ldg(HAoo + l1);
                     go = P2(__ldg(HBo + l0), __ldg(HBo + l1));
                     goo = P2(__ldg(HBoo + l0), __ldg(HBoo + l1));
-                    if (corr) {
-                        hp0 = __ldg(HAp + l0); hp1 = __ldg(HAp + l1);
-                        gp = P2(__ldg(HBp + l0), __ldg(HBp + l1));
-                        wcur = P2(__ldg(Wcur + l0), __ldg(Wcur + l1));
-                    }
                 }
                 if (MIXED) wlo = P2(__ldg(Lbase + l0), __ldg(Lbase + l1));
             }
             // aux texels of rows t+2 and t+3 owned by this strip, read-modify-written after their faces
-            bool aux_ok[2];
-            float2* ap[2];
-            float2 aux_old[2];
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const int gy = t + 2 + k;
-                const int cxa = xc < 2 ? 2 : xc, cya = gy < 2 ? 2 : gy;
-                aux_ok[k] = xc >= 1 && xc < nx + 2 && gy >= 1 && gy < ny + 2 && cxa >= x0 && cxa < x0 + (TW - 2) &&
-                            cya >= y0 && cya < y0 + MH;
-                ap[k] = AUX + (size_t(min(gy, NYm1)) * P + xc);
-                aux_old[k] = aux_ok[k] ? *ap[k] : make_float2(0.f, 0.f);
-            }
-            __syncthreads();  // (A) the previous step is complete: ring slots of rows t-4, t-3 are free
-            if (tid == 0) {
+            const bool aux0 = aux_col && t + 2 < aux_last, aux1 = aux_col && t + 3 < aux_last;
+            float2* const ap0 = AUX + (size_t(min(t + 2, NYm1)) * P + xc);
+            float2* const ap1 = AUX + (size_t(min(t + 3, NYm1)) * P + xc);
+            const float2 old0 = aux0 ? *ap0 : make_float2(0.f, 0.f), old1 = aux1 ? *ap1 : make_float2(0.f, 0.f);
+            __syncthreads();  // (A) the previous step is complete: the slot of pair t-4 is free
+            if (tid == 0 && j + 4 < npairs) {
                 fence_proxy_async();
-                if (t + 5 <= last_row) issue(t + 5);
-                if (t + 6 <= last_row) issue(t + 6);
+                issue(j + 4);        // the pair t + 6
             }
-            wait_row(t + 3);
-            wait_row(t + 4);
-            depth_row(t + 3);
-            depth_row(t + 4);
-            const int om2 = slot_of(t - 2) * RSTR, om1 = slot_of(t - 1) * RSTR, o0 = slot_of(t) * RSTR;
-            const int o1 = slot_of(t + 1) * RSTR, o2 = slot_of(t + 2) * RSTR, o3 = slot_of(t + 3) * RSTR;
-            const int o4 = slot_of(t + 4) * RSTR;
+            wait_pair(j + 3);        // the pair t + 4
+            depth_pair(s2, s4, false);
+            const float* const q0 = ring + s0 * SLOT;
+            const float* const q2 = ring + s2 * SLOT;
             // ---- faces of rows t+2, t+3 (Pass1), their aux, and the y fluxes of rows t, t+1 ----
             Face2 f;
-            faces_at2(ring, o1, o2, o3, o4, rc0, c, f);
+            faces_at2<TW>(q0 + rc0, q2 + rc0, ring + s4 * SLOT + rc0, c, f);
             const int npar = (j + 1) & 1, par = j & 1;
             fW[npar][0][0][tid] = f.hW.x; fW[npar][0][1][tid] = f.uW.x; fW[npar][0][2][tid] = f.vW.x;
             fW[npar][1][0][tid] = f.hW.y; fW[npar][1][1][tid] = f.uW.y; fW[npar][1][2][tid] = f.vW.y;
             fW[npar][0][3][tid] = f.wW.x; fW[npar][1][3][tid] = f.wW.y;
             {
                 const f2 md = mul2(add2(add2(f.hN, f.hE), add2(f.hS, f.hW)), S2(0.25f));
-                if (aux_ok[0]) {
-                    const float bw = (f.msd.x > M.tan_thr) ? 1.0f : aux_old[0].y;   // atan(msd) > threshold
-                    *ap[0] = make_float2(fmaxf(md.x, aux_old[0].x), bw * decay);
-                }
-                if (aux_ok[1]) {
-                    const float bw = (f.msd.y > M.tan_thr) ? 1.0f : aux_old[1].y;
-                    *ap[1] = make_float2(fmaxf(md.y, aux_old[1].x), bw * decay);
-                }
+                if (aux0) aux_step(ap0, old0, md.x, f.msd.x);
+                if (aux1) aux_step(ap1, old1, md.y, f.msd.y);
             }
             const float g = c.g, hg = c.half_g;
             f2 yf[3];   // north faces of rows t, t+1: (N(t) vs S(t+1)), (N(t+1) vs S(t+2))
@@ -1115,28 +1134,34 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
             __syncthreads();  // (B)
             // ---- Pass3 at (xc, t) and (xc, t+1) ----
             if (p3) {
-                const int am2 = om2 + rc, am1 = om1 + rc, a0 = o0 + rc, a1 = o1 + rc, a2 = o2 + rc, a3 = o3 + rc;
+                // this column in the pairs t-2, t, t+2 (index RW: the second row)
+                const float* const a = ring + sm * SLOT + rc;
+                const float* const b = q0 + rc;
+                const float* const d = q2 + rc;
+                const float* const da = dring + sm * DSLOT + rc;
+                const float* const db = dring + s0 * DSLOT + rc;
+                const float* const dd = dring + s2 * DSLOT + rc;
                 // rows t, t+1 as pairs; "d" = the row below, "u" = the row above
-                const f2 wc = P2(W[a0], W[a1]);
-                const f2 huc = P2(HU[a0], HU[a1]), hvc = P2(HV[a0], HV[a1]);
+                const f2 wc = P2(b[0], b[RW]);
+                const f2 huc = P2(b[HUo], b[HUo + RW]), hvc = P2(b[HVo], b[HVo + RW]);
                 // the bottom of cells (rc, t) and (rc, t+1) from the corner rows t .. t+2
-                const f2 cL0 = P2(Cr[am1], Cr[a0]), cL1 = P2(Cr[a0], Cr[a1]);
-                const f2 cR0 = P2(Cr[am1 + 1], Cr[a0 + 1]), cR1 = P2(Cr[a0 + 1], Cr[a1 + 1]);
+                const f2 cL0 = P2(a[CO + RW], b[CO]), cL1 = P2(b[CO], b[CO + RW]);
+                const f2 cR0 = P2(a[CO + RW + 1], b[CO + 1]), cR1 = P2(b[CO + 1], b[CO + RW + 1]);
                 const f2 BAh = corner_mean4(cL0, cR0, cL1, cR1), BXh = corner_mean2(cR0, cR1);
                 const f2 BYh = corner_mean2(cL1, cR1), BXw = corner_mean2(cL0, cL1), BYs = corner_mean2(cL0, cR0);
                 const f2 h = max2(S2(0.f), sub2(wc, BAh));
-                const f2 dh = P2(dring[a0], dring[a1]), d2 = mul2(dh, dh), d3 = mul2(d2, dh);
-                const f2 dl = P2(dring[a0 - 1], dring[a1 - 1]), dr = P2(dring[a0 + 1], dring[a1 + 1]);
-                const f2 dll = P2(dring[a0 - 2], dring[a1 - 2]), drr = P2(dring[a0 + 2], dring[a1 + 2]);
-                const f2 ddn = P2(dring[am1], dring[a0]), du = P2(dring[a1], dring[a2]);
-                const f2 ddd = P2(dring[am2], dring[am1]), duu = P2(dring[a2], dring[a3]);
+                const f2 dh = P2(db[0], db[RW]), d2 = mul2(dh, dh), d3 = mul2(d2, dh);
+                const f2 dl = P2(db[-1], db[RW - 1]), dr = P2(db[1], db[RW + 1]);
+                const f2 dll = P2(db[-2], db[RW - 2]), drr = P2(db[2], db[RW + 2]);
+                const f2 ddn = P2(da[RW], db[0]), du = P2(db[RW], dd[0]);
+                const f2 ddd = P2(da[0], da[RW]), duu = P2(dd[0], dd[RW]);
                 // eta = w - sea level enters only through differences, where the sea level cancels
-                const f2 ec = wc, el_ = P2(W[a0 - 1], W[a1 - 1]), er = P2(W[a0 + 1], W[a1 + 1]);
-                const f2 ed = P2(W[am1], W[a0]), eu_ = P2(W[a1], W[a2]);
-                const f2 ell = P2(W[a0 - 2], W[a1 - 2]), err = P2(W[a0 + 2], W[a1 + 2]);
-                const f2 edd = P2(W[am2], W[am1]), euu = P2(W[a2], W[a3]);
-                const f2 eul = P2(W[a1 - 1], W[a2 - 1]), eur = P2(W[a1 + 1], W[a2 + 1]);
-                const f2 edl = P2(W[am1 - 1], W[a0 - 1]), edr = P2(W[am1 + 1], W[a0 + 1]);
+                const f2 ec = wc, el_ = P2(b[-1], b[RW - 1]), er = P2(b[1], b[RW + 1]);
+                const f2 ed = P2(a[RW], b[0]), eu_ = P2(b[RW], d[0]);
+                const f2 ell = P2(b[-2], b[RW - 2]), err = P2(b[2], b[RW + 2]);
+                const f2 edd = P2(a[0], a[RW]), euu = P2(d[0], d[RW]);
+                const f2 eul = P2(b[RW - 1], d[-1]), eur = P2(b[RW + 1], d[1]);
+                const f2 edl = P2(a[RW - 1], b[-1]), edr = P2(a[RW + 1], b[1]);
                 const float odx = c.one_over_dx, ody = c.one_over_dy;
                 const float od2x = odx * odx, od3x = od2x * odx, od2y = ody * ody, od3y = od2y * ody;
                 const f2 two = S2(2.f), eight = S2(8.f);
@@ -1178,44 +1203,49 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
                 const f2 f0 = fl[0], f1 = add2(fl[1], s1), f2v = add2(fl[2], s2);
                 const f2 sixth = S2(1.0f / 6.0f);
                 const f2 Fs = mul2(mul2(sixth, dh),
-                                   fma2(ddx, mul2(S2(ody * 0.5f), sub2(P2(HV[a1], HV[a2]), P2(HV[am1], HV[a0]))),
-                                        mul2(ddy, mul2(S2(odx * 0.5f), sub2(P2(HV[a0 + 1], HV[a1 + 1]), P2(HV[a0 - 1], HV[a1 - 1]))))));
+                                   fma2(ddx, mul2(S2(ody * 0.5f), sub2(P2(b[HVo + RW], d[HVo]), P2(a[HVo + RW], b[HVo]))),
+                                        mul2(ddy, mul2(S2(odx * 0.5f), sub2(P2(b[HVo + 1], b[HVo + RW + 1]), P2(b[HVo - 1], b[HVo + RW - 1]))))));
                 const f2 Gs = mul2(mul2(sixth, dh),
-                                   fma2(ddx, mul2(S2(ody * 0.5f), sub2(P2(HU[a1], HU[a2]), P2(HU[am1], HU[a0]))),
-                                        mul2(ddy, mul2(S2(odx * 0.5f), sub2(P2(HU[a0 + 1], HU[a1 + 1]), P2(HU[a0 - 1], HU[a1 - 1]))))));
-                const f2 dt = S2(dtm);
+                                   fma2(ddx, mul2(S2(ody * 0.5f), sub2(P2(b[HUo + RW], d[HUo]), P2(a[HUo + RW], b[HUo]))),
+                                        mul2(ddy, mul2(S2(odx * 0.5f), sub2(P2(b[HUo + 1], b[HUo + RW + 1]), P2(b[HUo - 1], b[HUo + RW - 1]))))));
                 f2 dw, rhu, rhv;
                 f2 wbase = wc;
-                if (euler) {
-                    dw = mul2(dt, f0); rhu = mul2(dt, f1); rhv = mul2(dt, f2v);
-                } else if (!corr && ADAPT) {
-                    // variable-step AB3 (compute.hlsl:766-780) with the member's coefficients
-                    const float* q = M.ab;
-                    const f2 kA = S2(q[0]), A0 = S2(q[1]), A1 = S2(q[2]), A2 = S2(q[3]);
-                    const f2 K0 = S2(q[4]), K1 = S2(q[5]), K2 = S2(q[6]);
-                    const f2 o_x = P2(ho0.x, ho1.x), o_y = P2(ho0.y, ho1.y), o_z = P2(ho0.z, ho1.z), o_w = P2(ho0.w, ho1.w);
-                    const f2 q_x = P2(hoo0.x, hoo1.x), q_y = P2(hoo0.y, hoo1.y), q_z = P2(hoo0.z, hoo1.z), q_w = P2(hoo0.w, hoo1.w);
-                    dw = mul2(kA, fma2(A2, q_x, fma2(A1, o_x, mul2(A0, f0))));
-                    rhu = fma2(kA, fma2(A2, q_y, fma2(A1, o_y, mul2(A0, f1))), fma2(K2, q_w, fma2(K1, o_w, mul2(K0, Fs))));
-                    rhv = fma2(kA, fma2(A2, q_z, fma2(A1, o_z, mul2(A0, f2v))), fma2(K2, goo, fma2(K1, go, mul2(K0, Gs))));
-                } else if (!corr) {
-                    const f2 k12 = S2(dtm * (1.0f / 12.0f));
-                    const f2 o_x = P2(ho0.x, ho1.x), o_y = P2(ho0.y, ho1.y), o_z = P2(ho0.z, ho1.z), o_w = P2(ho0.w, ho1.w);
-                    const f2 q_x = P2(hoo0.x, hoo1.x), q_y = P2(hoo0.y, hoo1.y), q_z = P2(hoo0.z, hoo1.z), q_w = P2(hoo0.w, hoo1.w);
-                    const f2 c23 = S2(23.0f), c16 = S2(-16.0f), c5 = S2(5.0f);
-                    dw = mul2(k12, fma2(c5, q_x, fma2(c16, o_x, mul2(c23, f0))));
-                    rhu = fma2(k12, fma2(c5, q_y, fma2(c16, o_y, mul2(c23, f1))), add2(fma2(S2(-3.f), o_w, mul2(two, Fs)), q_w));
-                    rhv = fma2(k12, fma2(c5, q_z, fma2(c16, o_z, mul2(c23, f2v))), add2(fma2(S2(-3.f), go, mul2(two, Gs)), goo));
-                } else {
-                    const f2 k24 = S2(dtm * (1.0f / 24.0f));
-                    const f2 o_x = P2(ho0.x, ho1.x), o_y = P2(ho0.y, ho1.y), o_z = P2(ho0.z, ho1.z);
-                    const f2 q_x = P2(hoo0.x, hoo1.x), q_y = P2(hoo0.y, hoo1.y), q_z = P2(hoo0.z, hoo1.z);
-                    const f2 p_x = P2(hp0.x, hp1.x), p_y = P2(hp0.y, hp1.y), p_z = P2(hp0.z, hp1.z), p_w = P2(hp0.w, hp1.w);
-                    const f2 c9 = S2(9.f), c19 = S2(19.f), c5 = S2(-5.f);
-                    dw = mul2(k24, add2(fma2(c5, o_x, fma2(c19, p_x, mul2(c9, f0))), q_x));
-                    rhu = add2(fma2(k24, add2(fma2(c5, o_y, fma2(c19, p_y, mul2(c9, f1))), q_y), Fs), P2(-p_w.x, -p_w.y));
-                    rhv = add2(fma2(k24, add2(fma2(c5, o_z, fma2(c19, p_z, mul2(c9, f2v))), q_z), Gs), P2(-gp.x, -gp.y));
+                // what a predictor hands its correctors: 19 f - 5 f_old + f_oldold for w, and for hu and hv
+                // the same by dt/24 less F* (G*)
+                f2 kw = S2(0.f), ku = kw, kv = kw;
+                if (CORR) {
+                    const f2 k9 = S2(dtm * 0.375f);   // dt * 9 / 24
+                    dw = mul2(S2(dtm * (1.0f / 24.0f)), fma2(S2(9.f), f0, cw));
+                    rhu = fma2(k9, f1, add2(Fs, cu));
+                    rhv = fma2(k9, f2v, add2(Gs, cv));
                     wbase = wcur;
+                } else if (euler) {
+                    const f2 dt = S2(dtm);
+                    dw = mul2(dt, f0); rhu = mul2(dt, f1); rhv = mul2(dt, f2v);
+                } else {
+                    const f2 o_x = P2(ho0.x, ho1.x), o_y = P2(ho0.y, ho1.y), o_z = P2(ho0.z, ho1.z), o_w = P2(ho0.w, ho1.w);
+                    const f2 q_x = P2(hoo0.x, hoo1.x), q_y = P2(hoo0.y, hoo1.y), q_z = P2(hoo0.z, hoo1.z), q_w = P2(hoo0.w, hoo1.w);
+                    if (ADAPT) {
+                        // variable-step AB3 (compute.hlsl:766-780) with the member's coefficients
+                        const float* q = M.ab;
+                        const f2 kA = S2(q[0]), A0 = S2(q[1]), A1 = S2(q[2]), A2 = S2(q[3]);
+                        const f2 K0 = S2(q[4]), K1 = S2(q[5]), K2 = S2(q[6]);
+                        dw = mul2(kA, fma2(A2, q_x, fma2(A1, o_x, mul2(A0, f0))));
+                        rhu = fma2(kA, fma2(A2, q_y, fma2(A1, o_y, mul2(A0, f1))), fma2(K2, q_w, fma2(K1, o_w, mul2(K0, Fs))));
+                        rhv = fma2(kA, fma2(A2, q_z, fma2(A1, o_z, mul2(A0, f2v))), fma2(K2, goo, fma2(K1, go, mul2(K0, Gs))));
+                    } else {
+                        const f2 k12 = S2(dtm * (1.0f / 12.0f));
+                        const f2 c23 = S2(23.0f), c16 = S2(-16.0f), c5 = S2(5.0f);
+                        dw = mul2(k12, fma2(c5, q_x, fma2(c16, o_x, mul2(c23, f0))));
+                        rhu = fma2(k12, fma2(c5, q_y, fma2(c16, o_y, mul2(c23, f1))), add2(fma2(S2(-3.f), o_w, mul2(two, Fs)), q_w));
+                        rhv = fma2(k12, fma2(c5, q_z, fma2(c16, o_z, mul2(c23, f2v))), add2(fma2(S2(-3.f), go, mul2(two, Gs)), goo));
+                    }
+                    if (pa.handoff) {
+                        const f2 c19 = S2(19.f), c5 = S2(-5.f), k24 = S2((ADAPT ? M.dt_base : dtm) * (1.0f / 24.0f));
+                        kw = add2(fma2(c5, o_x, mul2(c19, f0)), q_x);
+                        ku = fma2(k24, add2(fma2(c5, o_y, mul2(c19, f1)), q_y), P2(-Fs.x, -Fs.y));
+                        kv = fma2(k24, add2(fma2(c5, o_z, mul2(c19, f2v)), q_z), P2(-Gs.x, -Gs.y));
+                    }
                 }
                 f2 wn = wbase, wl = wlo;
                 if (MIXED) {
@@ -1226,21 +1256,22 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
                 } else {
                     wn = add2(wbase, dw);
                 }
-                if (out_col) {
-                    Wout[e0] = wn.x;
-                    if (MIXED) Lout[e0] = wl.x;
-                    R0[e0] = rhu.x;
-                    R0[e0 + PL] = rhv.x;
-                    HAs[e0] = make_float4(f0.x, f1.x, f2v.x, Fs.x);
-                    HBs[e0] = Gs.x;
-                    if (row1) {
-                        Wout[e1] = wn.y;
-                        if (MIXED) Lout[e1] = wl.y;
-                        R0[e1] = rhu.y;
-                        R0[e1 + PL] = rhv.y;
-                        HAs[e1] = make_float4(f0.y, f1.y, f2v.y, Fs.y);
-                        HBs[e1] = Gs.y;
+                auto put = [&](size_t e, float w, float l, float ru, float rv, float4 ha, float hb, float3 hc) {
+                    Wout[e] = w;
+                    if (MIXED) Lout[e] = l;
+                    R0[e] = ru;
+                    R0[e + PL] = rv;
+                    if (!CORR && pa.handoff) {
+                        HCs[e] = hc.x; HCs[e + PL] = hc.y; HCs[e + 2 * PL] = hc.z;
+                    } else {
+                        HAs[e] = ha;
+                        HBs[e] = hb;
                     }
+                };
+                if (out_col) {
+                    put(e0, wn.x, wl.x, rhu.x, rhv.x, make_float4(f0.x, f1.x, f2v.x, Fs.x), Gs.x, make_float3(kw.x, ku.x, kv.x));
+                    if (row1)
+                        put(e1, wn.y, wl.y, rhu.y, rhv.y, make_float4(f0.y, f1.y, f2v.y, Fs.y), Gs.y, make_float3(kw.y, ku.y, kv.y));
                 }
                 if (stats) {   // GetStats (compute.hlsl:1319-1378) of the input state
                     const f2 q = div_by_h2(h, c.epsilon);
@@ -1273,8 +1304,10 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
             // the y flux through the north face of row t+1 is the south flux of the next pair's first row
             ypv[0] = yf[0].y; ypv[1] = yf[1].y; ypv[2] = yf[2].y;
             fp.set(f);
+            sm = s0; s0 = s2; s2 = s4;
+            s4 = next_slot(s4);
         }
-        seq = seq0 + unsigned(last_row - (y0 - 2) + 1);
+        seq = seq0 + unsigned(npairs);
         // ---- zero the ghost ring of the output state next to this strip (engine.cpp:1007) ----
         const int NX = c.NX, NY = c.NY;
         const bool west = x0 == 2, east = x0 + (TW - 2) >= nx + 2, south = y0 == 2, north = y0 + MH >= ny + 2;
@@ -1318,7 +1351,7 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
         }
     }
     if (__syncthreads_or(tma_late) && tid == 0) {
-        drain_ring(bars, RING2, requested);
+        drain_ring(bars, PRING, requested);
         atomic_max_nonneg(pa.late_flag, 1.0);
     }
 }
@@ -2781,20 +2814,25 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-// Row map of one NX x NY plane with pitch P floats: boxes of RBOX x 1 floats; reads outside
-// the plane return zero, like the reference's out-of-range texture loads.
-int encode_row_map(CUtensorMap* m, const float* plane, int NX, int NY, int P, std::string& err, int box_w = RBOX) {
+// Map of `planes` NX x NY planes with pitch P floats, `plane` floats apart: boxes of box_w x box_h floats
+// of every plane; reads outside a plane return zero, like the reference's out-of-range texture loads.
+int encode_map(CUtensorMap* m, const float* base, int NX, int NY, int P, int planes, size_t plane, int box_w, int box_h,
+               std::string& err) {
     auto enc = tensor_map_encoder();
     if (!enc) { err = "cuTensorMapEncodeTiled unavailable"; return CEL_ERR_CUDA; }
-    cuuint64_t dims[2] = {cuuint64_t(NX), cuuint64_t(NY)};
-    cuuint64_t strides[1] = {cuuint64_t(P) * sizeof(float)};
-    cuuint32_t box[2] = {cuuint32_t(box_w), 1u};
-    cuuint32_t estr[2] = {1u, 1u};
-    CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(plane), dims, strides, box, estr,
+    cuuint64_t dims[3] = {cuuint64_t(NX), cuuint64_t(NY), cuuint64_t(planes)};
+    cuuint64_t strides[2] = {cuuint64_t(P) * sizeof(float), cuuint64_t(plane) * sizeof(float)};
+    cuuint32_t box[3] = {cuuint32_t(box_w), cuuint32_t(box_h), cuuint32_t(planes)};
+    cuuint32_t estr[3] = {1u, 1u, 1u};
+    CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, planes > 1 ? 3 : 2, const_cast<float*>(base), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { err = "cuTensorMapEncodeTiled failed (" + std::to_string(int(r)) + ")"; return CEL_ERR_CUDA; }
     return CEL_OK;
+}
+// Row map of one plane: boxes of RBOX x 1 floats (k_march).
+int encode_row_map(CUtensorMap* m, const float* plane, int NX, int NY, int P, std::string& err) {
+    return encode_map(m, plane, NX, NY, P, 1, 0, RBOX, 1, err);
 }
 
 int dalloc(cel_lane* b, void** ptr, size_t bytes, std::string& err) {
@@ -2869,12 +2907,15 @@ ColsKernel cols_kernel(bool mixed, int cw, int nt) {
 }
 
 using March2Kernel = void (*)(const MemberDev*, const int4*, int, PassArgs);
-March2Kernel march2_kernel(bool mixed, bool adapt, int w) {
-    if (w == 96)
-        return mixed ? (adapt ? k_march2<true, true, 96> : k_march2<true, false, 96>)
-                     : (adapt ? k_march2<false, true, 96> : k_march2<false, false, 96>);
-    return mixed ? (adapt ? k_march2<true, true, 128> : k_march2<true, false, 128>)
-                 : (adapt ? k_march2<false, true, 128> : k_march2<false, false, 128>);
+size_t march2_smem(int w) { return w == 96 ? PairRing<96>::SMEM : PairRing<128>::SMEM; }
+template <int KIND>
+March2Kernel march2_kernel_kind(bool mixed, int w) {
+    if (w == 96) return mixed ? k_march2<true, KIND, 96> : k_march2<false, KIND, 96>;
+    return mixed ? k_march2<true, KIND, 128> : k_march2<false, KIND, 128>;
+}
+March2Kernel march2_kernel(bool mixed, int kind, int w) {
+    return kind == PASS_CORRECTOR ? march2_kernel_kind<PASS_CORRECTOR>(mixed, w)
+           : kind == PASS_ADAPTIVE ? march2_kernel_kind<PASS_ADAPTIVE>(mixed, w) : march2_kernel_kind<PASS_FIXED>(mixed, w);
 }
 
 int launch_pass(cel_lane* b, const PassArgs& pa, std::string& err) {
@@ -2885,7 +2926,8 @@ int launch_pass(cel_lane* b, const PassArgs& pa, std::string& err) {
         TimedLaunch t(&b->tm, b->stream, "fused_stencil");
         const bool ad = pa.scheme == CEL_SCHEME_PREDICTOR_ADAPTIVE;
         if (b->rows_per_step == 2) {
-            march2_kernel(b->mixed, ad, b->mw)<<<b->grid_stencil, b->mw, MARCH2_DYN_SMEM, b->stream>>>(
+            const int kind = pa.scheme == CEL_SCHEME_CORRECTOR ? PASS_CORRECTOR : ad ? PASS_ADAPTIVE : PASS_FIXED;
+            march2_kernel(b->mixed, kind, b->mw)<<<b->grid_stencil, b->mw, march2_smem(b->mw), b->stream>>>(
                 b->ddev, b->mtiles, b->nmtiles, pa);
         } else {
             auto* k = b->mixed ? (ad ? k_march<true, true> : k_march<true, false>)
@@ -3025,6 +3067,7 @@ int run_pass(cel_lane* b, bool first_of_step, std::string& err) {
     }
     pa.og = ix.og; pa.oog = ix.oog; pa.scr = ix.scr; pa.pred = ix.pred;
     pa.stats = first_of_step ? 1 : 0;
+    pa.handoff = s.is_predictor() && s.N > 0 ? 1 : 0;
     pa.friction = b->any_friction ? 1 : 0;
     pa.late_flag = b->late_flag;
     pa.spart = b->spart;
@@ -3290,13 +3333,14 @@ int configure_work(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::st
         B_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kc, nt, smem_cols));
         b->grid_cols = std::max(1, std::min(b->nbands, b->sms * std::max(occ, 1) * 4));
     }
-    // both variants of the stencil (fixed and adaptive predictor) run on the same grid
+    // every kind of pass runs on the same grid
     if (b->rows_per_step == 2) {
         occ = 1 << 20;
-        for (auto* k2 : {march2_kernel(b->mixed, false, mw), march2_kernel(b->mixed, true, mw)}) {
+        for (int kind : {PASS_FIXED, PASS_ADAPTIVE, PASS_CORRECTOR}) {
+            March2Kernel k2 = march2_kernel(b->mixed, kind, mw);
             int o = 0;
             B_TRY(allow_max_dynamic_smem(reinterpret_cast<const void*>(k2)));
-            B_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k2, mw, MARCH2_DYN_SMEM));
+            B_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k2, mw, march2_smem(mw)));
             occ = std::min(occ, o);
         }
     } else {
@@ -3406,6 +3450,7 @@ cel_lane* lane_create(int n, const cel_params* const* params, const float* const
         d.g64 = m.p.gravity;
         b->dt_host[i] = float(m.p.timestep);
         d.dtp = b->dt_table + i;
+        d.dt_base = b->dt_host[i];
         d.ab = b->ctl ? b->ctl[i].ab : nullptr;
         // planes: state 9 (+9 lo), bottom 3, rhs 2, history 12 + 8, aux 2, factors 6
         const int nplanes = 9 + (b->mixed ? 9 : 0) + 3 + 2 + 12 + 8 + 2 + 6;
@@ -3441,7 +3486,7 @@ cel_lane* lane_create(int n, const cel_params* const* params, const float* const
             for (int k = 0; k < 3; ++k) d.FYB[k] = static_cast<float*>(fp_) + k * nbm;
         }
         {   // TMA row maps: the three state buffers (w, hu, hv), then BA, BX, BY
-            std::vector<CUtensorMap> maps(13);
+            std::vector<CUtensorMap> maps(13 + 8);
             for (int sb = 0; sb < 3; ++sb)
                 for (int k = 0; k < 3; ++k)
                     if (encode_row_map(&maps[sb * 3 + k], d.S[sb][k], NX, NY, m.P, err)) return nullptr;
@@ -3453,10 +3498,17 @@ cel_lane* lane_create(int n, const cel_params* const* params, const float* const
             void* cp_ = nullptr;
             if (dalloc(b.get(), &cp_, sizeof(float) * size_t(d.PC) * (NY + 1), err)) return nullptr;
             d.CORN = static_cast<float*>(cp_);
-            if (encode_row_map(&maps[12], d.CORN, NX + 1, NY + 1, d.PC, err, CBOX)) return nullptr;
+            // the row-pair maps of k_march2 (128 and 96 threads): a state buffer's three planes as one 3-D
+            // tensor, and the corner grid
+            for (int wi = 0; wi < 2; ++wi) {
+                const int box = wi == 0 ? PairRing<128>::BOX : PairRing<96>::BOX;
+                for (int sb = 0; sb < 3; ++sb)
+                    if (encode_map(&maps[13 + 4 * wi + sb], d.S[sb][0], NX, NY, m.P, 3, m.plane, box, 2, err)) return nullptr;
+                if (encode_map(&maps[13 + 4 * wi + 3], d.CORN, NX + 1, NY + 1, d.PC, 1, 0, box, 2, err)) return nullptr;
+            }
             void* mp = nullptr;
-            if (dalloc(b.get(), &mp, sizeof(CUtensorMap) * 13, err)) return nullptr;
-            if (cudaMemcpy(mp, maps.data(), sizeof(CUtensorMap) * 13, cudaMemcpyHostToDevice) != cudaSuccess) {
+            if (dalloc(b.get(), &mp, sizeof(CUtensorMap) * maps.size(), err)) return nullptr;
+            if (cudaMemcpy(mp, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
                 err = "tensor map upload failed";
                 return nullptr;
             }
