@@ -176,10 +176,6 @@ __device__ void stats_reduce(double* acc, bool cnt_block, bool cnt_all, float h,
 #define CEL_MARCH_MIN_CTAS 5
 #endif
 constexpr int MARCH_MIN_CTAS = CEL_MARCH_MIN_CTAS;
-#ifndef CEL_MARCH2_MIN_CTAS
-#define CEL_MARCH2_MIN_CTAS 3
-#endif
-constexpr int MARCH2_MIN_CTAS = CEL_MARCH2_MIN_CTAS;   // the paired-row stencil (49.6 KB smem, 166 registers)
 constexpr int MW = 128;          // threads = columns with faces per row
 constexpr int MO = MW - 2;       // output columns per strip
 constexpr int MH_DEFAULT = 64;   // rows per strip unless tuned (each work item carries its height)
@@ -745,7 +741,7 @@ __global__ void __launch_bounds__(MW, MARCH_MIN_CTAS) k_march(const MemberDev* _
 //
 // The ring holds row pairs: one 3-D TMA box brings w, hu and hv of rows t, t+1, a second one the two
 // corner-grid rows above them (the bottom BA, BX, BY is rebuilt from the corners), onto one mbarrier.
-// A step's window is the pairs t-2 .. t+4, and the pair t+6 is requested a step ahead: PRING = 5 slots.
+// A step's window is the pairs t-2 .. t+4; the pair t+6 is on its way and t+8 is requested: PRING = 6.
 // Every shared-memory operand is one of four slot addresses plus a compile-time offset (the 9-row ring
 // before it took a remainder per row and 8 copies a step: without a corrector, 6.6 M cells at 123 -> 117 us
 // a launch).
@@ -758,10 +754,15 @@ __global__ void __launch_bounds__(MW, MARCH_MIN_CTAS) k_march(const MemberDev* _
 // 1.482 -> 1.374.  What the correctors add up is rounded once more than before (the combination, relative
 // 2^-24), as the rates themselves were; the states' distance from 64 bits is unchanged.
 // ---------------------------------------------------------------------------------------------
-// CTAs per SM the paired-row stencil is built for: 3 of 128 threads or 4 of 96 (12 warps either
-// way, within the register file at up to 168 registers per thread)
-constexpr int march2_min_ctas(int w) { return w == 128 ? MARCH2_MIN_CTAS : 4; }
-constexpr int PRING = 5;
+// CTAs per SM the paired-row stencil is built for: 4 of 128 threads or 5 of 96 (16 and 15 warps at 128
+// registers).  Its warps wait on each other's arithmetic more than on memory (issue slots were 59 % used
+// with 12 warps of 168 registers an SM, 66 % with 16, tail included), so warps count: 2048 x 2048 cells
+// 165 -> 138 us a launch, 28 members 1374 -> 1338 us a step.  Two changes made room: the statistics add up
+// in FP64 (one register pair a sum instead of two compensated pairs), and a single barrier a step, which
+// lets the warps of a CTA drift through Pass3 of one step and the faces of the next.  With two barriers
+// and compensated sums the same bound spilled 188 bytes a thread and the step took 1418 us.
+constexpr int march2_min_ctas(int w) { return w == 128 ? 4 : 5; }
+constexpr int PRING = 6;
 template <int TW>
 struct PairRing {
     static constexpr int BOX = TW + 8;                          // floats of a row: columns x0-2 .. x0+TW, from a
@@ -909,18 +910,6 @@ __device__ __forceinline__ void face_flux2(f2 hm, f2 um, f2 vm, f2 wm, f2 hp, f2
     for (int k = 0; k < 3; ++k) out[k] = mul2(fma2(apam, dU[k], sub2(mul2(ap, Fm[k]), mul2(am, Fp[k]))), inv);
 }
 
-// Kahan accumulation of a pair of rows
-struct Kahan2 {
-    f2 s = make_float2(0.f, 0.f), c = make_float2(0.f, 0.f);
-    __device__ __forceinline__ void add(f2 x) {
-        const f2 y = sub2(x, c);
-        const f2 t = add2(s, y);
-        c = sub2(sub2(t, s), y);
-        s = t;
-    }
-    __device__ __forceinline__ double value() const { return (double(s.x) - double(c.x)) + (double(s.y) - double(c.y)); }
-};
-
 template <bool MIXED, int KIND, int TW>
 __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const MemberDev* __restrict__ mems,
                                                                const int4* __restrict__ tiles, int ntiles, PassArgs pa) {
@@ -931,7 +920,7 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
     __shared__ float dring[PRING * DSLOT];  // still-water depth of the ring's rows
     __shared__ __align__(8) unsigned long long bars[PRING];
     __shared__ float fW[2][2][4][TW];       // [step parity][row of the pair][hW, uW, vW, wW][thread]
-    __shared__ float xb[2][3][TW];          // [row of the pair][component][thread]
+    __shared__ float xb[2][2][3][TW];       // [step parity][row of the pair][component][thread]
     constexpr int OFF = MIXED ? 18 : 9;
     constexpr int iR0 = OFF + 3, iH0 = OFF + 5, iAUX = OFF + 25;
     const int tid = threadIdx.x;
@@ -1024,9 +1013,9 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
             if (tid < 2) at(d2c);
         };
 
-        Kahan2 acc[5];
+        double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
         double mfull = 0.0;
-        f2 mx[4] = {S2(0.f), S2(0.f), S2(0.f), S2(0.f)};
+        float mx[4] = {0.f, 0.f, 0.f, 0.f};
         bool bad = false;
         // aux texels this thread owns: the ghost texels x = 1 / y = 1 go with column / row 2
         const int cxa = max(xc, 2);
@@ -1040,7 +1029,7 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
         __syncthreads();  // the previous strip is done with shared memory
         if (tid == 0) {
             fence_proxy_async();
-            for (int k = 0; k < 3; ++k) issue(k);   // pairs of the prologue and step -1
+            for (int k = 0; k < min(4, npairs); ++k) issue(k);   // pairs of the prologue and the steps -1 and 0
         }
         auto next_slot = [](int k) { return k + 1 == PRING ? 0 : k + 1; };
         const int sA = int(seq0 % PRING), sB = next_slot(sA), sC = next_slot(sB);
@@ -1066,6 +1055,7 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
             }
             fp.set(fq);
         }
+        __syncthreads();   // the prologue's west faces and depths are there
         // slots of the pairs t-2, t, t+2, t+4; at step -1 (t = y0 - 2) the pair t-2 is not used
         int sm = sZ, s0 = sA, s2 = sB, s4 = sC;
 
@@ -1097,11 +1087,6 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
             float2* const ap0 = AUX + (size_t(min(t + 2, NYm1)) * P + xc);
             float2* const ap1 = AUX + (size_t(min(t + 3, NYm1)) * P + xc);
             const float2 old0 = aux0 ? *ap0 : make_float2(0.f, 0.f), old1 = aux1 ? *ap1 : make_float2(0.f, 0.f);
-            __syncthreads();  // (A) the previous step is complete: the slot of pair t-4 is free
-            if (tid == 0 && j + 4 < npairs) {
-                fence_proxy_async();
-                issue(j + 4);        // the pair t + 6
-            }
             wait_pair(j + 3);        // the pair t + 4
             depth_pair(s2, s4, false);
             const float* const q0 = ring + s0 * SLOT;
@@ -1129,9 +1114,16 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
                            P2(fW[par][0][1][tn], fW[par][1][1][tn]), P2(fW[par][0][2][tn], fW[par][1][2][tn]),
                            P2(fW[par][0][3][tn], fW[par][1][3][tn]), g, hg, true, xo);
 #pragma unroll
-                for (int k = 0; k < 3; ++k) { xb[0][k][tid] = xo[k].x; xb[1][k][tid] = xo[k].y; }
+                for (int k = 0; k < 3; ++k) { xb[par][0][k][tid] = xo[k].x; xb[par][1][k][tid] = xo[k].y; }
             }
-            __syncthreads();  // (B)
+            // The one barrier of a step: this step's fluxes and depths are there, and every thread is done with
+            // Pass3 of the step before, so the slot of pair t-4 is free.  (What a thread writes past it goes
+            // to the other parity of fW and xb and to slots that Pass3 does not read.)
+            __syncthreads();
+            if (tid == 0 && j + 5 < npairs) {
+                fence_proxy_async();
+                issue(j + 5);        // the pair t + 8
+            }
             // ---- Pass3 at (xc, t) and (xc, t+1) ----
             if (p3) {
                 // this column in the pairs t-2, t, t+2 (index RW: the second row)
@@ -1196,7 +1188,7 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
                 for (int k = 0; k < 3; ++k) {
                     // x fluxes: west face (the neighbour's east face) minus east face; y fluxes: the
                     // south faces of rows t, t+1 are the north faces of rows t-1, t
-                    const f2 xw = P2(xb[0][k][tw], xb[1][k][tw]), xh = P2(xb[0][k][tid], xb[1][k][tid]);
+                    const f2 xw = P2(xb[par][0][k][tw], xb[par][1][k][tw]), xh = P2(xb[par][0][k][tid], xb[par][1][k][tid]);
                     const f2 ys = P2(ypv[k], yf[k].x);
                     fl[k] = fma2(sub2(xw, xh), S2(odx), mul2(sub2(ys, yf[k]), S2(ody)));
                 }
@@ -1279,20 +1271,21 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
                     const bool in_cols = out_col && xc < 2 + 4 * (nx / 4);
                     const bool b0 = in_cols && t < 2 + 4 * (ny / 4), b1 = in_cols && row1 && t + 1 < 2 + 4 * (ny / 4);
                     const bool a0_ = out_col, a1_ = out_col && row1;
-                    auto pick = [](bool k0, bool k1, f2 v_) { return P2(k0 ? v_.x : 0.f, k1 ? v_.y : 0.f); };
+                    auto add = [&](double& s_, f2 v_) { if (b0) s_ += double(v_.x); if (b1) s_ += double(v_.y); };
+                    auto top = [&](float& m_, f2 v_) { m_ = fmaxf(m_, fmaxf(b0 ? v_.x : 0.f, b1 ? v_.y : 0.f)); };
                     const f2 u2v2 = fma2(u, u, mul2(v, v));
                     const f2 cc = P2(sqrtf(c.g * h.x), sqrtf(c.g * h.y));
-                    acc[0].add(pick(b0, b1, h));
-                    acc[1].add(pick(b0, b1, mul2(h, fma2(S2(0.5f), h, BAh))));
-                    acc[2].add(pick(b0, b1, huc));
-                    acc[3].add(pick(b0, b1, hvc));
-                    acc[4].add(pick(b0, b1, fma2(huc, u, mul2(hvc, v))));
-                    mx[0] = max2(mx[0], pick(b0, b1, u2v2));
-                    mx[1] = max2(mx[1], pick(b0, b1, h));
+                    add(acc[0], h);
+                    add(acc[1], mul2(h, fma2(S2(0.5f), h, BAh)));
+                    add(acc[2], huc);
+                    add(acc[3], hvc);
+                    add(acc[4], fma2(huc, u, mul2(hvc, v)));
+                    top(mx[0], u2v2);
+                    top(mx[1], h);
                     const f2 cx = mul2(add2(P2(fabsf(u.x), fabsf(u.y)), cc), S2(odx));
                     const f2 cy = mul2(add2(P2(fabsf(v.x), fabsf(v.y)), cc), S2(ody));
-                    mx[2] = max2(mx[2], pick(b0, b1, max2(cx, cy)));
-                    mx[3] = max2(mx[3], pick(b0, b1, mul2(u2v2, q)));
+                    top(mx[2], max2(cx, cy));
+                    top(mx[3], mul2(u2v2, q));
                     // volume in FP64 from the compensated state (w + its low word)
                     if (a0_) mfull += fmax(0.0, double(wc.x) - double(BAh.x) + (MIXED ? double(wlo.x) : 0.0));
                     if (a1_) mfull += fmax(0.0, double(wc.y) - double(BAh.y) + (MIXED ? double(wlo.y) : 0.0));
@@ -1327,9 +1320,9 @@ __global__ void __launch_bounds__(TW, march2_min_ctas(TW)) k_march2(const Member
         }
         if (stats) {
             double sv[STATS_N];
-            for (int k = 0; k < 5; ++k) sv[k] = acc[k].value();
+            for (int k = 0; k < 5; ++k) sv[k] = acc[k];
             sv[5] = mfull;
-            for (int k = 0; k < 4; ++k) sv[6 + k] = fmaxf(mx[k].x, mx[k].y);
+            for (int k = 0; k < 4; ++k) sv[6 + k] = mx[k];
             sv[10] = bad ? 1.0 : 0.0;
             sv[11] = 0.0;
             for (int off = 16; off; off >>= 1)
@@ -2788,7 +2781,8 @@ struct cel_lane {
     bool col_tt = false;                // tile-transposed column solver (band width 16, "1 chunk")
     int mh = cel::MH_DEFAULT;           // stencil strip height (rows per CTA work item)
     int rows_per_step = 2;              // stencil rows per thread step: 1 (k_march) or 2 (k_march2)
-    int mw = 96;                        // stencil CTA width in threads (k_march2: 128 or 96)
+    int mw = 128;                       // stencil CTA width in threads (k_march2: 128 or 96)
+    bool mw_auto = true;                // ... by strip_split, until it is selected
     bool rows_chosen = false;           // the caller selected the stencil variant (lane_set_stencil_rows)
     std::vector<std::pair<int, int>> batch_sizes;   // (nx, ny) of every member of the batch, all lanes
     int max_nx = 0, max_ny = 0;
@@ -3176,41 +3170,48 @@ cudaError_t allow_max_dynamic_smem(const void* kernel) {
     return e;
 }
 
-// The strip height of a batch's stencil: at most mh_max rows, fewer where taller strips would leave
-// SMs idle.  A strip is a serial chain of row steps, so a batch with fewer strips than CTA slots takes
-// as long as one strip, and one with a few strips more than a whole number of waves takes a wave
-// more.  The cost of a height h is modelled as
+// The split of a batch's stencil: a strip height of at most mh_max rows, lower where taller strips would
+// leave SMs idle, and, with mw 0, the strip width (128 or 96 threads).  A strip is a serial chain of row
+// steps, so a batch with fewer strips than CTA slots takes as long as one strip, and one with a few
+// strips more than a whole number of waves takes a wave more.  The cost of a split is modelled as
 //   sum over waves of (row steps of a strip + PRO) x step(CTAs per SM in that wave),
-// where a step takes STEP_US alone on its SM (latency) and n x RATE_US with n CTAs beside it
-// (issue), and PRO steps stand for the prologue (filling the ring, the first faces).  Measured with
-// the paired-row stencil at 96 threads: 2.06 us a step on an idle GPU (512 x 64 cells, heights 8 to
-// 64) and 4.2 us at four CTAs an SM (16 M cells); the one-row stencil 1.5 and 3.6 (at five).
-// Against 64-row strips, ms per step: 512 x 64 cells 0.185 -> 0.068 (8 rows), 1024 x 1024 0.261 ->
-// 0.181 (24), 40 members of 128..512 a side 0.553 -> 0.522 (48); 16 M cells keep 64 rows (1.497;
-// 32 rows 1.515).  Heights change the split of the work, never a cell's arithmetic; every lane of a
-// batch takes the height of the whole batch, so the statistics do not depend on the lanes either.
-int strip_height(const cel_lane* b, int mo, int rps, int mw, int mh_max) {
-    constexpr int H_MIN = 8;
+// step(n) = BASE + n x RATE (latency, and the share of the SM that n CTAs have), PRO steps standing for
+// the prologue (filling the ring, the first faces).  Measured with the paired-row stencil at 128
+// threads: about 1.8 us a step with one CTA on an SM, 2.5 with two, 4.0 with the four that fit; at
+// 96 threads 3.8 with five.  Over nine batches of 32 thousand to 16 million cells and heights of 4 to 96
+// rows the choice costs 0.7 % more than the best height and width found by trying; us per step against
+// 64-row strips of 96 threads: 512 x 64 cells 158 -> 60 (4 rows), 1024 x 1024 250 -> 176 (16 rows of 128
+// threads), 40 members of 128..512 a side 517 -> 475 (40); 16 M cells keep 64 rows (128 threads 1338,
+// 96 1346; 32 rows 1368).  Splits change no cell's arithmetic; every lane takes the split of the whole
+// batch, so the statistics do not depend on the lanes either.
+int strip_split(const cel_lane* b, int rps, int& mw, int mh_max) {
+    constexpr int H_MIN = 4;
     constexpr double PRO = 2.5;
-    const int slots = rps == 1 ? MARCH_MIN_CTAS : march2_min_ctas(mw);
-    const double step_us = rps == 1 ? 1.5 : 2.1;
-    const double rate_us = (rps == 1 ? 3.6 : 4.2) / slots;
-    auto step = [&](double n) { return std::max(step_us, n * rate_us); };
-    const double sms = b->sms;
-    int best = mh_max;
+    int best = mh_max, best_w = mw ? mw : MW;
     double best_t = 1e300;
-    for (int h = std::min(H_MIN, mh_max);; h = std::min(h + 2, mh_max)) {
-        long long strips = 0;
-        for (const auto& m : b->batch_sizes) strips += (long long)((m.first + mo - 1) / mo) * ((m.second + h - 1) / h);
-        const double per_sm = std::ceil(strips / sms);
-        const double whole = std::floor(per_sm / slots), rest = per_sm - whole * slots;
-        const double t = ((h + rps - 1) / rps + PRO) * (whole * step(slots) + (rest > 0 ? step(rest) : 0.0));
-        if (t <= best_t) { best_t = t; best = h; }   // the taller of two equals: fewer prologues
-        if (h == mh_max) break;
+    for (int w : {128, 96}) {
+        if (mw && w != mw) continue;
+        const int mo = w - 2, slots = rps == 1 ? MARCH_MIN_CTAS : march2_min_ctas(w);
+        const double base_us = rps == 1 ? 0.9 : 1.0, rate_us = rps == 1 ? 0.54 : w == 128 ? 0.8 : 0.64;
+        auto step = [&](double n) { return n > 0 ? base_us + n * rate_us : 0.0; };
+        for (int h = std::min(H_MIN, mh_max);; h = std::min(h + 2, mh_max)) {
+            long long strips = 0;
+            for (const auto& m : b->batch_sizes) strips += (long long)((m.first + mo - 1) / mo) * ((m.second + h - 1) / h);
+            const double per_sm = std::ceil(strips / double(b->sms)), whole = std::floor(per_sm / slots);
+            const double t = ((h + rps - 1) / rps + PRO) * (whole * step(slots) + step(per_sm - whole * slots));
+            if (t < best_t || (t == best_t && w == best_w)) {   // the taller of two equals: fewer prologues
+                best_t = t;
+                best = h;
+                best_w = w;
+            }
+            if (h == mh_max) break;
+        }
     }
+    mw = best_w;
     return best;
 }
 
+// mw 0: the stencil width by strip_split.
 int configure_work(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::string& err) {
     // 32-column bands with 32, 64 or 128 chunks per column (nt = chunks x 32 = 1024, 2048, 4096):
     // the cluster solver, 8 chunks per CTA and nt / 256 CTAs per cluster
@@ -3246,10 +3247,9 @@ int configure_work(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::st
         }
     }
     if (rps != 1 && rps != 2) { err = "stencil rows per step must be 1 or 2"; return CEL_ERR_ARG; }
-    if (mw != 128 && mw != 96) { err = "stencil width must be 128 or 96 threads"; return CEL_ERR_ARG; }
+    if (mw != 0 && mw != 128 && mw != 96) { err = "stencil width must be 128 or 96 threads"; return CEL_ERR_ARG; }
     if (rps == 1) mw = MW;   // the one-row stencil has one width
     b->rows_per_step = rps;
-    const int mo = mw - 2;   // output columns per strip
     if (cw != 1 && cw != 8 && cw != 16 && cw != 32) { err = "column band width must be 1, 8, 16 or 32"; return CEL_ERR_ARG; }
     if (mh < 8 || mh > 1024) { err = "strip height must be in [8, 1024]"; return CEL_ERR_ARG; }
     const size_t smem_cols = tt ? sizeof(float) * size_t(TT_CW) * size_t((b->max_ny + 3) & ~3)
@@ -3257,7 +3257,8 @@ int configure_work(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::st
     if (smem_cols + COLS_STATIC_SMEM > 227 * 1024) { err = "column band too wide for the tallest member (shared memory)"; return CEL_ERR_ARG; }
     std::vector<int4> mt;
     std::vector<int2> bd, mr;
-    const int sh = strip_height(b, mo, rps, mw, mh);
+    const bool mw_auto = mw == 0;
+    const int sh = strip_split(b, rps, mw, mh), mo = mw - 2;   // strip height, output columns per strip
     for (int i = 0; i < int(b->mem.size()); ++i) {
         const HostSetup& hs = b->mem[i].hs;
         // a member's strips as equal as whole steps allow
@@ -3308,6 +3309,7 @@ int configure_work(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::st
     b->cnt = nt;
     b->mh = mh;
     b->mw = mw;
+    b->mw_auto = mw_auto;
     b->smem_cols = smem_cols;
     b->col_cl = cl;
     b->col_tt = tt;
@@ -3637,7 +3639,7 @@ cel_lane* lane_create(int n, const cel_params* const* params, const float* const
     }
     {   // column bands of 16 columns (8 for tall domains: shared-memory capacity), strips of 64 rows
         const int cw = (size_t(max_ny) * 16 * sizeof(float) + COLS_STATIC_SMEM <= 227 * 1024) ? 16 : 8;
-        if (configure_work(b.get(), cw, MH_DEFAULT, b->rows_per_step, b->mw, NTC_DEFAULT, err)) return nullptr;
+        if (configure_work(b.get(), cw, MH_DEFAULT, b->rows_per_step, 0, NTC_DEFAULT, err)) return nullptr;
     }
     b->sch.reset(*params[0]);
     cudaMemcpy(b->dt_table, b->dt_host, sizeof(float) * n, cudaMemcpyHostToDevice);
@@ -3949,7 +3951,7 @@ int lane_set_tuning(cel_lane* b, int tx, int ty, int pcr, std::string& err) {
     // swept serially), so the CTA has pcr x band width threads; 0 keeps the threads per CTA
     const int cw = tx > 0 ? tx : b->cw;
     const int nt = (pcr > 0 && cw > 1) ? pcr * cw : b->cnt;
-    return configure_work(b, cw, ty > 0 ? ty : b->mh, b->rows_per_step, b->mw, nt, err);
+    return configure_work(b, cw, ty > 0 ? ty : b->mh, b->rows_per_step, b->mw_auto ? 0 : b->mw, nt, err);
 }
 
 int lane_get_tuning(const cel_lane* b, int* tx, int* ty, int* rps) {
