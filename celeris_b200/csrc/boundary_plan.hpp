@@ -27,6 +27,15 @@ inline int corner_side(int corner, int q) {
 // A corner is one CTA's work: larger ones (two very wide sponges) are left to one launch per side.
 constexpr int BND_CORNER_MAX = 16384;
 
+// How a corner may be cut into pieces that take its two sides independently: a wall reads texels along its
+// own axis only, and every other kind the texel itself.
+enum CornerCut { CUT_NONE, CUT_ROWS, CUT_COLUMNS };
+inline CornerCut corner_cut(int corner, const int type[4]) {
+    const int a = corner_side(corner, 0), b = corner_side(corner, 1);
+    const int xside = (a == 1 || a == 3) ? a : b, yside = a + b - xside;
+    return type[yside] != CEL_BC_SOLID ? CUT_ROWS : type[xside] != CEL_BC_SOLID ? CUT_COLUMNS : CUT_NONE;
+}
+
 // Fills the eight rectangles (empty ones have no texels); false where the sides have to be launched
 // one after another: walls wide enough to read their own strip (W, S from 3, E, N from 4 cells), or
 // a domain so small that opposite corners meet.

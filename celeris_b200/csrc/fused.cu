@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "batch.hpp"
+#include "boundary_plan.hpp"
 #include "device_math.cuh"
 #include "engine_iface.hpp"
 #include "readback.hpp"
@@ -89,6 +90,7 @@ struct MemberDev {
                             // (b * ny + i) * band width + c
     int PC;
     BoundaryDesc bd[4];     // N, E, S, W
+    Rect breg[BND_REGIONS]; // regions of the one-launch boundary, where the sides allow it
     const float4* waves;
     const double* waves64;  // the same components in FP64, 4 per component (compensated form)
     const float* uts[4];    // (t, eta, hu, hv) tables, float
@@ -2327,180 +2329,221 @@ __host__ __device__ __forceinline__ int boundary_item_cells(int type) {
     return type == CEL_BC_SPONGE ? BND_CELLS : type == CEL_BC_IRREGULAR ? BND_IRR_CELLS : 256;
 }
 
+// One work item of side `side`: boundary_item_cells cells from `first` on of the rectangle (x0, y0, sw, sh).
+// phase 0: compute and write in place; 1: compute into the member's scratch; 2: copy back.
+template <bool MIXED>
+__device__ __noinline__ void boundary_item(const MemberDev& M, int side, int phase, int out, int x0, int y0, int sw, int sh,
+                                              int first) {
+    constexpr int SS = MIXED ? 6 : 3;   // strip floats per cell: w, hu, hv (+ their low words)
+    const SimConsts c = M.c;
+    const BoundaryDesc& b = M.bd[side];
+    const int NX = c.NX, NY = c.NY, P = M.P;
+    float* W = M.S[out][0];
+    float* HU = M.S[out][1];
+    float* HV = M.S[out][2];
+    float* LW = MIXED ? M.L[out][0] : nullptr;
+    float* LU = MIXED ? M.L[out][1] : nullptr;
+    float* LV = MIXED ? M.L[out][2] : nullptr;
+    const int cend = min(sw * sh, first + boundary_item_cells(b.type));   // this item's cells end here
+    if (b.type == CEL_BC_SPONGE && phase == 0) {
+        // Pointwise: the loads of all the thread's cells are issued before the first store.
+        const float sl = b.sea_level;
+        size_t gi[BND_CPT];
+        int cx[BND_CPT], cy[BND_CPT];
+        float vw[BND_CPT], vu[BND_CPT], vv[BND_CPT], ba[BND_CPT];
+        float l0[BND_CPT], l1[BND_CPT], l2[BND_CPT];
+        bool ok[BND_CPT];
+#pragma unroll
+        for (int k = 0; k < BND_CPT; ++k) {
+            const int cell = first + k * 256 + threadIdx.x;
+            ok[k] = cell < cend;
+            cx[k] = x0 + cell % sw; cy[k] = y0 + cell / sw;
+            gi[k] = size_t(cy[k]) * P + cx[k];
+            vw[k] = vu[k] = vv[k] = ba[k] = l0[k] = l1[k] = l2[k] = 0.f;
+            if (ok[k]) {
+                vw[k] = W[gi[k]]; vu[k] = HU[gi[k]]; vv[k] = HV[gi[k]]; ba[k] = M.BA[gi[k]];
+                if (MIXED) { l0[k] = LW[gi[k]]; l1[k] = LU[gi[k]]; l2[k] = LV[gi[k]]; }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < BND_CPT; ++k) {
+            if (!ok[k]) continue;
+            const float gam = sponge_gamma(M, b, side, cx[k], cy[k], ba[k]);
+            if (MIXED) {
+                sponge_apply_d(gam, b.sea_level64, vw[k], l0[k], vu[k], l1[k], vv[k], l2[k]);
+                W[gi[k]] = vw[k]; HU[gi[k]] = vu[k]; HV[gi[k]] = vv[k];
+                LW[gi[k]] = l0[k]; LU[gi[k]] = l1[k]; LV[gi[k]] = l2[k];
+            } else {
+                W[gi[k]] = gam * (vw[k] - sl) + sl;
+                HU[gi[k]] = gam * vu[k];
+                HV[gi[k]] = gam * vv[k];
+            }
+        }
+        return;
+    }
+    if (b.type == CEL_BC_IRREGULAR && phase != 2) {
+        // one cell per warp, its components spread over the lanes (BND_IRR_CELLS per item)
+        const int lane = threadIdx.x & 31;
+        const int cell = first + (threadIdx.x >> 5);
+        if (cell >= cend) return;   // warp-uniform
+        const int x = x0 + cell % sw, y = y0 + cell / sw;
+        const size_t gi = size_t(y) * P + x;
+        const bool colwise = (side == 1 || side == 3);
+        const int along = colwise ? y : x;
+        const int lim = colwise ? c.ny : c.nx;
+        float o[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // w, hu, hv, then their low words
+        if (along >= 2 && along < lim + 2) {
+            if (MIXED) {
+                const double dh = fmax(0.0, b.sea_level64 - double(M.BA[gi]));
+                const double xx = (side == 1) ? double(x - NX) * M.dx64 : double(x) * M.dx64;
+                const double yy = (side == 0) ? double(y - NY) * M.dy64 : double(y) * M.dy64;
+                double r[3];
+                irregular_warp_d(b, M.waves64, xx, yy, *M.time64, dh, M.g64, lane, r);
+                for (int q = 0; q < 3; ++q) split_hl(r[q], o[q], o[3 + q]);
+            } else {
+                const float dh = fmaxf(0.f, b.sea_level - M.BA[gi]);
+                const float xx = (side == 1) ? float(x - NX) * c.dx : float(x) * c.dx;
+                const float yy = (side == 0) ? float(y - NY) * c.dy : float(y) * c.dy;
+                const float3 r = irregular_warp(b, M.waves, xx, yy, *M.time32, dh, c.g, lane);
+                o[0] = r.x; o[1] = r.y; o[2] = r.z;
+            }
+        }
+        if (lane == 0) {
+            if (phase == 1) {
+                for (int q = 0; q < SS; ++q) M.strip[SS * cell + q] = o[q];
+            } else {
+                W[gi] = o[0]; HU[gi] = o[1]; HV[gi] = o[2];
+                if (MIXED) { LW[gi] = o[3]; LU[gi] = o[4]; LV[gi] = o[5]; }
+            }
+        }
+        return;
+    }
+    const int cpt = (b.type == CEL_BC_SPONGE) ? BND_CPT : 1;
+    for (int k = 0; k < cpt; ++k) {
+        const int cell = first + k * 256 + threadIdx.x;
+        if (cell >= cend) break;   // cells ascend with k
+        const int x = x0 + cell % sw, y = y0 + cell / sw;
+        const size_t gi = size_t(y) * P + x;
+        if (phase == 2) {
+            W[gi] = M.strip[SS * cell]; HU[gi] = M.strip[SS * cell + 1]; HV[gi] = M.strip[SS * cell + 2];
+            if (MIXED) { LW[gi] = M.strip[SS * cell + 3]; LU[gi] = M.strip[SS * cell + 4]; LV[gi] = M.strip[SS * cell + 5]; }
+            continue;
+        }
+        float ow = 0.f, ou = 0.f, ov = 0.f;
+        float lw = 0.f, lu = 0.f, lv = 0.f;
+        const float sl = b.sea_level;
+        if (b.type == CEL_BC_SOLID) {
+            int qx, qy;
+            solid_source(side, x, y, c.nx, c.ny, qx, qy);
+            float sw_ = 0.f, su = 0.f, sv = 0.f, lw_ = 0.f, lu_ = 0.f, lv_ = 0.f;
+            if (qx >= 0 && qy >= 0 && qx < NX && qy < NY) {
+                const size_t qi = size_t(qy) * P + qx;
+                sw_ = W[qi]; su = HU[qi]; sv = HV[qi];
+                if (MIXED) { lw_ = LW[qi]; lu_ = LU[qi]; lv_ = LV[qi]; }
+            }
+            ow = sw_; lw = lw_;
+            ou = (side == 1 || side == 3) ? -su : su; lu = (side == 1 || side == 3) ? -lu_ : lu_;
+            ov = (side == 0 || side == 2) ? -sv : sv; lv = (side == 0 || side == 2) ? -lv_ : lv_;
+        } else if (b.type == CEL_BC_SPONGE) {
+            ow = W[gi]; ou = HU[gi]; ov = HV[gi];
+            const float gam = sponge_gamma(M, b, side, x, y, M.BA[gi]);
+            if (MIXED) {
+                lw = LW[gi]; lu = LU[gi]; lv = LV[gi];
+                sponge_apply_d(gam, b.sea_level64, ow, lw, ou, lu, ov, lv);
+            } else {
+                ow = gam * (ow - sl) + sl;
+                ou = gam * ou;
+                ov = gam * ov;
+            }
+        } else if (b.type == CEL_BC_SINEWAVE) {
+            if (MIXED) {
+                const double dh = fmax(0.0, b.sea_level64 - double(M.BA[gi]));
+                const double xx = (side == 1) ? double(x - NX) * M.dx64 : double(x) * M.dx64;
+                const double yy = (side == 0) ? double(y - NY) * M.dy64 : double(y) * M.dy64;
+                double e = 0.0, hu = 0.0, hv = 0.0;
+                if (dh > CEL_MIN_DEPTH_D)
+                    sine_wave_d(xx, yy, *M.time64, dh, b.amplitude64, b.period64, b.theta64, 0.0, M.g64, e, hu, hv);
+                split_hl(e + b.sea_level64, ow, lw);
+                split_hl(hu, ou, lu);
+                split_hl(hv, ov, lv);
+            } else {
+                const float dh = fmaxf(0.f, sl - M.BA[gi]);
+                const float xx = (side == 1) ? float(x - NX) * c.dx : float(x) * c.dx;
+                const float yy = (side == 0) ? float(y - NY) * c.dy : float(y) * c.dy;
+                float e = 0.f, hu = 0.f, hv = 0.f;
+                if (dh > CEL_MIN_DEPTH) sine_wave(xx, yy, *M.time32, dh, b.amplitude, b.period, b.theta, 0.f, c.g, e, hu, hv);
+                ow = e + sl; ou = hu; ov = hv;
+            }
+        } else if (b.type == CEL_BC_UTS) {
+            if (MIXED) {
+                double v[3];
+                uts_lookup<double>(M.uts64[side], M.nuts[side], *M.time64, v);
+                split_hl(v[0] + b.sea_level64, ow, lw);
+                split_hl(v[1], ou, lu);
+                split_hl(v[2], ov, lv);
+            } else {
+                float v[3];
+                uts_lookup<float>(M.uts[side], M.nuts[side], *M.time32, v);
+                ow = v[0] + sl; ou = v[1]; ov = v[2];
+            }
+        }
+        if (phase == 1) {
+            M.strip[SS * cell] = ow; M.strip[SS * cell + 1] = ou; M.strip[SS * cell + 2] = ov;
+            if (MIXED) { M.strip[SS * cell + 3] = lw; M.strip[SS * cell + 4] = lu; M.strip[SS * cell + 5] = lv; }
+        } else {
+            W[gi] = ow; HU[gi] = ou; HV[gi] = ov;
+            if (MIXED) { LW[gi] = lw; LU[gi] = lu; LV[gi] = lv; }
+        }
+    }
+}
+
+// A side's strip, clamped to the texture
+__device__ __forceinline__ Rect side_strip(const MemberDev& M, int side) {
+    const int NX = M.c.NX, NY = M.c.NY, w = M.bd[side].width;
+    if (side == 0) return Rect{0, max(NY - w, 0), NX, NY};
+    if (side == 1) return Rect{max(NX - w, 0), 0, NX, NY};
+    if (side == 2) return Rect{0, 0, NX, min(w, NY)};
+    return Rect{0, 0, min(w, NX), NY};
+}
+
+// One side's launch (members whose sides cannot run together, boundary_plan.hpp)
 template <bool MIXED>
 __global__ void __launch_bounds__(256, 2) k_boundary(const MemberDev* __restrict__ mems, const int2* __restrict__ items,
                                                   int nitems, int side, int phase, int out) {
-    constexpr int SS = MIXED ? 6 : 3;   // strip floats per cell: w, hu, hv (+ their low words)
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const int2 wi = items[it];
         const MemberDev& M = mems[wi.x];
-        const SimConsts c = M.c;
-        const BoundaryDesc& b = M.bd[side];
-        const int NX = c.NX, NY = c.NY, P = M.P;
-        int x0, y0, sw, sh;
-        if (side == 0) { x0 = 0; sw = NX; y0 = NY - b.width; sh = b.width; }
-        else if (side == 1) { x0 = NX - b.width; sw = b.width; y0 = 0; sh = NY; }
-        else if (side == 2) { x0 = 0; sw = NX; y0 = 0; sh = b.width; }
-        else { x0 = 0; sw = b.width; y0 = 0; sh = NY; }
-        if (x0 < 0) { sw += x0; x0 = 0; }
-        if (y0 < 0) { sh += y0; y0 = 0; }
-        sw = min(sw, NX - x0); sh = min(sh, NY - y0);
-        float* W = M.S[out][0];
-        float* HU = M.S[out][1];
-        float* HV = M.S[out][2];
-        float* LW = MIXED ? M.L[out][0] : nullptr;
-        float* LU = MIXED ? M.L[out][1] : nullptr;
-        float* LV = MIXED ? M.L[out][2] : nullptr;
-        const int cend = min(sw * sh, wi.y + boundary_item_cells(b.type));   // this item's cells end here
-        if (b.type == CEL_BC_SPONGE && phase == 0) {
-            // Pointwise: the loads of all the thread's cells are issued before the first store.
-            const float sl = b.sea_level;
-            size_t gi[BND_CPT];
-            int cx[BND_CPT], cy[BND_CPT];
-            float vw[BND_CPT], vu[BND_CPT], vv[BND_CPT], ba[BND_CPT];
-            float l0[BND_CPT], l1[BND_CPT], l2[BND_CPT];
-            bool ok[BND_CPT];
-#pragma unroll
-            for (int k = 0; k < BND_CPT; ++k) {
-                const int cell = wi.y + k * 256 + threadIdx.x;
-                ok[k] = cell < cend;
-                cx[k] = x0 + cell % sw; cy[k] = y0 + cell / sw;
-                gi[k] = size_t(cy[k]) * P + cx[k];
-                vw[k] = vu[k] = vv[k] = ba[k] = l0[k] = l1[k] = l2[k] = 0.f;
-                if (ok[k]) {
-                    vw[k] = W[gi[k]]; vu[k] = HU[gi[k]]; vv[k] = HV[gi[k]]; ba[k] = M.BA[gi[k]];
-                    if (MIXED) { l0[k] = LW[gi[k]]; l1[k] = LU[gi[k]]; l2[k] = LV[gi[k]]; }
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < BND_CPT; ++k) {
-                if (!ok[k]) continue;
-                const float gam = sponge_gamma(M, b, side, cx[k], cy[k], ba[k]);
-                if (MIXED) {
-                    sponge_apply_d(gam, b.sea_level64, vw[k], l0[k], vu[k], l1[k], vv[k], l2[k]);
-                    W[gi[k]] = vw[k]; HU[gi[k]] = vu[k]; HV[gi[k]] = vv[k];
-                    LW[gi[k]] = l0[k]; LU[gi[k]] = l1[k]; LV[gi[k]] = l2[k];
-                } else {
-                    W[gi[k]] = gam * (vw[k] - sl) + sl;
-                    HU[gi[k]] = gam * vu[k];
-                    HV[gi[k]] = gam * vv[k];
-                }
-            }
-            continue;
-        }
-        if (b.type == CEL_BC_IRREGULAR && phase != 2) {
-            // one cell per warp, its components spread over the lanes (BND_IRR_CELLS per item)
-            const int lane = threadIdx.x & 31;
-            const int cell = wi.y + (threadIdx.x >> 5);
-            if (cell >= cend) continue;   // warp-uniform
-            const int x = x0 + cell % sw, y = y0 + cell / sw;
-            const size_t gi = size_t(y) * P + x;
-            const bool colwise = (side == 1 || side == 3);
-            const int along = colwise ? y : x;
-            const int lim = colwise ? c.ny : c.nx;
-            float o[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // w, hu, hv, then their low words
-            if (along >= 2 && along < lim + 2) {
-                if (MIXED) {
-                    const double dh = fmax(0.0, b.sea_level64 - double(M.BA[gi]));
-                    const double xx = (side == 1) ? double(x - NX) * M.dx64 : double(x) * M.dx64;
-                    const double yy = (side == 0) ? double(y - NY) * M.dy64 : double(y) * M.dy64;
-                    double r[3];
-                    irregular_warp_d(b, M.waves64, xx, yy, *M.time64, dh, M.g64, lane, r);
-                    for (int q = 0; q < 3; ++q) split_hl(r[q], o[q], o[3 + q]);
-                } else {
-                    const float dh = fmaxf(0.f, b.sea_level - M.BA[gi]);
-                    const float xx = (side == 1) ? float(x - NX) * c.dx : float(x) * c.dx;
-                    const float yy = (side == 0) ? float(y - NY) * c.dy : float(y) * c.dy;
-                    const float3 r = irregular_warp(b, M.waves, xx, yy, *M.time32, dh, c.g, lane);
-                    o[0] = r.x; o[1] = r.y; o[2] = r.z;
-                }
-            }
-            if (lane == 0) {
-                if (phase == 1) {
-                    for (int q = 0; q < SS; ++q) M.strip[SS * cell + q] = o[q];
-                } else {
-                    W[gi] = o[0]; HU[gi] = o[1]; HV[gi] = o[2];
-                    if (MIXED) { LW[gi] = o[3]; LU[gi] = o[4]; LV[gi] = o[5]; }
-                }
-            }
-            continue;
-        }
-        const int cpt = (b.type == CEL_BC_SPONGE) ? BND_CPT : 1;
-        for (int k = 0; k < cpt; ++k) {
-            const int cell = wi.y + k * 256 + threadIdx.x;
-            if (cell >= cend) break;   // cells ascend with k
-            const int x = x0 + cell % sw, y = y0 + cell / sw;
-            const size_t gi = size_t(y) * P + x;
-            if (phase == 2) {
-                W[gi] = M.strip[SS * cell]; HU[gi] = M.strip[SS * cell + 1]; HV[gi] = M.strip[SS * cell + 2];
-                if (MIXED) { LW[gi] = M.strip[SS * cell + 3]; LU[gi] = M.strip[SS * cell + 4]; LV[gi] = M.strip[SS * cell + 5]; }
-                continue;
-            }
-            float ow = 0.f, ou = 0.f, ov = 0.f;
-            float lw = 0.f, lu = 0.f, lv = 0.f;
-            const float sl = b.sea_level;
-            if (b.type == CEL_BC_SOLID) {
-                int qx, qy;
-                solid_source(side, x, y, c.nx, c.ny, qx, qy);
-                float sw_ = 0.f, su = 0.f, sv = 0.f, lw_ = 0.f, lu_ = 0.f, lv_ = 0.f;
-                if (qx >= 0 && qy >= 0 && qx < NX && qy < NY) {
-                    const size_t qi = size_t(qy) * P + qx;
-                    sw_ = W[qi]; su = HU[qi]; sv = HV[qi];
-                    if (MIXED) { lw_ = LW[qi]; lu_ = LU[qi]; lv_ = LV[qi]; }
-                }
-                ow = sw_; lw = lw_;
-                ou = (side == 1 || side == 3) ? -su : su; lu = (side == 1 || side == 3) ? -lu_ : lu_;
-                ov = (side == 0 || side == 2) ? -sv : sv; lv = (side == 0 || side == 2) ? -lv_ : lv_;
-            } else if (b.type == CEL_BC_SPONGE) {
-                ow = W[gi]; ou = HU[gi]; ov = HV[gi];
-                const float gam = sponge_gamma(M, b, side, x, y, M.BA[gi]);
-                if (MIXED) {
-                    lw = LW[gi]; lu = LU[gi]; lv = LV[gi];
-                    sponge_apply_d(gam, b.sea_level64, ow, lw, ou, lu, ov, lv);
-                } else {
-                    ow = gam * (ow - sl) + sl;
-                    ou = gam * ou;
-                    ov = gam * ov;
-                }
-            } else if (b.type == CEL_BC_SINEWAVE) {
-                if (MIXED) {
-                    const double dh = fmax(0.0, b.sea_level64 - double(M.BA[gi]));
-                    const double xx = (side == 1) ? double(x - NX) * M.dx64 : double(x) * M.dx64;
-                    const double yy = (side == 0) ? double(y - NY) * M.dy64 : double(y) * M.dy64;
-                    double e = 0.0, hu = 0.0, hv = 0.0;
-                    if (dh > CEL_MIN_DEPTH_D)
-                        sine_wave_d(xx, yy, *M.time64, dh, b.amplitude64, b.period64, b.theta64, 0.0, M.g64, e, hu, hv);
-                    split_hl(e + b.sea_level64, ow, lw);
-                    split_hl(hu, ou, lu);
-                    split_hl(hv, ov, lv);
-                } else {
-                    const float dh = fmaxf(0.f, sl - M.BA[gi]);
-                    const float xx = (side == 1) ? float(x - NX) * c.dx : float(x) * c.dx;
-                    const float yy = (side == 0) ? float(y - NY) * c.dy : float(y) * c.dy;
-                    float e = 0.f, hu = 0.f, hv = 0.f;
-                    if (dh > CEL_MIN_DEPTH) sine_wave(xx, yy, *M.time32, dh, b.amplitude, b.period, b.theta, 0.f, c.g, e, hu, hv);
-                    ow = e + sl; ou = hu; ov = hv;
-                }
-            } else if (b.type == CEL_BC_UTS) {
-                if (MIXED) {
-                    double v[3];
-                    uts_lookup<double>(M.uts64[side], M.nuts[side], *M.time64, v);
-                    split_hl(v[0] + b.sea_level64, ow, lw);
-                    split_hl(v[1], ou, lu);
-                    split_hl(v[2], ov, lv);
-                } else {
-                    float v[3];
-                    uts_lookup<float>(M.uts[side], M.nuts[side], *M.time32, v);
-                    ow = v[0] + sl; ou = v[1]; ov = v[2];
-                }
-            }
-            if (phase == 1) {
-                M.strip[SS * cell] = ow; M.strip[SS * cell + 1] = ou; M.strip[SS * cell + 2] = ov;
-                if (MIXED) { M.strip[SS * cell + 3] = lw; M.strip[SS * cell + 4] = lu; M.strip[SS * cell + 5] = lv; }
-            } else {
-                W[gi] = ow; HU[gi] = ou; HV[gi] = ov;
-                if (MIXED) { LW[gi] = lw; LU[gi] = lu; LV[gi] = lv; }
-            }
+        const Rect r = side_strip(M, side);
+        boundary_item<MIXED>(M, side, phase, out, r.x0, r.y0, r.x1 - r.x0, r.y1 - r.y0, wi.y);
+    }
+}
+
+// All four sides of every member in one launch.  Item: {member, region, first, rows}: a segment's cells
+// from `first` on, or of a corner the rows (rows > 0) or columns (rows < 0) from `first` on, whose two sides
+// the CTA takes in drawing order (a wave-maker's corner texels cost most: uncut, 80 of them in one CTA of
+// the 2048 x 2048 coast took 40 us, as long as four launches).  Four launches of a few thousand threads
+// each were bound by launch latency, 2.4 us a graph node on 512 x 64 cells: us per step there 57.4 ->
+// 43.3, harbour 1017 x 643 (3 passes) 243 -> 182, 1024 x 1024 176 -> 156, 2048 x 2048 490 -> 461.
+template <bool MIXED>
+__global__ void __launch_bounds__(256, 2) k_boundary_all(const MemberDev* __restrict__ mems, const int4* __restrict__ items,
+                                                         int nitems, int out) {
+    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
+        const int4 wi = items[it];
+        const MemberDev& M = mems[wi.x];
+        Rect r = M.breg[wi.y];
+        const bool corner = wi.y >= 4;
+        if (corner && wi.w > 0) { r.y0 = wi.z; r.y1 = min(r.y1, wi.z + wi.w); }
+        if (corner && wi.w < 0) { r.x0 = wi.z; r.x1 = min(r.x1, wi.z - wi.w); }
+        for (int q = 0; q < (corner ? 2 : 1); ++q) {
+            const int side = corner ? corner_side(wi.y - 4, q) : wi.y;
+            const Rect s = side_strip(M, side);
+            const int x0 = max(r.x0, s.x0), x1 = min(r.x1, s.x1), y0 = max(r.y0, s.y0), y1 = min(r.y1, s.y1);
+            const int n = x1 > x0 && y1 > y0 ? (x1 - x0) * (y1 - y0) : 0;
+            const int cells = boundary_item_cells(M.bd[side].type);
+            const int begin = corner ? 0 : wi.z, end = corner ? n : min(n, wi.z + 1);
+            for (int first = begin; first < end; first += cells)
+                boundary_item<MIXED>(M, side, 0, out, x0, y0, x1 - x0, y1 - y0, first);
+            if (corner) __syncthreads();   // (uniform: the whole CTA is on this item)
         }
     }
 }
@@ -2744,7 +2787,8 @@ struct cel_lane {
     double* spart = nullptr;                    // their statistics
     int2* rows = nullptr; int nrows = 0;
     int2* bands = nullptr; int nbands = 0;
-    int2* bitems[4] = {nullptr, nullptr, nullptr, nullptr};
+    int4* ball = nullptr; int nball = 0;        // work items of the one-launch boundary
+    int2* bitems[4] = {nullptr, nullptr, nullptr, nullptr};   // of the sides' own launches (other members)
     int nbitems[4] = {0, 0, 0, 0};
     bool two_phase[4] = {false, false, false, false};
     double* stats_all = nullptr;       // members * STATS_N, gathered by the first pass of each step
@@ -2974,6 +3018,12 @@ int launch_pass(cel_lane* b, const PassArgs& pa, std::string& err) {
     }
     B_TRY(cudaEventRecord(b->ev_join, b->side));
     B_TRY(cudaStreamWaitEvent(b->stream, b->ev_join, 0));
+    if (b->nball > 0) {
+        const int g = std::min(b->nball, b->sms * 8);
+        TimedLaunch t(&b->tm, b->stream, "boundary");
+        if (b->mixed) k_boundary_all<true><<<g, 256, 0, b->stream>>>(b->ddev, b->ball, b->nball, pa.out);
+        else k_boundary_all<false><<<g, 256, 0, b->stream>>>(b->ddev, b->ball, b->nball, pa.out);
+    }
     for (int side : {1, 0, 3, 2}) {
         if (b->nbitems[side] == 0) continue;
         const int g = std::min(b->nbitems[side], b->sms * 8);
@@ -3426,7 +3476,7 @@ cel_lane* lane_create(int n, const cel_params* const* params, const float* const
             cudaMemcpy(b->ctl, c0.data(), n * sizeof(DtCtl), cudaMemcpyHostToDevice);
         }
     }
-    std::vector<int4> tiles;
+    std::vector<int4> tiles, ball, corners;
     std::vector<int2> rows, bitems[4];
     int max_nx = 0, max_ny = 0;
     for (int i = 0; i < n; ++i) {
@@ -3568,10 +3618,37 @@ cel_lane* lane_create(int n, const cel_params* const* params, const float* const
                 d.uts64[s] = static_cast<double*>(up);
                 d.nuts[s] = bb.n_uts;
             }
-            const int cellsn = (s == 0 || s == 2) ? NX * std::min(bb.width, NY) : std::min(bb.width, NX) * NY;
-            for (int c0 = 0; c0 < cellsn; c0 += boundary_item_cells(bb.type)) bitems[s].push_back(make_int2(i, c0));
-            // a solid strip wider than 2 reads ghost cells of its own strip: compute, then write
-            if (bb.type == CEL_BC_SOLID && bb.width >= 3) b->two_phase[s] = true;
+        }
+        const int btype[4] = {d.bd[0].type, d.bd[1].type, d.bd[2].type, d.bd[3].type};
+        const int bwidth[4] = {d.bd[0].width, d.bd[1].width, d.bd[2].width, d.bd[3].width};
+        if (plan_boundary(m.hs.nx, m.hs.ny, btype, bwidth, d.breg)) {
+            for (int k = BND_REGIONS - 1; k >= 0; --k) {   // corners first: they take longest
+                const int n = std::max(0, d.breg[k].x1 - d.breg[k].x0) * std::max(0, d.breg[k].y1 - d.breg[k].y0);
+                if (k >= 4) {
+                    if (n <= 0) continue;
+                    // pieces of about one item of the costlier side
+                    const int cells = std::min({boundary_item_cells(btype[corner_side(k - 4, 0)]),
+                                                boundary_item_cells(btype[corner_side(k - 4, 1)]), 256});
+                    const Rect& r = d.breg[k];
+                    const CornerCut cut = corner_cut(k - 4, btype);
+                    const int across = cut == CUT_ROWS ? r.x1 - r.x0 : r.y1 - r.y0, len = std::max(1, cells / across);
+                    if (cut == CUT_ROWS)
+                        for (int y = r.y0; y < r.y1; y += len) corners.push_back(make_int4(i, k, y, len));
+                    else if (cut == CUT_COLUMNS)
+                        for (int x = r.x0; x < r.x1; x += len) corners.push_back(make_int4(i, k, x, -len));
+                    else
+                        corners.push_back(make_int4(i, k, 0, 0));
+                } else {
+                    for (int c0 = 0; c0 < n; c0 += boundary_item_cells(btype[k])) ball.push_back(make_int4(i, k, c0, 0));
+                }
+            }
+        } else {
+            for (int s = 0; s < 4; ++s) {
+                const int cellsn = (s == 0 || s == 2) ? NX * std::min(bwidth[s], NY) : std::min(bwidth[s], NX) * NY;
+                for (int c0 = 0; c0 < cellsn; c0 += boundary_item_cells(btype[s])) bitems[s].push_back(make_int2(i, c0));
+                // a solid strip wider than 2 reads ghost cells of its own strip: compute, then write
+                if (btype[s] == CEL_BC_SOLID && bwidth[s] >= 3) b->two_phase[s] = true;
+            }
         }
         {
             size_t strip = 0;
@@ -3612,6 +3689,8 @@ cel_lane* lane_create(int n, const cel_params* const* params, const float* const
         return CEL_OK;
     };
     if (upload_list(tiles, &b->tiles, b->ntiles) || upload_list(rows, &b->rows, b->nrows)) return nullptr;
+    corners.insert(corners.end(), ball.begin(), ball.end());
+    if (upload_list(corners, &b->ball, b->nball)) return nullptr;
     for (int s = 0; s < 4; ++s)
         if (upload_list(bitems[s], &b->bitems[s], b->nbitems[s])) return nullptr;
     {
@@ -3993,7 +4072,7 @@ int lane_col_threads(const cel_lane* b) { return b->cnt; }
 KernelTimer* lane_timer(cel_lane* b) { return &b->tm; }
 
 int lane_launches_per_step(const cel_lane* b) {
-    int per_pass = 3;  // stencil, row solve, column solve
+    int per_pass = 3 + (b->nball > 0 ? 1 : 0);  // stencil, row solve, column solve, boundaries
     for (int s = 0; s < 4; ++s)
         if (b->nbitems[s] > 0) per_pass += b->two_phase[s] ? 2 : 1;
     // adaptive batches add the dt choice before every pass and the CFL reduction before the predictor

@@ -65,33 +65,47 @@ int main() {
             for (int y = q.y0; y < q.y1; ++y)
                 for (int x = q.x0; x < q.x1; ++x) want[size_t(y) * NX + x] = value(src, s, x, y, nullptr);
         }
-        std::vector<int> writer(pre.size(), -1);
-        std::vector<std::vector<int>> reads(BND_REGIONS);
-        std::vector<u64> got = pre;
+        // the regions, the corners cut into single rows or columns where that is allowed
+        struct Piece { int k; Rect r; };
+        std::vector<Piece> pieces;
         for (int k = 0; k < BND_REGIONS; ++k) {
+            const CornerCut cut = k < 4 ? CUT_NONE : corner_cut(k - 4, type);
+            if (cut == CUT_ROWS)
+                for (int y = R[k].y0; y < R[k].y1; ++y) pieces.push_back({k, {R[k].x0, y, R[k].x1, y + 1}});
+            else if (cut == CUT_COLUMNS)
+                for (int x = R[k].x0; x < R[k].x1; ++x) pieces.push_back({k, {x, R[k].y0, x + 1, R[k].y1}});
+            else
+                pieces.push_back({k, R[k]});
+        }
+        std::vector<int> writer(pre.size(), -1);
+        std::vector<std::vector<int>> reads(pieces.size());
+        std::vector<u64> got = pre;
+        for (int q = 0; q < int(pieces.size()); ++q) {
+            const int k = pieces[q].k;
+            const Rect rect = pieces[q].r;
             std::vector<u64> local = pre;   // a region sees the state before the launch, and its own writes
-            for (int q = 0; q < (k < 4 ? 1 : 2); ++q) {
-                const int s = k < 4 ? k : corner_side(k - 4, q);
+            for (int turn = 0; turn < (k < 4 ? 1 : 2); ++turn) {
+                const int s = k < 4 ? k : corner_side(k - 4, turn);
                 Rect t = strip(s);
-                t = {std::max(t.x0, R[k].x0), std::max(t.y0, R[k].y0), std::min(t.x1, R[k].x1), std::min(t.y1, R[k].y1)};
+                t = {std::max(t.x0, rect.x0), std::max(t.y0, rect.y0), std::min(t.x1, rect.x1), std::min(t.y1, rect.y1)};
                 const std::vector<u64> src = local;
                 for (int y = t.y0; y < t.y1; ++y)
                     for (int x = t.x0; x < t.x1; ++x) {
                         const int e = y * NX + x;
-                        const size_t seen = reads[k].size();
-                        local[e] = got[e] = value(src, s, x, y, &reads[k]);
-                        if (writer[e] >= 0 && writer[e] != k) ++races;
-                        writer[e] = k;
-                        for (size_t i = seen; i < reads[k].size(); ++i) {   // written in place in the same sweep
-                            const int ry = reads[k][i] / NX, rx = reads[k][i] % NX;
-                            if (reads[k][i] != e && rx >= t.x0 && rx < t.x1 && ry >= t.y0 && ry < t.y1) ++races;
+                        const size_t seen = reads[q].size();
+                        local[e] = got[e] = value(src, s, x, y, &reads[q]);
+                        if (writer[e] >= 0 && writer[e] != q) ++races;
+                        writer[e] = q;
+                        for (size_t i = seen; i < reads[q].size(); ++i) {   // written in place in the same sweep
+                            const int ry = reads[q][i] / NX, rx = reads[q][i] % NX;
+                            if (reads[q][i] != e && rx >= t.x0 && rx < t.x1 && ry >= t.y0 && ry < t.y1) ++races;
                         }
                     }
             }
         }
-        for (int k = 0; k < BND_REGIONS; ++k)
-            for (int e : reads[k])
-                if (writer[e] >= 0 && writer[e] != k) ++races;
+        for (int q = 0; q < int(pieces.size()); ++q)
+            for (int e : reads[q])
+                if (writer[e] >= 0 && writer[e] != q) ++races;
         if (got != want) ++wrong;
     }
     std::printf("%ld %ld %ld %ld\n", planned, refused, wrong, races);
