@@ -77,7 +77,7 @@ class Engine:
         check(lib().cel_set_stream(self.h, C.c_void_p(stream_ptr or 0)))
 
     def state(self) -> np.ndarray:
-        out = np.zeros(self.shape + (4,), dtype=np.float32)
+        out = np.empty(self.shape + (4,), dtype=np.float32)   # (every value is written)
         check(lib().cel_get_state(self.h, _fp(out)))
         return out
 
@@ -92,7 +92,7 @@ class Engine:
         return out
 
     def aux(self) -> np.ndarray:
-        out = np.zeros(self.shape + (4,), dtype=np.float32)
+        out = np.empty(self.shape + (4,), dtype=np.float32)   # (every value is written)
         check(lib().cel_get_aux(self.h, _fp(out)))
         return out
 
@@ -219,15 +219,15 @@ class Batch:
         return [arr[i].as_dict() for i in range(self.n)]
 
     def state(self, i: int) -> np.ndarray:
-        out = np.zeros(self.shapes[i] + (4,), dtype=np.float32)
+        out = np.empty(self.shapes[i] + (4,), dtype=np.float32)
         check(lib().cel_batch_get_state(self.h, i, _fp(out)))
         return out
 
     def state_parts(self, i: int):
         """Member i's state as (hi, lo) float textures; hi + lo is the compensated state (lo = 0 in
         the FP32 forms)."""
-        hi = np.zeros(self.shapes[i] + (4,), dtype=np.float32)
-        lo = np.zeros(self.shapes[i] + (4,), dtype=np.float32)
+        hi = np.empty(self.shapes[i] + (4,), dtype=np.float32)
+        lo = np.empty(self.shapes[i] + (4,), dtype=np.float32)
         check(lib().cel_batch_get_state_parts(self.h, i, _fp(hi), _fp(lo)))
         return hi, lo
 
@@ -236,7 +236,7 @@ class Batch:
         check(lib().cel_batch_set_state(self.h, i, _fp(a)))
 
     def aux(self, i: int) -> np.ndarray:
-        out = np.zeros(self.shapes[i] + (4,), dtype=np.float32)
+        out = np.empty(self.shapes[i] + (4,), dtype=np.float32)
         check(lib().cel_batch_get_aux(self.h, i, _fp(out)))
         return out
 
