@@ -29,18 +29,13 @@ constexpr int BX2 = 32, BY2 = 8;
 
 inline dim3 grid2(int w, int h) { return dim3((w + BX2 - 1) / BX2, (h + BY2 - 1) / BY2); }
 
-// ---- Pass1 (compute.hlsl:380-458): faces h,u,v {N,E,S,W}; aux; region [1,nx+3)x[1,ny+3) ----
-__global__ void k_pass1(const float4* __restrict__ st, const float4* __restrict__ bot,
-                        const float4* __restrict__ aux1, float4* __restrict__ H, float4* __restrict__ U,
-                        float4* __restrict__ V, float4* __restrict__ aux2, SimConsts c) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    if (x >= c.nx + 3 || y >= c.ny + 3) return;
+// ---- Pass1 (compute.hlsl:380-458) at texel i: faces h,u,v {N,E,S,W} and the breaking slope ----
+__device__ __forceinline__ void faces_of(const float4* __restrict__ st, const float4* __restrict__ bot, size_t i,
+                                         const SimConsts& c, float4& h, float4& u, float4& v, float& msd) {
     const int NX = c.NX;
-    const size_t i = size_t(y) * NX + x;
     const float4 cc = st[i], s = st[i - NX], n = st[i + NX], w = st[i - 1], e = st[i + 1];
     const float BN = bot[i].x, BE = bot[i].y, BS = bot[i - NX].x, BW = bot[i - 1].y;
-    float wN, wE, wS, wW, huN, huE, huS, huW, hvN, hvE, hvS, hvW, sd, msd;
+    float wN, wE, wS, wW, huN, huE, huS, huW, hvN, hvE, hvS, hvW, sd;
     reconstruct_sd(c.two_theta, w.x, cc.x, e.x, wW, wE, sd);
     msd = sd * c.one_over_dx;
     reconstruct_sd(c.two_theta, s.x, cc.x, n.x, wS, wN, sd);
@@ -51,19 +46,35 @@ __global__ void k_pass1(const float4* __restrict__ st, const float4* __restrict_
     reconstruct(c.two_theta, s.z, cc.z, n.z, hvS, hvN);
     correct_w(BW, BE, cc.x, wW, wE);
     correct_w(BS, BN, cc.x, wS, wN);
-    const float4 h = make_float4(wN - BN, wE - BE, wS - BS, wW - BW);
-    float4 u, v;
+    h = make_float4(wN - BN, wE - BE, wS - BS, wW - BW);
     float q;
     q = div_by_h(h.x, c.epsilon); u.x = q * huN; v.x = q * hvN;
     q = div_by_h(h.y, c.epsilon); u.y = q * huE; v.y = q * hvE;
     q = div_by_h(h.z, c.epsilon); u.z = q * huS; v.z = q * hvS;
     q = div_by_h(h.w, c.epsilon); u.w = q * huW; v.w = q * hvW;
-    H[i] = h; U[i] = u; V[i] = v;
-    const float4 a1 = aux1[i];
+}
+// ... and its inundation / breaking record of a texel
+__device__ __forceinline__ float4 aux_of(const float4& a1, const float4& h, float msd, const SimConsts& c) {
     const float mid = fmaxf((h.x + h.y + h.z + h.w) / 4.0f, a1.x);
     float bw = a1.w;
     if (msd > c.dissipation_threshold) bw = 1.0f;
-    aux2[i] = make_float4(mid, 0.f, msd, bw);
+    return make_float4(mid, 0.f, msd, bw);
+}
+
+// Pass1 into textures, region [1,nx+3)x[1,ny+3): only where the next pass must take the faces of a state
+// that is about to change (addSolitaryWave does not rebuild them, engine.cpp:2154-2219).
+__global__ void k_pass1(const float4* __restrict__ st, const float4* __restrict__ bot,
+                        const float4* __restrict__ aux1, float4* __restrict__ H, float4* __restrict__ U,
+                        float4* __restrict__ V, float4* __restrict__ aux2, SimConsts c) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x + 1;
+    const int y = blockIdx.y * blockDim.y + threadIdx.y + 1;
+    if (x >= c.nx + 3 || y >= c.ny + 3) return;
+    const size_t i = size_t(y) * c.NX + x;
+    float4 h, u, v;
+    float msd;
+    faces_of(st, bot, i, c, h, u, v, msd);
+    H[i] = h; U[i] = u; V[i] = v;
+    aux2[i] = aux_of(aux1[i], h, msd, c);
 }
 
 // ---- Pass2 (compute.hlsl:470-542): KP flux between the cell on a face's low side (m) and the one on
@@ -89,9 +100,9 @@ struct Pass3Args {
     const float4* st; const float4* bot; const float4* H; const float4* U; const float4* V;
     const float4* aux2; float4* aux1;
     const float4* ABCx; const float4* ABCy;
-    const float4* og; const float4* oog; const float4* ofg; const float4* oofg;
-    const float4* cur; const float4* pred; const float4* fgpred;
-    float4* out; float4* sgrad; float4* sfg;
+    const float4* og; const float4* oog; const float2* ofg; const float2* oofg;   // F*, G* as pairs
+    const float4* cur; const float4* pred; const float2* fgpred;
+    float4* out; float4* sgrad; float2* sfg;
     float dt, dt_old, dt_old_old;
     float decay;   // pow(|white-water decay rate|, dt)
     int scheme;
@@ -113,35 +124,55 @@ __device__ __forceinline__ void second_order(float yn, float y1, float y2, float
     o[2] = r * yn + g * y1 + bb * y2;
 }
 
-// ---- Pass2 and Pass3Predictor (compute.hlsl:470-542, 616-812) in one kernel, every texel of the new
-// state written once: zero on the ghost frame (engine.cpp:1007), the right-hand sides inside.  A cell
-// takes the fluxes of its four faces from the stored face states (each flux is computed by the two
-// cells that share the face, from the same values), so the flux textures, their clears and their
-// round trip through memory are gone.  It is bound by the flux arithmetic (IEEE divisions and square
-// roots) once the textures are in L2: 12.5 us on 512 x 64 cells and 76 us on 1001 x 777 by event timing,
-// where Pass2 and Pass3 took 8.5 + 8.6 and 24 + 51 us beside three clears.  The white-water decay of Pass2
-// runs on its own region [1,nx+2)x[1,ny+2). ----
-__global__ void k_pass23(Pass3Args a, SimConsts c) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= c.NX || y >= c.NY) return;
+// ---- Pass1, Pass2 and Pass3Predictor (compute.hlsl:380-542, 616-812) in one kernel, every texel of the
+// new state written once: zero on the ghost frame (engine.cpp:1007), the right-hand sides inside.  A CTA
+// forms the faces of its 32 x 8 texels and the ring around them in shared memory, and a cell takes the
+// fluxes of its four faces from there (each flux is computed by the two cells that share the face, from
+// the same values), so neither the face nor the flux textures make a round trip through memory: 96 and 32
+// bytes a cell and pass less, against 340 face computations for 256 cells.  STORED: the faces come from the
+// textures (k_pass1).  The record's update runs on its own region [1,nx+2)x[1,ny+2).
+// Bound by the IEEE divisions and square roots on small domains (latency) and by memory on large ones;
+// event times: 512 x 64 cells Pass1, Pass2, Pass3 8.6 + 8.5 + 8.6 us and three clears -> 14.7 us, 1001 x 777
+// 23 + 24 + 51 us and the clears -> 69 us. ----
+constexpr int FW = BX2 + 2, FH = BY2 + 2;
+template <bool STORED>
+__global__ void __launch_bounds__(BX2 * BY2) k_pass123(Pass3Args a, SimConsts c) {
+    __shared__ float4 fh[STORED ? 1 : FW * FH], fu[STORED ? 1 : FW * FH], fv[STORED ? 1 : FW * FH];
+    __shared__ float fm[STORED ? 1 : FW * FH];
+    const int x = blockIdx.x * BX2 + threadIdx.x;
+    const int y = blockIdx.y * BY2 + threadIdx.y;
     const int NX = c.NX;
+    const int f = (int(threadIdx.y) + 1) * FW + int(threadIdx.x) + 1;   // this cell in the tile
+    if (!STORED) {
+        const int xf = int(blockIdx.x * BX2) - 1, yf = int(blockIdx.y * BY2) - 1;
+        for (int k = threadIdx.y * BX2 + threadIdx.x; k < FW * FH; k += BX2 * BY2) {
+            const int gx = xf + k % FW, gy = yf + k / FW;
+            if (gx < 1 || gy < 1 || gx >= c.nx + 3 || gy >= c.ny + 3) continue;
+            faces_of(a.st, a.bot, size_t(gy) * NX + gx, c, fh[k], fu[k], fv[k], fm[k]);
+        }
+        __syncthreads();
+    }
+    if (x >= NX || y >= c.NY) return;
     const size_t i = size_t(y) * NX + x;
     if (x >= 1 && y >= 1 && x < c.nx + 2 && y < c.ny + 2) {
-        const float4 a2 = a.aux2[i];
+        const float4 a2 = STORED ? a.aux2[i] : aux_of(a.aux1[i], fh[f], fm[f], c);
         a.aux1[i] = make_float4(a2.x, 0.f, a2.z, a2.w * a.decay);
     }
     if (x < 2 || y < 2 || x >= c.nx + 2 || y >= c.ny + 2) {
         a.out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
-    const float4 hc = a.H[i], uc = a.U[i], vc = a.V[i];
-    const float4 hw = a.H[i - 1], uw = a.U[i - 1], vw = a.V[i - 1], he = a.H[i + 1], ue = a.U[i + 1], ve = a.V[i + 1];
-    const float4 hs = a.H[i - NX], us = a.U[i - NX], vs = a.V[i - NX], hn = a.H[i + NX], un = a.U[i + NX], vn = a.V[i + NX];
-    const float3 xh = x_flux(hc.y, uc.y, vc.y, he.w, ue.w, ve.w, c.g, c.half_g);
-    const float3 xw = x_flux(hw.y, uw.y, vw.y, hc.w, uc.w, vc.w, c.g, c.half_g);
-    const float3 yh = y_flux(hc.x, uc.x, vc.x, hn.z, un.z, vn.z, c.g, c.half_g);
-    const float3 ys = y_flux(hs.x, us.x, vs.x, hc.z, uc.z, vc.z, c.g, c.half_g);
+    float3 xh, xw, yh, ys;
+    {
+        auto H = [&](int dx, int dy) { return STORED ? a.H[i + dx + ptrdiff_t(dy) * NX] : fh[f + dx + dy * FW]; };
+        auto U = [&](int dx, int dy) { return STORED ? a.U[i + dx + ptrdiff_t(dy) * NX] : fu[f + dx + dy * FW]; };
+        auto V = [&](int dx, int dy) { return STORED ? a.V[i + dx + ptrdiff_t(dy) * NX] : fv[f + dx + dy * FW]; };
+        const float4 hc = H(0, 0), uc = U(0, 0), vc = V(0, 0);
+        xh = x_flux(hc.y, uc.y, vc.y, H(1, 0).w, U(1, 0).w, V(1, 0).w, c.g, c.half_g);
+        xw = x_flux(H(-1, 0).y, U(-1, 0).y, V(-1, 0).y, hc.w, uc.w, vc.w, c.g, c.half_g);
+        yh = y_flux(hc.x, uc.x, vc.x, H(0, 1).z, U(0, 1).z, V(0, 1).z, c.g, c.half_g);
+        ys = y_flux(H(0, -1).x, U(0, -1).x, V(0, -1).x, hc.z, uc.z, vc.z, c.g, c.half_g);
+    }
     const float4* st = a.st;
     const float4* bot = a.bot;
     const float BYh = bot[i].x, BXh = bot[i].y, BAh = bot[i].z;
@@ -175,7 +206,10 @@ __global__ void k_pass23(Pass3Args a, SimConsts c) {
     const float P1y = Bg * (d3) * ((euu - 2 * eu + 2 * ed - edd) * (0.5f * od3y) +
                                    (eur + eul - 2 * eu + 2 * ed - edr - edl) * (0.5f * ody * od2x));
     const float P2y = Bg * (d2) * (ddy * (exx + 2 * eyy) + ddx * exy);
-    const float fr = friction_calc(cc.y, cc.z, h, c.friction, c.is_manning, c.g, c.epsilon);
+    // Both friction laws give 0 * |momentum| for a zero coefficient, whatever the (finite) depth: the two
+    // double-precision powers are left out then (h - h carries a depth that is not finite).
+    const float fr = c.friction == 0.f ? 0.f * sqrtf(cc.y * cc.y + cc.z * cc.z) + (h - h)
+                                       : friction_calc(cc.y, cc.z, h, c.friction, c.is_manning, c.g, c.epsilon);
     const float s1 = -c.g_over_dx * h * (BXh - BXw) - cc.y * fr + (P1x + P2x);
     const float s2 = -c.g_over_dy * h * (BYh - BYs) - cc.z * fr + (P1y + P2y);
     const float f0 = (xw.x - xh.x) * odx + (ys.x - yh.x) * ody + 0.f;
@@ -191,7 +225,8 @@ __global__ void k_pass23(Pass3Args a, SimConsts c) {
         huO = cx.x * l.y + cx.y * cc.y + cx.z * r.y + dt * f1;
         hvO = cy.x * d.z + cy.y * cc.z + cy.z * u.z + dt * f2;
     } else {
-        const float4 o = a.og[i], oo = a.oog[i], fo = a.ofg[i], foo = a.oofg[i];
+        const float4 o = a.og[i], oo = a.oog[i];
+        const float2 fo = a.ofg[i], foo = a.oofg[i];
         if (a.scheme == CEL_SCHEME_PREDICTOR) {
             wO = cc.x + dt / 12.0f * (23.0f * f0 - 16.0f * o.x + 5.0f * oo.x);
             huO = cx.x * l.y + cx.y * cc.y + cx.z * r.y + dt / 12.0f * (23.0f * f1 - 16.0f * o.y + 5.0f * oo.y) +
@@ -210,7 +245,8 @@ __global__ void k_pass23(Pass3Args a, SimConsts c) {
                   dt / 6.0f * (cf[0] * dG[0] + cf[1] * dG[1] + cf[2] * dG[2]);
         } else {  // corrector
             const float4 qc = a.cur[i], qr = a.cur[i + 1], ql = a.cur[i - 1], qu = a.cur[i + NX], qd = a.cur[i - NX];
-            const float4 pr = a.pred[i], fp = a.fgpred[i];
+            const float4 pr = a.pred[i];
+            const float2 fp = a.fgpred[i];
             wO = qc.x + dt / 24.0f * (9 * f0 + 19 * pr.x - 5 * o.x + 1 * oo.x);
             huO = cx.x * ql.y + cx.y * qc.y + cx.z * qr.y + dt / 24.0f * (9 * f1 + 19 * pr.y - 5 * o.y + 1 * oo.y) + Fs -
                   fp.x;
@@ -220,7 +256,7 @@ __global__ void k_pass23(Pass3Args a, SimConsts c) {
     }
     a.out[i] = make_float4(wO, huO, hvO, 0.f);
     a.sgrad[i] = make_float4(f0, f1, f2, 0.f);
-    a.sfg[i] = make_float4(Fs, Gs, 0.f, 0.f);
+    a.sfg[i] = make_float2(Fs, Gs);
 }
 
 // ---- Cyclic reduction (compute.hlsl:835-947), every level of a system in one CTA -----------
@@ -233,13 +269,13 @@ __global__ void k_pass23(Pass3Args a, SimConsts c) {
 // results do not change a bit.
 //
 // A draw per level, the shader's way, costs 2 log2(n) launches a direction, most of which touch a
-// few elements.  Here a CTA keeps a system's levels in shared memory: CTAs [0, ny) take one row each,
-// the others CR_COLS adjacent columns (whose level 0 they read from the state when they need it instead
-// of keeping it).  What bounds it is latency, since the levels are a serial chain: the coefficients of
+// few elements.  Here a CTA keeps a system's levels in shared memory: the first CTAs take CR_COLS
+// adjacent columns each (whose level 0 they read from the state when they need it instead of keeping it),
+// the others one row.  What bounds it is latency, since the levels are a serial chain: the coefficients of
 // a level are loaded before the barrier that ends the level before it, and levels of at most 32
 // elements run in one warp.  hu and hv go back into the state in place (CopyFromXxAndXy,
 // compute.hlsl:814-823, is folded in).  Measured by event timing, a pass's solves: 512 x 64 cells 32
-// launches and 210 us -> 14.7 us, 1001 x 777 cells 38 launches and 295 us -> 53 us.
+// launches and 210 us -> 14.7 us, 1001 x 777 cells 38 launches and 295 us -> 42 us.
 constexpr int CR_MAX_LEVELS = 16;
 constexpr int CR_THREADS = 256;
 constexpr int CR_COLS = 4;              // columns of a column CTA: 64-byte pieces of a state row
@@ -315,6 +351,7 @@ __device__ __forceinline__ void cr_solve(const CrLevels& L, float* __restrict__ 
         __syncthreads();
     }
     for (int k = 1; k < L.tail; ++k) {
+#pragma unroll 4
         for (int i = t; i < L.len[k]; i += T) reduce(k, i, i == t ? q : k12(k, i));
         if (t == 0) lv[size_t(L.off[k] + L.len[k]) * W] = 0.f;
         if (k + 1 < L.K) q = k12(k + 1, t);
@@ -337,6 +374,7 @@ __device__ __forceinline__ void cr_solve(const CrLevels& L, float* __restrict__ 
     s = acb(L.tail - 1, t);
     __syncthreads();
     for (int k = L.tail - 1; k >= 0; --k) {
+#pragma unroll 4
         for (int j = t; 2 * j < L.len[k]; j += T) substitute(k, j, j == t ? s : acb(k, j));
         if (k > 0) {
             s = acb(k - 1, t);
@@ -349,12 +387,13 @@ __device__ __forceinline__ void cr_solve(const CrLevels& L, float* __restrict__ 
 template <bool SMEM_X, bool SMEM_Y>
 __global__ void __launch_bounds__(CR_THREADS) k_cr(SolveArgs a, SimConsts c) {
     extern __shared__ float cr_sm[];
-    const int rows = c.ny, b = blockIdx.x;
-    if (b < rows) {
+    // columns first: a column CTA has four systems and the strided reads
+    const int rows = c.ny, bands = (c.nx + CR_COLS - 1) / CR_COLS, b = int(blockIdx.x) - bands;
+    if (b >= 0) {
         float* lv = SMEM_X ? cr_sm : a.scratch + size_t(b) * a.x.total;
         cr_solve<true>(a.x, lv, reinterpret_cast<float*>(a.st + size_t(b + 2) * c.NX + 2) + 1, 4, b, 0, true);
     } else {
-        const int band = b - rows, col = band * CR_COLS + int(threadIdx.x) % CR_COLS;
+        const int band = blockIdx.x, col = band * CR_COLS + int(threadIdx.x) % CR_COLS;
         float* lv = SMEM_Y ? cr_sm
                            : a.scratch + (SMEM_X ? 0 : size_t(rows) * a.x.total) + size_t(band) * a.y.total * CR_COLS;
         cr_solve<false>(a.y, lv, reinterpret_cast<float*>(a.st + size_t(2) * c.NX + 2 + col) + 2, size_t(4) * c.NX, col, c.nx,
@@ -512,89 +551,97 @@ __global__ void __launch_bounds__(256) k_boundary_all(float4* st, const float4* 
 }
 
 // ---- GetStats (compute.hlsl:1319-1378) and its FP64 reduction in one launch -------------
-// One thread per 4x4 block (the texture's partial sums, kept for getWaterHeight) with the FP64 volume
-// and the non-finite flag of its cells; blocks cut off by the far edges count for those two only.  Each
-// CTA leaves one set of FP64 partials, and the last one to finish adds them up in CTA order, so the
-// totals do not depend on scheduling.  (The reduction by one CTA over every cell took 313 us on
-// 1001 x 777 cells, one SM of 148 reading everything.)
+// A lane per cell, 16 lanes per 4x4 block: every lane forms its cell's terms, and the block's sums
+// take them in the shader's order from the lanes (the texture's partial sums, kept for getWaterHeight, do
+// not change a bit).  Blocks cut off by the far edges count for the FP64 volume and the non-finite flag
+// only.  Each CTA leaves one set of FP64 partials, and the last one to finish adds them up in CTA order, so
+// the totals do not depend on scheduling.  A thread per block chained 16 cells' divisions and roots (16.9 us
+// by event timing on 512 x 64 cells), and the reduction by one CTA over every cell before that took 313 us
+// on 1001 x 777.
 // out: [0..4] sums, [5..8] maxima, [9] the volume, [10] 1 if a state value is not finite
-constexpr int STATS_THREADS = 64;
+constexpr int STATS_THREADS = 256;
+constexpr int STATS_CTAS = 592;   // at most: 4 per SM
 __global__ void __launch_bounds__(STATS_THREADS) k_stats(const float4* __restrict__ st, const float4* __restrict__ bot,
                                                          float* __restrict__ blocks, SimConsts c, double* __restrict__ part,
                                                          unsigned int* __restrict__ done, double* __restrict__ out) {
     __shared__ double sm[STATS_THREADS / 32][11];
     __shared__ bool last;
     const int nbx = c.nx / 4, nby = c.ny / 4, tbx = (c.nx + 3) / 4, tby = (c.ny + 3) / 4;
-    const int k = blockIdx.x * STATS_THREADS + threadIdx.x;
+    const int lane = threadIdx.x & 31, cell = lane & 15;
     double v[11] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    if (k < tbx * tby) {
-        const int bx = k % tbx, by = k / tbx;
-        const bool whole = bx < nbx && by < nby;
-        const int jn = min(4, c.ny - 4 * by), in = min(4, c.nx - 4 * bx);
-        float sh = 0, sb = 0, shu = 0, shv = 0, sk = 0, mu = 0, mh = 0, mc = 0, mf = 0;
-        for (int j = 0; j < jn; ++j)
-            for (int ii = 0; ii < in; ++ii) {
-                const size_t i = size_t(by * 4 + j + 2) * c.NX + bx * 4 + ii + 2;
-                const float4 s = st[i];
-                const float B = bot[i].z;
-                if (!isfinite(s.x) || !isfinite(s.y) || !isfinite(s.z)) v[10] = 1.0;
-                v[9] += fmax(0.0, double(s.x) - double(B));
-                const float h = fmaxf(0.f, s.x - B);
-                const float cc = sqrtf(c.g * h);
-                const float q = div_by_h(h, c.epsilon);
-                const float u = q * s.y, w = q * s.z;
-                sh += h; sb += h * (B + 0.5f * h); shu += s.y; shv += s.z;
-                sk += (s.y * u + s.z * w);
-                const float u2v2 = u * u + w * w;
-                mu = fmaxf(mu, u2v2); mh = fmaxf(mh, h);
-                mc = fmaxf(mc, (fabsf(u) + cc) * c.one_over_dx);
-                mc = fmaxf(mc, (fabsf(w) + cc) * c.one_over_dy);
-                mf = fmaxf(mf, u2v2 * q);
-            }
-        if (whole) {
+    // (the trip count is the same for a CTA: the shuffles need whole warps)
+    for (int k0 = blockIdx.x * (STATS_THREADS / 16); k0 < tbx * tby; k0 += gridDim.x * (STATS_THREADS / 16)) {
+        const int k = k0 + int(threadIdx.x >> 4);   // block
+        const int bx = k % tbx, by = k / tbx, x = 4 * bx + (cell & 3), y = 4 * by + (cell >> 2);
+        const bool here = by < tby && x < c.nx && y < c.ny, whole = bx < nbx && by < nby;
+        float q[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (here) {
+            const size_t i = size_t(y + 2) * c.NX + x + 2;
+            const float4 s = st[i];
+            const float B = bot[i].z;
+            if (!isfinite(s.x) || !isfinite(s.y) || !isfinite(s.z)) v[10] = 1.0;
+            v[9] += fmax(0.0, double(s.x) - double(B));
+            const float h = fmaxf(0.f, s.x - B);
+            const float cc = sqrtf(c.g * h);
+            const float d = div_by_h(h, c.epsilon);
+            const float u = d * s.y, w = d * s.z;
+            const float u2v2 = u * u + w * w;
+            q[0] = h; q[1] = h * (B + 0.5f * h); q[2] = s.y; q[3] = s.z;
+            q[4] = (s.y * u + s.z * w);
+            q[5] = u2v2; q[6] = h;
+            q[7] = fmaxf((fabsf(u) + cc) * c.one_over_dx, (fabsf(w) + cc) * c.one_over_dy);
+            q[8] = u2v2 * d;
+        }
+        float sum[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int t = 0; t < 16; ++t)
+            for (int m = 0; m < 5; ++m) sum[m] += __shfl_sync(0xffffffffu, q[m], (lane & 16) + t);
+        for (int off = 8; off; off >>= 1)
+            for (int m = 5; m < 9; ++m) q[m] = fmaxf(q[m], __shfl_xor_sync(0xffffffffu, q[m], off));
+        if (whole && cell == 0) {
             float* o = blocks + (size_t(by) * nbx + bx) * 9;
-            o[0] = sh; o[1] = sb; o[2] = shu; o[3] = shv; o[4] = sk; o[5] = mu; o[6] = mh; o[7] = mc; o[8] = mf;
-            v[0] = sh; v[1] = sb; v[2] = shu; v[3] = shv; v[4] = sk;
-            v[5] = mu; v[6] = mh; v[7] = mc; v[8] = mf;
+            for (int m = 0; m < 5; ++m) { o[m] = sum[m]; v[m] += double(sum[m]); }
+            for (int m = 5; m < 9; ++m) { o[m] = fmaxf(0.f, q[m]); v[m] = fmax(v[m], double(o[m])); }
         }
     }
-    auto is_max = [](int q) { return (q >= 5 && q < 9) || q == 10; };
+    auto is_max = [](int m) { return (m >= 5 && m < 9) || m == 10; };
     auto cta_reduce = [&]() {   // thread 0 ends with the CTA's totals
-        for (int q = 0; q < 11; ++q) {
-            double x = v[q];
+        for (int m = 0; m < 11; ++m) {
+            double a = v[m];
             for (int off = 16; off; off >>= 1) {
-                const double y = __shfl_down_sync(0xffffffffu, x, off);
-                x = is_max(q) ? fmax(x, y) : x + y;
+                const double o = __shfl_down_sync(0xffffffffu, a, off);
+                a = is_max(m) ? fmax(a, o) : a + o;
             }
-            if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5][q] = x;
+            if (lane == 0) sm[threadIdx.x >> 5][m] = a;
         }
         __syncthreads();
-        if (threadIdx.x == 0)
-            for (int q = 0; q < 11; ++q) {
-                v[q] = sm[0][q];
-                for (int w = 1; w < STATS_THREADS / 32; ++w) v[q] = is_max(q) ? fmax(v[q], sm[w][q]) : v[q] + sm[w][q];
-            }
+        if (threadIdx.x < 11) {
+            const int m = threadIdx.x;
+            double a = sm[0][m];
+            for (int w = 1; w < STATS_THREADS / 32; ++w) a = is_max(m) ? fmax(a, sm[w][m]) : a + sm[w][m];
+            v[0] = a;   // thread m holds total m
+        }
     };
     cta_reduce();
-    if (threadIdx.x == 0) {
-        for (int q = 0; q < 11; ++q) part[size_t(blockIdx.x) * 11 + q] = v[q];
+    if (threadIdx.x < 11) {
+        part[size_t(blockIdx.x) * 11 + threadIdx.x] = v[0];
         __threadfence();
-        last = atomicAdd(done, 1u) == gridDim.x - 1;
     }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
     __threadfence();
-    for (int q = 0; q < 11; ++q) v[q] = 0.0;
+    for (int m = 0; m < 11; ++m) v[m] = 0.0;
     for (int b = threadIdx.x; b < int(gridDim.x); b += STATS_THREADS)
-        for (int q = 0; q < 11; ++q) {
-            const double y = __ldcg(part + size_t(b) * 11 + q);
-            v[q] = is_max(q) ? fmax(v[q], y) : v[q] + y;
+        for (int m = 0; m < 11; ++m) {
+            const double a = __ldcg(part + size_t(b) * 11 + m);
+            v[m] = is_max(m) ? fmax(v[m], a) : v[m] + a;
         }
+    __syncthreads();   // the first reduction's reads of sm are done
     cta_reduce();
-    if (threadIdx.x == 0) {
-        for (int q = 0; q < 11; ++q) out[q] = v[q];
-        *done = 0u;
-    }
+    if (threadIdx.x < 11) out[threadIdx.x] = v[0];
+    if (threadIdx.x == 0) *done = 0u;
 }
 
 // AddSolitaryWave (compute.hlsl:949-976) over [1,nx+3)x[1,ny+3), reading a copy of the state
@@ -622,6 +669,9 @@ public:
     Scheme sch;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
+    cudaStream_t sstream = nullptr;          // the statistics run beside the pass that they precede
+    cudaEvent_t ev_state = nullptr, ev_stats = nullptr;
+    bool stats_pending = false;              // ... and the engine's stream has not waited for them yet
     KernelTimer tm;
     Readback rb;
     size_t ntex = 0;
@@ -631,7 +681,8 @@ public:
     // (the reference copies them aside, engine.cpp:1050-1058: 48 bytes a cell and predictor).
     float4 *st[3] = {nullptr, nullptr, nullptr}, *H = nullptr, *U = nullptr, *V = nullptr;
     float4 *AUX1 = nullptr, *AUX2 = nullptr, *BOT = nullptr;
-    float4 *GRAD[4] = {nullptr, nullptr, nullptr, nullptr}, *FG[4] = {nullptr, nullptr, nullptr, nullptr}, *STRIP = nullptr;
+    float4 *GRAD[4] = {nullptr, nullptr, nullptr, nullptr}, *STRIP = nullptr;
+    float2* FG[4] = {nullptr, nullptr, nullptr, nullptr};
     float4* WAVES = nullptr;
     float4 *ABCx = nullptr, *ABCy = nullptr;                        // level-0 systems (the right-hand sides' products)
     float2 *K12x = nullptr, *K12y = nullptr;                        // reduction multipliers of every level
@@ -652,7 +703,10 @@ public:
     int wave_off[4] = {0, 0, 0, 0};
     int sim_idx = 0, cur_i = 0, old_i = 0, oldold_i = 1, scratch_i = 2, spare_i = 3, pred_i = 3;
     int uts_iter[4] = {1, 1, 1, 1};
-    bool bootstrap_needed = true;
+    // Faces belong to the current state (the pass forms them) unless a solitary wave was added since the last
+    // pass: the reference built them at the end of that pass and does not rebuild them then.
+    bool faces_pending = false;   // a pass has run since the last remesh, state or terrain change
+    bool faces_stored = false;    // H, U, V and AUX2 hold the faces of the state before the wave
     std::vector<float> terrain;   // bathymetry grid given by set_bathymetry (used by remesh)
     int terrain_nx = 0, terrain_ny = 0;
     // stats bookkeeping for the latest device-side GetStats
@@ -663,6 +717,9 @@ public:
         for (void* a : allocs) cudaFree(a);
         for (cel_boundary* b : {&p.west, &p.east, &p.south, &p.north})
             if (b->uts) std::free(b->uts);
+        if (sstream) cudaStreamDestroy(sstream);
+        if (ev_state) cudaEventDestroy(ev_state);
+        if (ev_stats) cudaEventDestroy(ev_stats);
         if (own_stream && stream) cudaStreamDestroy(stream);
         (void)cudaGetLastError();   // teardown has no caller to report to; leave no stale error behind
     }
@@ -688,6 +745,9 @@ public:
         CEL_CUDA_TRY(cudaGetDevice(&dev));
         CEL_CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         own_stream = true;
+        CEL_CUDA_TRY(cudaStreamCreateWithFlags(&sstream, cudaStreamNonBlocking));
+        CEL_CUDA_TRY(cudaEventCreateWithFlags(&ev_state, cudaEventDisableTiming));
+        CEL_CUDA_TRY(cudaEventCreateWithFlags(&ev_stats, cudaEventDisableTiming));
         c = make_consts(p, hs, hs.NX);
         ntex = size_t(hs.NX) * hs.NY;
         for (float4** t : {&st[0], &st[1], &st[2], &H, &U, &V, &AUX1, &AUX2, &BOT, &STRIP, &ABCx, &ABCy})
@@ -727,7 +787,7 @@ public:
         const int nb = std::max(1, (hs.nx / 4) * (hs.ny / 4));
         if (int e = dalloc(blocks, size_t(nb) * 9)) return e;
         if (int e = dalloc(dstats, 16)) return e;
-        stats_ctas = (((hs.nx + 3) / 4) * ((hs.ny + 3) / 4) + STATS_THREADS - 1) / STATS_THREADS;
+        stats_ctas = std::min(STATS_CTAS, (((hs.nx + 3) / 4) * ((hs.ny + 3) / 4) * 16 + STATS_THREADS - 1) / STATS_THREADS);
         if (int e = dalloc(spart, size_t(stats_ctas) * 11)) return e;
         if (int e = dalloc(sdone, 1)) return e;
         if (int e = init_boundary()) return e;
@@ -867,13 +927,14 @@ public:
         for (size_t i = 0; i < ntex; ++i) s[i] = make_float4(hs.ic[3 * i], hs.ic[3 * i + 1], hs.ic[3 * i + 2], 0.f);
         CEL_CUDA_TRY(cudaMemcpyAsync(st[0], s.data(), ntex * sizeof(float4), cudaMemcpyHostToDevice, stream));
         CEL_CUDA_TRY(cudaMemcpyAsync(st[1], s.data(), ntex * sizeof(float4), cudaMemcpyHostToDevice, stream));
-        for (float4* t : {H, U, V, AUX1, AUX2, GRAD[0], GRAD[1], GRAD[2], GRAD[3], FG[0], FG[1], FG[2], FG[3]})
+        for (float4* t : {H, U, V, AUX1, AUX2, GRAD[0], GRAD[1], GRAD[2], GRAD[3]})
             CEL_CUDA_TRY(cudaMemsetAsync(t, 0, ntex * sizeof(float4), stream));
+        for (float2* t : FG) CEL_CUDA_TRY(cudaMemsetAsync(t, 0, ntex * sizeof(float2), stream));
         CEL_CUDA_TRY(cudaStreamSynchronize(stream));
         sch.reset(p);
         sim_idx = 0; cur_i = 0; old_i = 0; oldold_i = 1; scratch_i = 2; spare_i = 3; pred_i = 3;
         for (int& u : uts_iter) u = 1;
-        bootstrap_needed = true;
+        faces_pending = faces_stored = false;
         return CEL_OK;
     }
 
@@ -945,13 +1006,19 @@ public:
         }
     }
 
-    int run_stats_kernels() {
+    int run_stats_kernels(cudaStream_t s) {
         (void)cudaGetLastError();
         {
-            TimedLaunch tl(&tm, stream, "plain_stats");
-            k_stats<<<stats_ctas, STATS_THREADS, 0, stream>>>(st[sim_idx], BOT, blocks, c, spart, sdone, dstats);
+            TimedLaunch tl(&tm, s, "plain_stats");
+            k_stats<<<stats_ctas, STATS_THREADS, 0, s>>>(st[sim_idx], BOT, blocks, c, spart, sdone, dstats);
         }
         CEL_CUDA_TRY(cudaGetLastError());
+        return CEL_OK;
+    }
+    int join_stats() {
+        if (!stats_pending) return CEL_OK;
+        stats_pending = false;
+        CEL_CUDA_TRY(cudaStreamWaitEvent(stream, ev_stats, 0));
         return CEL_OK;
     }
 
@@ -975,7 +1042,8 @@ public:
 
     // resetTimestep: GetStats on the current state, then dt (engine.cpp:1536-1756)
     int reset_timestep(float, float, cel_stats* out) override {
-        if (int e = run_stats_kernels()) return e;
+        if (int e = join_stats()) return e;
+        if (int e = run_stats_kernels(stream)) return e;
         double v[16];
         CEL_CUDA_TRY(cudaMemcpyAsync(v, dstats, sizeof(double) * 11, cudaMemcpyDeviceToHost, stream));
         CEL_CUDA_TRY(cudaStreamSynchronize(stream));
@@ -996,7 +1064,14 @@ public:
     // resetTimestep without a host readback (fixed dt); adaptive dt needs the CFL on the host.
     int reset_timestep_device() {
         if (sch.adaptive) return reset_timestep(0.f, 0.f, nullptr);
-        if (int e = run_stats_kernels()) return e;
+        // On a stream of their own, beside the pass that follows (which reads the same state and writes
+        // another one); that pass ends by waiting for them.  5 of 37 us a pass on 512 x 64 cells.
+        if (int e = join_stats()) return e;
+        CEL_CUDA_TRY(cudaEventRecord(ev_state, stream));
+        CEL_CUDA_TRY(cudaStreamWaitEvent(sstream, ev_state, 0));
+        if (int e = run_stats_kernels(sstream)) return e;
+        CEL_CUDA_TRY(cudaEventRecord(ev_stats, sstream));
+        stats_pending = true;
         sch.choose_dt(0.f);
         last_stats_scheme = sch.time_scheme;
         last_stats_dt = sch.dt;
@@ -1005,6 +1080,7 @@ public:
     }
 
     int get_stats(cel_stats* out) override {
+        if (int e = join_stats()) return e;
         double v[16];
         CEL_CUDA_TRY(cudaMemcpyAsync(v, dstats, sizeof(double) * 11, cudaMemcpyDeviceToHost, stream));
         CEL_CUDA_TRY(cudaStreamSynchronize(stream));
@@ -1030,11 +1106,6 @@ public:
         }
         float4* old_state = st[sim_idx];
         float4* new_state = st[out_i];
-        if (bootstrap_needed) {
-            TimedLaunch tl(&tm, stream, "plain_pass1");
-            k_pass1<<<grid2(hs.nx + 2, hs.ny + 2), blk, 0, stream>>>(old_state, BOT, AUX1, H, U, V, AUX2, c);
-            bootstrap_needed = false;
-        }
         Pass3Args a{};
         a.st = old_state; a.bot = BOT; a.H = H; a.U = U; a.V = V; a.aux2 = AUX2; a.aux1 = AUX1;
         a.ABCx = ABCx; a.ABCy = ABCy;
@@ -1045,8 +1116,9 @@ public:
         a.decay = float(std::pow(double(std::fabs(c.whitewater_decay_rate)), double(sch.dt)));
         a.scheme = sch.time_scheme;
         {
-            TimedLaunch tl(&tm, stream, "plain_pass23");
-            k_pass23<<<grid2(hs.NX, hs.NY), blk, 0, stream>>>(a, c);
+            TimedLaunch tl(&tm, stream, "plain_pass123");
+            if (faces_stored) k_pass123<true><<<grid2(hs.NX, hs.NY), blk, 0, stream>>>(a, c);
+            else k_pass123<false><<<grid2(hs.NX, hs.NY), blk, 0, stream>>>(a, c);
         }
         const bool was_predictor = sch.is_predictor();
         // the implicit systems along x and y, in place (engine.cpp:1060-1217)
@@ -1057,11 +1129,10 @@ public:
             k<<<hs.ny + (hs.nx + CR_COLS - 1) / CR_COLS, CR_THREADS, smem_cr, stream>>>(solve, c);
         }
         boundaries(new_state);
-        {
-            TimedLaunch tl(&tm, stream, "plain_pass1");
-            k_pass1<<<grid2(hs.nx + 2, hs.ny + 2), blk, 0, stream>>>(new_state, BOT, AUX1, H, U, V, AUX2, c);
-        }
         CEL_CUDA_TRY(cudaGetLastError());
+        if (int e = join_stats()) return e;
+        faces_pending = true;
+        faces_stored = false;
         const bool book = sch.after_pass();
         if (book) {
             const int o = old_i, oo = oldold_i, s = scratch_i;
@@ -1103,7 +1174,7 @@ public:
     int set_state(const float* rgba) override {
         CEL_CUDA_TRY(cudaMemcpyAsync(st[sim_idx], rgba, ntex * sizeof(float4), cudaMemcpyHostToDevice, stream));
         CEL_CUDA_TRY(cudaStreamSynchronize(stream));
-        bootstrap_needed = true;
+        faces_pending = faces_stored = false;
         return CEL_OK;
     }
     int read_texture(const float4* t, float* rgba) {
@@ -1148,7 +1219,7 @@ public:
         terrain.assign(z, z + size_t(bnx) * bny);
         terrain_nx = bnx;
         terrain_ny = bny;
-        bootstrap_needed = true;
+        faces_pending = faces_stored = false;
         return CEL_OK;
     }
 
@@ -1158,6 +1229,7 @@ public:
         const float W = float(p.width), L = float(p.length);
         if (hs.nx < 4 || hs.ny < 4) { err = "getWaterHeight needs at least one 4x4 block"; return CEL_ERR_STATE; }
         if (!sch.initialized) { if (int e = reset_timestep(0.f, 0.f, nullptr)) return e; }
+        if (int e = join_stats()) return e;
         int ix = 0, iy = 0;
         water_height_block(hs.nx, hs.ny, W, L, x, y, ix, iy);
         float sum_h = 0.f;
@@ -1172,6 +1244,10 @@ public:
         // the state texture is updated in place from a copy; faces are not rebuilt
         // (engine.cpp:2154-2219 leaves bootstrap_needed unchanged)
         float4* s = st[sim_idx];
+        if (faces_pending && !faces_stored) {
+            k_pass1<<<grid2(hs.nx + 2, hs.ny + 2), dim3(BX2, BY2), 0, stream>>>(s, BOT, AUX1, H, U, V, AUX2, c);
+            faces_stored = true;
+        }
         CEL_CUDA_TRY(cudaMemcpyAsync(STRIP, s, ntex * sizeof(float4), cudaMemcpyDeviceToDevice, stream));
         const float th = float(theta_deg) * CEL_PI_HOST / 180.0f;
         k_add_solitary<<<grid2(hs.nx + 2, hs.ny + 2), dim3(BX2, BY2), 0, stream>>>(STRIP, BOT, s, c, float(Hh), th,

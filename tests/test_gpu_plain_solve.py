@@ -37,3 +37,32 @@ def test_plain_sizes_bit_for_bit(celeris, nx, ny, kind):
     assert got["max_depth"] == (float(np.maximum(f(0), st[:ny // 4 * 4, :nx // 4 * 4, 0] - ba[:ny // 4 * 4, :nx // 4 * 4]).max())
                                 if blocks.size else 0.0)
     assert got["health"] == 0
+
+
+def test_faces_of_the_state_before_a_solitary_wave(celeris):
+    """The pass after addSolitaryWave takes the faces (and the record) of the state before it, however many
+    waves were added; a wave before the first pass, a new state and later passes rebuild them."""
+    p, z, bnx, bny = cases.small_case(67, 45, "sponge", correction_steps=1)
+    ref, eng = O.Oracle(p, z, bnx, bny, "f32"), celeris.Engine(p, z, "plain")
+
+    def both(f):
+        f(ref)
+        f(eng)
+
+    def same():
+        assert np.array_equal(eng.state()[..., :3].astype(np.float64), ref.state()[..., :3])
+        np.testing.assert_allclose(eng.aux()[2:-2, 2:-2, 0], ref.aux()[2:-2, 2:-2, 0], rtol=1e-6, atol=1e-7)
+
+    both(lambda e: e.add_solitary_wave(0.1, 10.0, 20.0, 10.0))     # before the first pass
+    both(lambda e: e.physical_steps(4))
+    same()
+    both(lambda e: e.add_solitary_wave(0.2, 30.0, 25.0, 12.0))
+    both(lambda e: e.add_solitary_wave(0.1, -40.0, 35.0, 20.0))
+    both(lambda e: e.physical_steps(3))
+    same()
+    both(lambda e: e.add_solitary_wave(0.05, 0.0, 30.0, 20.0))
+    s = eng.state()
+    eng.set_state(s)
+    ref.set_state(s.astype(np.float64))
+    both(lambda e: e.physical_steps(3))
+    same()
