@@ -1601,8 +1601,9 @@ __global__ void __launch_bounds__(NT, cols_min_ctas(NT)) k_cols(const MemberDev*
     static_assert(NCH % LN == 0, "carry scan layout");
     constexpr int CU = 8;
     extern __shared__ float cs[];
-    __shared__ float carP[NCH][CW], carY[NCH][CW], carQ[NCH][CW], carZ0[NCH][CW], carZ1[NCH][CW];
-    __shared__ float cin_f[NCH][CW], cin_b[NCH][CW];
+    // (rows of CW + 1 words: the carry scans read down a column of these, on 2 to 8 banks without the pad)
+    __shared__ float carP[NCH][CW + 1], carY[NCH][CW + 1], carQ[NCH][CW + 1], carZ0[NCH][CW + 1], carZ1[NCH][CW + 1];
+    __shared__ float cin_f[NCH][CW + 1], cin_b[NCH][CW + 1];
     const int c = threadIdx.x % CW, k = threadIdx.x / CW;
     for (int it = blockIdx.x; it < nbands; it += gridDim.x) {
         const int2 bd = bands[it];
@@ -2710,34 +2711,43 @@ __global__ void k_rcp_selftest(const float* __restrict__ x, float* __restrict__ 
 
 // End of a physical step: advance the clocks by the dt of the step's last pass and, in adaptive
 // batches, shift the controller's dt queue (engine.cpp:1507-1518).
-// One warp per member: the totals of the step's first pass from its strips' partials, added in the
-// order of the strips, so that they depend neither on scheduling nor on the lanes of the batch; then
-// the clock.
-__global__ void k_advance_time(const MemberDev* __restrict__ mems, DtCtl* __restrict__ ctl, int n,
-                               const int2* __restrict__ strips, const double* __restrict__ spart) {
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (i >= n) return;
+// One CTA per member: the totals of the step's first pass from its strips' partials, added in an order
+// that the number of strips fixes, so that they depend neither on scheduling nor on the lanes of the batch;
+// then the clock.  Thread (s, k) adds total k of the strips s, s + ADV_STRIPS, ...: whole lines of the
+// strips' rows of STATS_N doubles.  (One warp per member took 16 us, cold, for the 576 strips of 1024 x
+// 1024 cells, on every step's critical path.)
+constexpr int ADV_STRIPS = 32;
+__global__ void __launch_bounds__(ADV_STRIPS * STATS_N) k_advance_time(const MemberDev* __restrict__ mems,
+                                                                       DtCtl* __restrict__ ctl,
+                                                                       const int2* __restrict__ strips,
+                                                                       const double* __restrict__ spart) {
+    __shared__ double part[ADV_STRIPS][STATS_N];
+    const int i = blockIdx.x, k = threadIdx.x % STATS_N, s = threadIdx.x / STATS_N;
     const MemberDev& M = mems[i];
     const int2 r = strips[i];   // first strip, number of strips
-    double v[STATS_N - 1];
-    for (int k = 0; k < STATS_N - 1; ++k) v[k] = 0.0;
-    for (int t = lane; t < r.y; t += 32)
-        for (int k = 0; k < STATS_N - 1; ++k) {
-            const double a = spart[size_t(r.x + t) * STATS_N + k];
-            v[k] = (k >= 6) ? fmax(v[k], a) : v[k] + a;
+    const bool top = k >= 6;    // maxima and the health flag
+    double v = 0.0;
+    if (k < STATS_N - 1) {
+        const double* p = spart + size_t(r.x) * STATS_N + k;
+#pragma unroll 4
+        for (int t = s; t < r.y; t += ADV_STRIPS) {
+            const double a = p[size_t(t) * STATS_N];
+            v = top ? fmax(v, a) : v + a;
         }
-    for (int off = 16; off; off >>= 1)
-        for (int k = 0; k < STATS_N - 1; ++k) {
-            const double o = __shfl_down_sync(0xffffffffu, v[k], off);
-            v[k] = (k >= 6) ? fmax(v[k], o) : v[k] + o;
+    }
+    part[s][k] = v;
+    __syncthreads();
+    if (s == 0 && k < STATS_N - 1) {
+        for (int q = 1; q < ADV_STRIPS; ++q) v = top ? fmax(v, part[q][k]) : v + part[q][k];
+        M.stats[k] = v;
+    }
+    if (threadIdx.x == STATS_N - 1) {
+        *M.time64 += double(*M.dtp);
+        *M.time32 += *M.dtp;
+        if (ctl) {
+            ctl[i].dt_old_old = ctl[i].dt_old;
+            ctl[i].dt_old = ctl[i].dt;
         }
-    if (lane != 0) return;
-    for (int k = 0; k < STATS_N - 1; ++k) M.stats[k] = v[k];
-    *M.time64 += double(*M.dtp);
-    *M.time32 += *M.dtp;
-    if (ctl) {
-        ctl[i].dt_old_old = ctl[i].dt_old;
-        ctl[i].dt_old = ctl[i].dt;
     }
 }
 
@@ -3125,8 +3135,7 @@ int run_pass(cel_lane* b, bool first_of_step, std::string& err) {
     if (book) {
         const int o = ix.og, oo = ix.oog, sc = ix.scr;
         ix.og = sc; ix.oog = o; ix.scr = oo;
-        k_advance_time<<<(int(b->mem.size()) + 3) / 4, 128, 0, b->stream>>>(b->ddev, b->ctl, int(b->mem.size()), b->mrange,
-                                                                            b->spart);
+        k_advance_time<<<int(b->mem.size()), ADV_STRIPS * STATS_N, 0, b->stream>>>(b->ddev, b->ctl, b->mrange, b->spart);
         B_TRY(cudaGetLastError());
     } else if (was_pred) {
         ix.pred = ix.scr;
