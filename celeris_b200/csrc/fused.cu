@@ -2145,7 +2145,7 @@ __global__ void __launch_bounds__(256, 2) k_cols_cluster(const MemberDev* __rest
 
 // ---------------------------------------------------------------------------------------------
 // Boundary strips (compute.hlsl:985-1309), one side per launch over every member.
-// work item: {member, first strip cell}; 256 strip cells per item, BND_CELLS for a sponge strip
+// work item: {member, first strip cell}; BND_T strip cells per item, BND_CELLS for a sponge strip
 // (its threads take BND_CPT cells each and issue all their loads before the first store), and
 // BND_IRR_CELLS for an irregular wave-maker strip (one cell per warp, its components spread over
 // the lanes).  The narrow strips of the other kinds keep one cell per thread, so they still spread
@@ -2322,21 +2322,30 @@ __device__ __forceinline__ void sponge_apply_d(double gam, double sl, float& w, 
     split_hl(gam * (double(v) + double(lv)), v, lv);
 }
 
-constexpr int BND_CPT = 4;
-constexpr int BND_CELLS = 256 * BND_CPT;
-constexpr int BND_IRR_CELLS = 256 / 32;   // irregular wave-maker strips: one cell per warp
+// A sponge strip is a few loads, an FP64 scaling and the stores a cell; the wave-makers' FP64 functions set
+// the registers.  With CTAs of 256 threads, four cells each, two an SM, the loads in flight bound it.  128
+// threads with two cells each, five CTAs an SM at 96 registers (112 B spilled), took the 2048 x 2048 coast's
+// launch from 26.6 to 22.5 us, 40 members' from 20.7 to 16.4, 8 members' of 256 x 256 from 12.1 to 10.0.
+// Six an SM spill 464 B (8 members 95.3 us a step for 94.2), four are too few (coast 24.6 us).
+constexpr int BND_T = 128;
+constexpr int BND_CPT = 2;
+constexpr int BND_CELLS = BND_T * BND_CPT;
+constexpr int BND_IRR_CELLS = BND_T / 32;   // irregular wave-maker strips: one cell per warp
 
 __host__ __device__ __forceinline__ int boundary_item_cells(int type) {
-    return type == CEL_BC_SPONGE ? BND_CELLS : type == CEL_BC_IRREGULAR ? BND_IRR_CELLS : 256;
+    return type == CEL_BC_SPONGE ? BND_CELLS : type == CEL_BC_IRREGULAR ? BND_IRR_CELLS : BND_T;
 }
 
 // One work item of side `side`: boundary_item_cells cells from `first` on of the rectangle (x0, y0, sw, sh).
 // phase 0: compute and write in place; 1: compute into the member's scratch; 2: copy back.
-template <bool MIXED>
-__device__ __noinline__ void boundary_item(const MemberDev& M, int side, int phase, int out, int x0, int y0, int sw, int sh,
+// ONCE: the launch that draws all sides, where phase is 0: without the other phases' code its wave-makers and
+// sponges fit the registers of five CTAs an SM.
+template <bool MIXED, bool ONCE>
+__device__ __forceinline__ void boundary_item(const MemberDev& M, int side, int phase_, int out, int x0, int y0, int sw, int sh,
                                               int first) {
     constexpr int SS = MIXED ? 6 : 3;   // strip floats per cell: w, hu, hv (+ their low words)
-    const SimConsts c = M.c;
+    const SimConsts& c = M.c;
+    const int phase = ONCE ? 0 : phase_;
     const BoundaryDesc& b = M.bd[side];
     const int NX = c.NX, NY = c.NY, P = M.P;
     float* W = M.S[out][0];
@@ -2356,7 +2365,7 @@ __device__ __noinline__ void boundary_item(const MemberDev& M, int side, int pha
         bool ok[BND_CPT];
 #pragma unroll
         for (int k = 0; k < BND_CPT; ++k) {
-            const int cell = first + k * 256 + threadIdx.x;
+            const int cell = first + k * BND_T + threadIdx.x;
             ok[k] = cell < cend;
             cx[k] = x0 + cell % sw; cy[k] = y0 + cell / sw;
             gi[k] = size_t(cy[k]) * P + cx[k];
@@ -2421,7 +2430,7 @@ __device__ __noinline__ void boundary_item(const MemberDev& M, int side, int pha
     }
     const int cpt = (b.type == CEL_BC_SPONGE) ? BND_CPT : 1;
     for (int k = 0; k < cpt; ++k) {
-        const int cell = first + k * 256 + threadIdx.x;
+        const int cell = first + k * BND_T + threadIdx.x;
         if (cell >= cend) break;   // cells ascend with k
         const int x = x0 + cell % sw, y = y0 + cell / sw;
         const size_t gi = size_t(y) * P + x;
@@ -2509,13 +2518,13 @@ __device__ __forceinline__ Rect side_strip(const MemberDev& M, int side) {
 
 // One side's launch (members whose sides cannot run together, boundary_plan.hpp)
 template <bool MIXED>
-__global__ void __launch_bounds__(256, 2) k_boundary(const MemberDev* __restrict__ mems, const int2* __restrict__ items,
+__global__ void __launch_bounds__(BND_T, 4) k_boundary(const MemberDev* __restrict__ mems, const int2* __restrict__ items,
                                                   int nitems, int side, int phase, int out) {
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const int2 wi = items[it];
         const MemberDev& M = mems[wi.x];
         const Rect r = side_strip(M, side);
-        boundary_item<MIXED>(M, side, phase, out, r.x0, r.y0, r.x1 - r.x0, r.y1 - r.y0, wi.y);
+        boundary_item<MIXED, false>(M, side, phase, out, r.x0, r.y0, r.x1 - r.x0, r.y1 - r.y0, wi.y);
     }
 }
 
@@ -2526,7 +2535,7 @@ __global__ void __launch_bounds__(256, 2) k_boundary(const MemberDev* __restrict
 // each were bound by launch latency, 2.4 us a graph node on 512 x 64 cells: us per step there 57.4 ->
 // 43.3, harbour 1017 x 643 (3 passes) 243 -> 182, 1024 x 1024 176 -> 156, 2048 x 2048 490 -> 461.
 template <bool MIXED>
-__global__ void __launch_bounds__(256, 2) k_boundary_all(const MemberDev* __restrict__ mems, const int4* __restrict__ items,
+__global__ void __launch_bounds__(BND_T, 5) k_boundary_all(const MemberDev* __restrict__ mems, const int4* __restrict__ items,
                                                          int nitems, int out) {
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const int4 wi = items[it];
@@ -2543,7 +2552,7 @@ __global__ void __launch_bounds__(256, 2) k_boundary_all(const MemberDev* __rest
             const int cells = boundary_item_cells(M.bd[side].type);
             const int begin = corner ? 0 : wi.z, end = corner ? n : min(n, wi.z + 1);
             for (int first = begin; first < end; first += cells)
-                boundary_item<MIXED>(M, side, 0, out, x0, y0, x1 - x0, y1 - y0, first);
+                boundary_item<MIXED, true>(M, side, 0, out, x0, y0, x1 - x0, y1 - y0, first);
             if (corner) __syncthreads();   // (uniform: the whole CTA is on this item)
         }
     }
@@ -3029,26 +3038,26 @@ int launch_pass(cel_lane* b, const PassArgs& pa, std::string& err) {
     B_TRY(cudaEventRecord(b->ev_join, b->side));
     B_TRY(cudaStreamWaitEvent(b->stream, b->ev_join, 0));
     if (b->nball > 0) {
-        const int g = std::min(b->nball, b->sms * 8);
+        const int g = std::min(b->nball, b->sms * 16);
         TimedLaunch t(&b->tm, b->stream, "boundary");
-        if (b->mixed) k_boundary_all<true><<<g, 256, 0, b->stream>>>(b->ddev, b->ball, b->nball, pa.out);
-        else k_boundary_all<false><<<g, 256, 0, b->stream>>>(b->ddev, b->ball, b->nball, pa.out);
+        if (b->mixed) k_boundary_all<true><<<g, BND_T, 0, b->stream>>>(b->ddev, b->ball, b->nball, pa.out);
+        else k_boundary_all<false><<<g, BND_T, 0, b->stream>>>(b->ddev, b->ball, b->nball, pa.out);
     }
     for (int side : {1, 0, 3, 2}) {
         if (b->nbitems[side] == 0) continue;
-        const int g = std::min(b->nbitems[side], b->sms * 8);
+        const int g = std::min(b->nbitems[side], b->sms * 16);
         TimedLaunch t(&b->tm, b->stream, "boundary");
         if (b->two_phase[side]) {
             if (b->mixed) {
-                k_boundary<true><<<g, 256, 0, b->stream>>>(b->ddev, b->bitems[side], b->nbitems[side], side, 1, pa.out);
-                k_boundary<true><<<g, 256, 0, b->stream>>>(b->ddev, b->bitems[side], b->nbitems[side], side, 2, pa.out);
+                k_boundary<true><<<g, BND_T, 0, b->stream>>>(b->ddev, b->bitems[side], b->nbitems[side], side, 1, pa.out);
+                k_boundary<true><<<g, BND_T, 0, b->stream>>>(b->ddev, b->bitems[side], b->nbitems[side], side, 2, pa.out);
             } else {
-                k_boundary<false><<<g, 256, 0, b->stream>>>(b->ddev, b->bitems[side], b->nbitems[side], side, 1, pa.out);
-                k_boundary<false><<<g, 256, 0, b->stream>>>(b->ddev, b->bitems[side], b->nbitems[side], side, 2, pa.out);
+                k_boundary<false><<<g, BND_T, 0, b->stream>>>(b->ddev, b->bitems[side], b->nbitems[side], side, 1, pa.out);
+                k_boundary<false><<<g, BND_T, 0, b->stream>>>(b->ddev, b->bitems[side], b->nbitems[side], side, 2, pa.out);
             }
         } else {
-            if (b->mixed) k_boundary<true><<<g, 256, 0, b->stream>>>(b->ddev, b->bitems[side], b->nbitems[side], side, 0, pa.out);
-            else k_boundary<false><<<g, 256, 0, b->stream>>>(b->ddev, b->bitems[side], b->nbitems[side], side, 0, pa.out);
+            if (b->mixed) k_boundary<true><<<g, BND_T, 0, b->stream>>>(b->ddev, b->bitems[side], b->nbitems[side], side, 0, pa.out);
+            else k_boundary<false><<<g, BND_T, 0, b->stream>>>(b->ddev, b->bitems[side], b->nbitems[side], side, 0, pa.out);
         }
     }
     B_TRY(cudaGetLastError());
@@ -3637,7 +3646,7 @@ cel_lane* lane_create(int n, const cel_params* const* params, const float* const
                     if (n <= 0) continue;
                     // pieces of about one item of the costlier side
                     const int cells = std::min({boundary_item_cells(btype[corner_side(k - 4, 0)]),
-                                                boundary_item_cells(btype[corner_side(k - 4, 1)]), 256});
+                                                boundary_item_cells(btype[corner_side(k - 4, 1)]), BND_T});
                     const Rect& r = d.breg[k];
                     const CornerCut cut = corner_cut(k - 4, btype);
                     const int across = cut == CUT_ROWS ? r.x1 - r.x0 : r.y1 - r.y0, len = std::max(1, cells / across);
