@@ -425,7 +425,11 @@ def main():
     # the paired-row stencil rebuilds the bottom from the corner grid (4 B); the one-row stencil
     # reads BA, BX and BY (12 B)
     bottom = 0.0 if batch.stencil_rows == 2 else 8.0
-    stencil_bytes_cell = ((104 + bottom + comp) + N * (128 + bottom + comp)) / (1 + N)  # average over pass kinds
+    # a predictor reads state 12, corners 4, two steps' rates 40 and aux 8 and writes w 4, right-hand sides 8, aux 8 and
+    # its combination of the rates for the corrector 12 (without correctors its own rates, 20); a corrector reads
+    # state 12, corners 4, that combination 12, aux 8 and w 4 and writes 4 + 8 + 8 and its rates, 20
+    pred_bytes, corr_bytes = (96 if N else 104) + bottom + comp, 80 + bottom + comp
+    stencil_bytes_cell = (pred_bytes + N * corr_bytes) / (1 + N)  # average over pass kinds
     avg_launch_s = st_ms / max(st_n, 1) / 1e3
     cells_launch = cells / lanes
     achieved = stencil_bytes_cell * cells_launch / avg_launch_s / 1e9 if avg_launch_s > 0 else 0.0
@@ -437,16 +441,18 @@ def main():
         peak, peak_src = 6650.0, "fallback"
     # DRAM bytes per cell of one stencil launch measured by ncu (dram__bytes_read.sum +
     # dram__bytes_write.sum / cells) on the first 8 members of this ensemble in one lane, mixed form,
-    # paired-row stencil at 96 threads per strip (corner-grid bottom): predictor 106.9, corrector
-    # 132.9; scaled here to this launch's cells.
-    ncu_bytes_cell = {"mixed": (106.9, 132.9)}
+    # paired-row stencil at 128 threads per strip: predictor 99.9, corrector 80.2; scaled here to this
+    # launch's cells.
+    ncu_bytes_cell = {"mixed": (99.9, 80.2)}
     traffic = None
     if args.form in ncu_bytes_cell:
         pb, cbytes = ncu_bytes_cell[args.form]
         traffic = (pb + N * cbytes) / (1 + N) * cells_launch
     total_kernel_ms = sum(v[0] for v in kt.values())
     shares = {k: round(v[0] / total_kernel_ms, 4) for k, v in kt.items()} if total_kernel_ms > 0 else {}
-    step_bytes = cb.byte_model(args.form, N)[1]
+    # a pass's two solves read the right-hand sides, three factors each and their base and write 8 (16 more
+    # with the low words)
+    step_bytes = pred_bytes + N * corr_bytes + (1 + N) * (48 + 2 * comp)
 
     # ---- per-domain forms (the comparison): each member its own engine, launched one after another
     def per_domain(form: str, psteps: int = 30):

@@ -1,19 +1,21 @@
 // Fused, batched B200 form of the Celeris timestep path.
 //
 // One pass (predictor, corrector or Euler) of every domain in a batch is three kernels plus the
-// boundary kernels, each launched once for all domains over a cross-domain work list:
-//   k_march    : Pass1 (minmod reconstruction, positivity fix, desingularised velocities) +
+// boundary kernel, each launched once for all domains over a cross-domain work list:
+//   k_march2   : Pass1 (minmod reconstruction, positivity fix, desingularised velocities) +
 //                Pass2 (Kurganov-Petrova central-upwind fluxes) + Pass3Predictor (flux
 //                divergence, bed slope, friction, Madsen-Sorensen dispersion, F*/G*, AB3/AM4
 //                combination) + white-water/inundation aux + the GetStats reduction, marching
-//                down 126-column strips with a 6-row shared-memory ring.  It writes the new w
+//                down strips of 126 or 94 columns two rows at a time with a shared-memory ring of
+//                six row pairs (k_march: one row at a time).  It writes the new w
 //                and, for hu and hv, the right-hand side of the implicit dispersive system in
 //                increment form: M dhu = r, hu_new = hu_base + dhu.
-//   k_rows / k_cols : the tridiagonal solves along x (one CTA per row) and y (one CTA per band
+//   k_rows / k_cols : the tridiagonal solves along x (one warp per row) and y (one CTA per band
 //                of 16 columns), a chunked Thomas elimination whose forward and backward sweeps
 //                are first-order linear recurrences combined across chunks by a scan; the
 //                time-invariant LU factors are precomputed per domain.
-//   k_boundary : East, North, West, South strips in the reference's order (one launch each).
+//   k_boundary_all : the four strips in the reference's order, corners apart (boundary_plan.hpp); members
+//                whose sides depend on one another take k_boundary, one launch a side.
 // The whole physical step (predictor + correctors) is captured once per buffer-rotation phase
 // into CUDA graphs and replayed.
 //
@@ -2144,7 +2146,8 @@ __global__ void __launch_bounds__(256, 2) k_cols_cluster(const MemberDev* __rest
 }
 
 // ---------------------------------------------------------------------------------------------
-// Boundary strips (compute.hlsl:985-1309), one side per launch over every member.
+// Boundary strips (compute.hlsl:985-1309) over every member: all sides in one launch (k_boundary_all), or
+// one side per launch (k_boundary).
 // work item: {member, first strip cell}; BND_T strip cells per item, BND_CELLS for a sponge strip
 // (its threads take BND_CPT cells each and issue all their loads before the first store), and
 // BND_IRR_CELLS for an irregular wave-maker strip (one cell per warp, its components spread over
@@ -3206,8 +3209,10 @@ int build_graphs(cel_lane* b, std::string& err) {
 }  // namespace
 
 void byte_model(int form, int N, double& stencil, double& step) {
-    // Algorithmic HBM bytes per interior cell (compulsory traffic of this design), for the
-    // paired-row stencil (k_march2), which rebuilds the bottom from the corner grid:
+    // Algorithmic HBM bytes per interior cell of a step whose every pass keeps its rates, the figure this
+    // entry point has always returned.  A predictor that hands its correctors one combination of the rates
+    // moves 8 fewer and a corrector 48 fewer (96 and 80).  For the paired-row stencil (k_march2), which
+    // rebuilds the bottom from the corner grid:
     //  stencil, predictor: read state 12 + corner grid 4 + history 40 + aux 8;
     //                      write w 4 + rhs 8 + history 20 + aux 8  -> 104
     //  stencil, corrector: + predicted history 20 + CURRENT_STATE w 4  -> 128

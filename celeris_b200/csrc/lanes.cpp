@@ -7,8 +7,8 @@
 // for at its end (a join), so to the caller a batch behaves as one stream-ordered object.  A step
 // launches the lanes' graphs in turn, one physical step at a time, and the GPU runs them side by
 // side: one lane's boundary strips, clock advance and kernel tails, which leave most SMs idle,
-// overlap another lane's stencil.  Every member's arithmetic is the same in any lane, so the
-// results do not depend on the split.
+// overlap another lane's stencil.  Every member's arithmetic is the same in any lane, and every lane
+// takes the strip split of the whole batch, so neither results nor statistics depend on the split.
 #include <algorithm>
 #include <memory>
 #include <numeric>
