@@ -383,6 +383,26 @@ __device__ __forceinline__ void cr_solve(const CrLevels& L, float* __restrict__ 
     }
 }
 
+// A level's coefficients as k_cr reads them, from its textures (2 texels of border; pitch len + 4 in rows, NX in
+// columns): for equation i of system s the two multipliers, from the level before, and for every second
+// one its own three.
+__global__ void k_pack_level(const float4* __restrict__ prev, const float4* __restrict__ cur, bool rows, int n, int len,
+                             int prev_pitch, int NX, float2* __restrict__ k12, float4* __restrict__ acb) {
+    const size_t e = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (e >= size_t(len) * n) return;
+    const int s = int(rows ? e / len : e % n), i = int(rows ? e % len : e / n);
+    if (prev) {
+        const size_t si = rows ? 1 : NX;
+        const float4* p = prev + size_t(s + 2) * (rows ? prev_pitch : 1) + size_t(2 * i + 2) * si;
+        k12[e] = make_float2(p[si].x / p[0].y, p[si].z / p[2 * si].y);
+    }
+    const int half = (len + 1) / 2;
+    if (i < half) {
+        const float4 q = cur[size_t(s + 2) * (rows ? len + 4 : 1) + size_t(2 * i + 2) * (rows ? 1 : NX)];
+        acb[rows ? size_t(s) * half + i : size_t(i) * n + s] = make_float4(q.x, q.z, q.y, 0.f);
+    }
+}
+
 // SMEM_X / SMEM_Y: the rows' / the columns' levels fit in shared memory.
 template <bool SMEM_X, bool SMEM_Y>
 __global__ void __launch_bounds__(CR_THREADS) k_cr(SolveArgs a, SimConsts c) {
@@ -861,53 +881,30 @@ public:
         return upload_solve();
     }
 
-    // The solve's coefficients from the host's levels, on the engine's stream.
+    // The solve's coefficients from the host's levels, on the engine's stream.  Packed on the device (on the
+    // host it took 11 of the 89 ms of a 1001 x 777 engine's creation): levels above the first pass through H and U,
+    // which every caller clears next.
     int upload_solve() {
-        // texel (i + 2) of system s (from 0) of a level
-        auto pack = [](const std::vector<std::vector<Float4>>& abc, const CrLevels& L, bool rows, int n, int NX,
-                       std::vector<float2>& k12, std::vector<float4>& acb) {
-            for (int k = 0; k < L.K; ++k) {
-                const size_t ss = rows ? size_t(L.len[k] + 4) : 1, si = rows ? 1 : size_t(NX);
-                const size_t ps = k > 0 && rows ? size_t(L.len[k - 1] + 4) : 1;
-                const int half = (L.len[k] + 1) / 2;
-                auto equation = [&](int s, int i, size_t to) {
-                    const Float4* p = &abc[k - 1][size_t(s + 2) * ps + size_t(2 * i + 2) * si];
-                    k12[L.koff[k] + to] = make_float2(p[si].x / p[0].y, p[si].z / p[2 * si].y);
-                };
-                auto even = [&](int s, int j, size_t to) {
-                    const Float4& q = abc[k][size_t(s + 2) * ss + size_t(2 * j + 2) * si];
-                    acb[L.soff[k] + to] = make_float4(q.x, q.z, q.y, 0.f);
-                };
-                if (rows) {
-                    for (int s = 0; s < n; ++s) {
-                        for (int i = 0; k > 0 && i < L.len[k]; ++i) equation(s, i, size_t(s) * L.len[k] + i);
-                        for (int j = 0; j < half; ++j) even(s, j, size_t(s) * half + j);
-                    }
-                } else {
-                    for (int i = 0; k > 0 && i < L.len[k]; ++i)
-                        for (int s = 0; s < n; ++s) equation(s, i, size_t(i) * n + s);
-                    for (int j = 0; j < half; ++j)
-                        for (int s = 0; s < n; ++s) even(s, j, size_t(j) * n + s);
-                }
-            }
-        };
         for (const bool rows : {true, false}) {
             const CrLevels& L = rows ? solve.x : solve.y;
-            const int n = rows ? hs.ny : hs.nx;
-            size_t equations = 0, evens = 0;
-            for (int k = 0; k < L.K; ++k) {
-                if (k > 0) equations += size_t(L.len[k]) * n;
-                evens += size_t((L.len[k] + 1) / 2) * n;
-            }
-            std::vector<float2> k12(equations);
-            std::vector<float4> acb(evens);
             const auto& abc = rows ? hs.ABCx : hs.ABCy;
-            pack(abc, L, rows, n, hs.NX, k12, acb);
-            CEL_CUDA_TRY(cudaMemcpyAsync(rows ? ABCx : ABCy, abc[0].data(), ntex * sizeof(float4), cudaMemcpyHostToDevice, stream));
-            CEL_CUDA_TRY(cudaMemcpyAsync(rows ? K12x : K12y, k12.data(), k12.size() * sizeof(float2), cudaMemcpyHostToDevice, stream));
-            CEL_CUDA_TRY(cudaMemcpyAsync(rows ? ACBx : ACBy, acb.data(), acb.size() * sizeof(float4), cudaMemcpyHostToDevice, stream));
-            CEL_CUDA_TRY(cudaStreamSynchronize(stream));   // before the host copies go out of scope
+            const float4* prev = nullptr;
+            for (int k = 0; k < L.K; ++k) {
+                float4* cur = k == 0 ? (rows ? ABCx : ABCy) : (k & 1) ? H : U;
+                const size_t count = k == 0 ? ntex : abc[k].size();
+                if (count > ntex) { err = "a cyclic reduction level is larger than the domain"; return CEL_ERR_CUDA; }
+                CEL_CUDA_TRY(cudaMemcpyAsync(cur, abc[k].data(), count * sizeof(float4), cudaMemcpyHostToDevice, stream));
+                const int n = rows ? hs.ny : hs.nx, len = L.len[k];
+                const size_t total = size_t(len) * n;
+                if (total)
+                    k_pack_level<<<unsigned((total + 255) / 256), 256, 0, stream>>>(
+                        prev, cur, rows, n, len, k > 0 && rows ? L.len[k - 1] + 4 : 0, hs.NX, (rows ? K12x : K12y) + L.koff[k],
+                        (rows ? ACBx : ACBy) + L.soff[k]);
+                CEL_CUDA_TRY(cudaGetLastError());
+                prev = cur;
+            }
         }
+        CEL_CUDA_TRY(cudaStreamSynchronize(stream));   // before the host copies go out of scope
         return CEL_OK;
     }
 
