@@ -441,9 +441,9 @@ def main():
         peak, peak_src = 6650.0, "fallback"
     # DRAM bytes per cell of one stencil launch measured by ncu (dram__bytes_read.sum +
     # dram__bytes_write.sum / cells) on the first 8 members of this ensemble in one lane, mixed form,
-    # paired-row stencil at 128 threads per strip: predictor 99.9, corrector 80.2; scaled here to this
+    # paired-row stencil at 128 threads per strip: predictor 99.7, corrector 79.9; scaled here to this
     # launch's cells.
-    ncu_bytes_cell = {"mixed": (99.9, 80.2)}
+    ncu_bytes_cell = {"mixed": (99.7, 79.9)}
     traffic = None
     if args.form in ncu_bytes_cell:
         pb, cbytes = ncu_bytes_cell[args.form]
