@@ -29,6 +29,7 @@ UNITS = [
     ("capi.cpp", []),
     ("lanes.cpp", []),
     ("plain.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
+    ("readback.cpp", []),
     ("readback.cu", []),
     ("fused.cu", ["-prec-div=false", "-prec-sqrt=false", "-ftz=true"]),
 ]

@@ -3926,21 +3926,19 @@ static int read_texels(cel_lane* b, int i, PackMode mode, float* rgba, std::stri
     a.mode = mode;
     (void)cudaGetLastError();
     const size_t bytes = size_t(m.hs.NX) * m.hs.NY * sizeof(float4);
-    if (bytes <= READBACK_DIRECT) {
-        // small: formed in the history slot that the next pass overwrites (4 planes of at least NX columns),
-        // then one copy
-        float4* scratch = d.HA[b->ix.scr];
-        B_TRY(launch_pack(a, 0, bytes / sizeof(float4), scratch, b->stream));
-        B_TRY(cudaMemcpyAsync(rgba, scratch, bytes, cudaMemcpyDeviceToHost, b->stream));
-        B_TRY(cudaStreamSynchronize(b->stream));
-        return CEL_OK;
-    }
-    return b->rb.read(rgba, bytes, b->stream,
-                      [&](size_t off, size_t n, char* slot) {
-                          return launch_pack(a, off / sizeof(float4), n / sizeof(float4), reinterpret_cast<float4*>(slot),
-                                             b->stream);
-                      },
-                      err);
+    return b->rb.read(
+        rgba, bytes, b->stream,
+        [&](char* dst) {
+            // formed in the history slot that the next pass overwrites (4 planes of at least NX columns), then
+            // one copy
+            float4* scratch = d.HA[b->ix.scr];
+            cudaError_t e = launch_pack(a, 0, bytes / sizeof(float4), scratch, b->stream);
+            return e == cudaSuccess ? cudaMemcpyAsync(dst, scratch, bytes, cudaMemcpyDeviceToHost, b->stream) : e;
+        },
+        [&](size_t off, size_t n, char* slot) {
+            return launch_pack(a, off / sizeof(float4), n / sizeof(float4), reinterpret_cast<float4*>(slot), b->stream);
+        },
+        err);
 }
 
 // The state as two float textures whose sum is the compensated value: hi = the stored state, lo =

@@ -1175,16 +1175,14 @@ public:
         return CEL_OK;
     }
     int read_texture(const float4* t, float* rgba) {
-        if (ntex * sizeof(float4) <= READBACK_DIRECT) {
-            CEL_CUDA_TRY(cudaMemcpyAsync(rgba, t, ntex * sizeof(float4), cudaMemcpyDeviceToHost, stream));
-            CEL_CUDA_TRY(cudaStreamSynchronize(stream));
-            return CEL_OK;
-        }
-        return rb.read(rgba, ntex * sizeof(float4), stream,
-                       [&](size_t off, size_t n, char* slot) {
-                           return cudaMemcpyAsync(slot, reinterpret_cast<const char*>(t) + off, n, cudaMemcpyDeviceToHost, stream);
-                       },
-                       err);
+        const size_t bytes = ntex * sizeof(float4);
+        return rb.read(
+            rgba, bytes, stream,
+            [&](char* dst) { return cudaMemcpyAsync(dst, t, bytes, cudaMemcpyDeviceToHost, stream); },
+            [&](size_t off, size_t n, char* slot) {
+                return cudaMemcpyAsync(slot, reinterpret_cast<const char*>(t) + off, n, cudaMemcpyDeviceToHost, stream);
+            },
+            err);
     }
     int get_state(float* rgba) override {
         return read_texture(st[sim_idx], rgba);

@@ -36,12 +36,15 @@ public:
     Readback(const Readback&) = delete;
     Readback& operator=(const Readback&) = delete;
     ~Readback();
-    // dst[0, bytes): enqueue(offset, n, slot) puts the work that fills slot[0, n) with the bytes from
-    // `offset` on the stream; it may be called from helper threads.  Returns a CEL_* status.
-    int read(void* dst, size_t bytes, cudaStream_t s,
-             const std::function<cudaError_t(size_t offset, size_t n, char* slot)>& enqueue, std::string& err);
+    // Fills dst[0, bytes) and waits.  part(offset, n, slot) puts the work that fills slot[0, n) with the
+    // bytes from `offset` on the stream; it may be called from helper threads.  whole(dst) puts work and one
+    // copy there that fill dst at once: for reads up to READBACK_DIRECT, and where there are no slots to be
+    // had (a limit on pinned memory).  Returns a CEL_* status.
+    int read(void* dst, size_t bytes, cudaStream_t s, const std::function<cudaError_t(char* dst)>& whole,
+             const std::function<cudaError_t(size_t offset, size_t n, char* slot)>& part, std::string& err);
 
 private:
+    int read_whole(char* dst, cudaStream_t s, const std::function<cudaError_t(char* dst)>& whole, std::string& err);
     cudaEvent_t ev_[READBACK_SLOTS] = {};   // created by the first read through slots
 };
 
