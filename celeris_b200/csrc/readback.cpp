@@ -57,9 +57,28 @@ void give_block(char* p) {
     cudaFreeHost(p);
 }
 
+// The owner's device for the length of a read: launches and events need it current (a new thread starts on
+// device 0).
+class OnDevice {
+public:
+    explicit OnDevice(int dev) {
+        if (dev >= 0 && cudaGetDevice(&before_) == cudaSuccess && before_ != dev) moved_ = cudaSetDevice(dev) == cudaSuccess;
+    }
+    OnDevice(const OnDevice&) = delete;
+    OnDevice& operator=(const OnDevice&) = delete;
+    ~OnDevice() {
+        if (moved_) cudaSetDevice(before_);
+    }
+
+private:
+    int before_ = 0;
+    bool moved_ = false;
+};
+
 }  // namespace
 
 Readback::Readback() {
+    if (cudaGetDevice(&dev_) != cudaSuccess) dev_ = -1;
     std::lock_guard<std::mutex> lock(g_pool_mutex);
     g_pool.reserve(READBACK_CACHED);
     ++g_users;
@@ -86,6 +105,7 @@ int Readback::read_whole(char* dst, cudaStream_t s, const std::function<cudaErro
 int Readback::read(void* dst, size_t bytes, cudaStream_t s, const std::function<cudaError_t(char* dst)>& whole,
                    const std::function<cudaError_t(size_t offset, size_t n, char* slot)>& part, std::string& err) {
     if (bytes == 0) return CEL_OK;
+    const OnDevice on(dev_);
     if (bytes <= READBACK_DIRECT) return read_whole(static_cast<char*>(dst), s, whole, err);
     const size_t chunk = std::min(READBACK_SLOT, bytes);
     const size_t chunks = (bytes + chunk - 1) / chunk;
@@ -95,7 +115,7 @@ int Readback::read(void* dst, size_t bytes, cudaStream_t s, const std::function<
     cudaError_t first = cudaSuccess;
     for (int k = 0; k < READBACK_SLOTS && first == cudaSuccess; ++k)
         if (!ev_[k]) first = cudaEventCreateWithFlags(&ev_[k], cudaEventDisableTiming);
-    int dev = 0;
+    int dev = 0;   // for the helper threads
     if (first == cudaSuccess) first = cudaGetDevice(&dev);
     char* const block = first == cudaSuccess ? take_block(first) : nullptr;
     if (!block) {   // no slots (a limit on pinned memory): one copy needs none

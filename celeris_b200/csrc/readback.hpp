@@ -32,7 +32,7 @@ constexpr int READBACK_SLOTS = 2 * READBACK_WORKERS;
 constexpr int READBACK_CACHED = 4;
 class Readback {
 public:
-    Readback();
+    Readback();   // on its owner's device, where every read runs, whichever device is current in the caller's thread
     Readback(const Readback&) = delete;
     Readback& operator=(const Readback&) = delete;
     ~Readback();
@@ -45,6 +45,7 @@ public:
 
 private:
     int read_whole(char* dst, cudaStream_t s, const std::function<cudaError_t(char* dst)>& whole, std::string& err);
+    int dev_ = -1;                          // the owner's device
     cudaEvent_t ev_[READBACK_SLOTS] = {};   // created by the first read through slots
 };
 

@@ -115,6 +115,17 @@ int main(int argc, char** argv) {
             g_refuse_pinned = g_refuse_events = false;
             Readback rb;   // and the slots again once there are some
             if (src.read(rb, dst.data(), own, err) != CEL_OK || (src.parts == 0) != small) return fail("slots not tried again");
+        } else if (rule == "device") {   // a thread whose current device is another one than the engine's
+            g_engine_device = t_device = 1;
+            {
+                Readback rb;
+                t_device = 0;
+                for (int k = 0; k < 2; ++k) {
+                    if (src.read(rb, dst.data(), own, err) != CEL_OK || dst != src.data) return fail("wrong bytes");
+                    if (t_device != 0) return fail("the caller's device was changed");
+                }
+            }
+            if (g_wrong_device != 0) return fail("called on the wrong device");
         } else {
             return fail("unknown rule");
         }
