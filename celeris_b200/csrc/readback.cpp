@@ -107,6 +107,19 @@ int Readback::read(void* dst, size_t bytes, cudaStream_t s, const std::function<
     if (bytes == 0) return CEL_OK;
     const OnDevice on(dev_);
     if (bytes <= READBACK_DIRECT) return read_whole(static_cast<char*>(dst), s, whole, err);
+    // Memory that the runtime knows is copied into at once.  Pinned by the caller it takes the bus's rate, and
+    // the slots' host copy only adds to that (plain form, 2052 x 2052 texels 2.6 -> 1.2 ms, 704 x 504 0.52 -> 0.11);
+    // the host must not write into device memory.
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
+        (void)cudaGetLastError();
+        at.type = cudaMemoryTypeUnregistered;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) {
+        const int st = read_whole(static_cast<char*>(dst), s, whole, err);
+        if (st == CEL_OK || at.type == cudaMemoryTypeDevice) return st;
+        (void)cudaGetLastError();   // such as memory that is registered in part: through slots
+    }
     const size_t chunk = std::min(READBACK_SLOT, bytes);
     const size_t chunks = (bytes + chunk - 1) / chunk;
     // starting a thread takes as long as copying a few hundred kB

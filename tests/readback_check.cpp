@@ -126,6 +126,24 @@ int main(int argc, char** argv) {
                 }
             }
             if (g_wrong_device != 0) return fail("called on the wrong device");
+        } else if (rule == "pinned") {   // memory that the runtime knows: one copy, as into any small destination
+            g_known = dst.data();
+            g_known_end = g_known + n;
+            Readback rb;
+            for (cudaMemoryType type : {cudaMemoryTypeHost, cudaMemoryTypeManaged}) {
+                g_known_type = type;
+                const int before = src.wholes;
+                std::fill(dst.begin(), dst.end(), 0);
+                if (src.read(rb, dst.data(), own, err) != CEL_OK || dst != src.data) return fail("wrong bytes");
+                if (src.wholes != before + 1 || src.parts != 0) return fail("not copied into at once");
+            }
+            src.whole_error = cudaErrorInvalidValue;   // such as memory that is only partly registered: slots
+            g_known_type = cudaMemoryTypeHost;
+            std::fill(dst.begin(), dst.end(), 0);
+            const int st = src.read(rb, dst.data(), own, err);
+            if (!small && (st != CEL_OK || dst != src.data || src.parts == 0)) return fail("no second route");
+            g_known_type = cudaMemoryTypeDevice;       // never written by the host
+            if (src.read(rb, dst.data(), own, err) == CEL_OK) return fail("the host wrote into device memory");
         } else {
             return fail("unknown rule");
         }
