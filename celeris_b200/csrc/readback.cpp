@@ -125,6 +125,7 @@ int Readback::read(void* dst, size_t bytes, cudaStream_t s, const std::function<
     // starting a thread takes as long as copying a few hundred kB
     int workers = int(std::min<size_t>(READBACK_WORKERS, bytes / READBACK_SHARE));
     workers = std::max(1, std::min(workers, int(std::thread::hardware_concurrency())));
+    if (s == cudaStreamPerThread) workers = 1;   // in a helper thread this name is another stream, which waits for nothing
     cudaError_t first = cudaSuccess;
     for (int k = 0; k < READBACK_SLOTS && first == cudaSuccess; ++k)
         if (!ev_[k]) first = cudaEventCreateWithFlags(&ev_[k], cudaEventDisableTiming);

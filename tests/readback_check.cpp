@@ -144,6 +144,10 @@ int main(int argc, char** argv) {
             if (!small && (st != CEL_OK || dst != src.data || src.parts == 0)) return fail("no second route");
             g_known_type = cudaMemoryTypeDevice;       // never written by the host
             if (src.read(rb, dst.data(), own, err) == CEL_OK) return fail("the host wrote into device memory");
+        } else if (rule == "thread") {   // the per-thread stream is the calling thread's: no other may use it
+            Readback rb;
+            if (src.read(rb, dst.data(), cudaStreamPerThread, err) != CEL_OK || dst != src.data) return fail("wrong bytes");
+            if (src.threads != std::set<std::thread::id>{std::this_thread::get_id()}) return fail("another thread's stream");
         } else {
             return fail("unknown rule");
         }

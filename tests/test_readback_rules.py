@@ -18,6 +18,6 @@ def check(tmp_path_factory):
     return lambda rule: subprocess.run([exe, rule], capture_output=True, text=True, check=True, timeout=120).stdout.strip()
 
 
-@pytest.mark.parametrize("rule", ["slots", "refused", "device", "pinned"])
+@pytest.mark.parametrize("rule", ["slots", "refused", "device", "pinned", "thread"])
 def test_read_rule(check, rule):
     assert check(rule) == "ok"
