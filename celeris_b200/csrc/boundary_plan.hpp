@@ -36,6 +36,28 @@ inline CornerCut corner_cut(int corner, const int type[4]) {
     return type[yside] != CEL_BC_SOLID ? CUT_ROWS : type[xside] != CEL_BC_SOLID ? CUT_COLUMNS : CUT_NONE;
 }
 
+// put(Rect): the corner r cut into pieces of at most `cells` texels (or one row or column of a wall's corner), each
+// of which takes the two sides by itself.  Where neither side is a wall every texel stands alone, and the
+// corner is cut both ways: in whole rows, a wave-maker along a sponge of 2000 cells left two rows to two CTAs
+// (compensated form, 64 waves, 8192 x 64 cells: 778 us a step, 4000 cells 1413; cut both ways 188 and 222).
+template <class F>
+inline void corner_pieces(int corner, const int type[4], const Rect& r, int cells, F&& put) {
+    if (r.x1 <= r.x0 || r.y1 <= r.y0) return;
+    const int a = corner_side(corner, 0), b = corner_side(corner, 1);
+    const CornerCut cut = corner_cut(corner, type);
+    int w = r.x1 - r.x0, h = r.y1 - r.y0;
+    if (type[a] != CEL_BC_SOLID && type[b] != CEL_BC_SOLID) {
+        w = std::min(w, cells);
+        h = std::min(h, std::max(1, cells / w));
+    } else if (cut == CUT_ROWS) {
+        h = std::min(h, std::max(1, cells / w));
+    } else if (cut == CUT_COLUMNS) {
+        w = std::min(w, std::max(1, cells / h));
+    }
+    for (int y = r.y0; y < r.y1; y += h)
+        for (int x = r.x0; x < r.x1; x += w) put(Rect{x, y, std::min(x + w, r.x1), std::min(y + h, r.y1)});
+}
+
 // Fills the eight rectangles (empty ones have no texels); false where the sides have to be launched
 // one after another: walls wide enough to read their own strip (W, S from 3, E, N from 4 cells), or
 // a domain so small that opposite corners meet.

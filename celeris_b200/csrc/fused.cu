@@ -2510,6 +2510,9 @@ __device__ __forceinline__ void boundary_item(const MemberDev& M, int side, int 
     }
 }
 
+// x and y (below 65536: domains have at most 32768 cells a side) in one word of a work item
+inline int pack_xy(int x, int y) { return int(unsigned(x) | unsigned(y) << 16); }
+
 // A side's strip, clamped to the texture
 __device__ __forceinline__ Rect side_strip(const MemberDev& M, int side) {
     const int NX = M.c.NX, NY = M.c.NY, w = M.bd[side].width;
@@ -2531,10 +2534,10 @@ __global__ void __launch_bounds__(BND_T, 4) k_boundary(const MemberDev* __restri
     }
 }
 
-// All four sides of every member in one launch.  Item: {member, region, first, rows}: a segment's cells
-// from `first` on, or of a corner the rows (rows > 0) or columns (rows < 0) from `first` on, whose two sides
-// the CTA takes in drawing order (a wave-maker's corner texels cost most: uncut, 80 of them in one CTA of
-// the 2048 x 2048 coast took 40 us, as long as four launches).  Four launches of a few thousand threads
+// All four sides of every member in one launch.  Item: {member, region, first}: a segment's cells from
+// `first` on; or {member, region, position, extent}: a piece of a corner (pack_xy), whose two sides the CTA
+// takes in drawing order (a wave-maker's corner texels cost most: uncut, 80 of them in one CTA of the
+// 2048 x 2048 coast took 40 us, as long as four launches).  Four launches of a few thousand threads
 // each were bound by launch latency, 2.4 us a graph node on 512 x 64 cells: us per step there 57.4 ->
 // 43.3, harbour 1017 x 643 (3 passes) 243 -> 182, 1024 x 1024 176 -> 156, 2048 x 2048 490 -> 461.
 template <bool MIXED>
@@ -2545,8 +2548,10 @@ __global__ void __launch_bounds__(BND_T, 5) k_boundary_all(const MemberDev* __re
         const MemberDev& M = mems[wi.x];
         Rect r = M.breg[wi.y];
         const bool corner = wi.y >= 4;
-        if (corner && wi.w > 0) { r.y0 = wi.z; r.y1 = min(r.y1, wi.z + wi.w); }
-        if (corner && wi.w < 0) { r.x0 = wi.z; r.x1 = min(r.x1, wi.z - wi.w); }
+        if (corner) {
+            const int x = wi.z & 0xffff, y = int(unsigned(wi.z) >> 16);
+            r = Rect{x, y, x + (wi.w & 0xffff), y + int(unsigned(wi.w) >> 16)};
+        }
         for (int q = 0; q < (corner ? 2 : 1); ++q) {
             const int side = corner ? corner_side(wi.y - 4, q) : wi.y;
             const Rect s = side_strip(M, side);
@@ -3648,19 +3653,12 @@ cel_lane* lane_create(int n, const cel_params* const* params, const float* const
             for (int k = BND_REGIONS - 1; k >= 0; --k) {   // corners first: they take longest
                 const int n = std::max(0, d.breg[k].x1 - d.breg[k].x0) * std::max(0, d.breg[k].y1 - d.breg[k].y0);
                 if (k >= 4) {
-                    if (n <= 0) continue;
                     // pieces of about one item of the costlier side
                     const int cells = std::min({boundary_item_cells(btype[corner_side(k - 4, 0)]),
                                                 boundary_item_cells(btype[corner_side(k - 4, 1)]), BND_T});
-                    const Rect& r = d.breg[k];
-                    const CornerCut cut = corner_cut(k - 4, btype);
-                    const int across = cut == CUT_ROWS ? r.x1 - r.x0 : r.y1 - r.y0, len = std::max(1, cells / across);
-                    if (cut == CUT_ROWS)
-                        for (int y = r.y0; y < r.y1; y += len) corners.push_back(make_int4(i, k, y, len));
-                    else if (cut == CUT_COLUMNS)
-                        for (int x = r.x0; x < r.x1; x += len) corners.push_back(make_int4(i, k, x, -len));
-                    else
-                        corners.push_back(make_int4(i, k, 0, 0));
+                    corner_pieces(k - 4, btype, d.breg[k], cells, [&](const Rect& q) {
+                        corners.push_back(make_int4(i, k, pack_xy(q.x0, q.y0), pack_xy(q.x1 - q.x0, q.y1 - q.y0)));
+                    });
                 } else {
                     for (int c0 = 0; c0 < n; c0 += boundary_item_cells(btype[k])) ball.push_back(make_int4(i, k, c0, 0));
                 }
