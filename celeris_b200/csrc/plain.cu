@@ -280,6 +280,8 @@ constexpr int CR_MAX_LEVELS = 16;
 constexpr int CR_THREADS = 256;
 constexpr int CR_COLS = 4;              // columns of a column CTA: 64-byte pieces of a state row
 constexpr size_t CR_SMEM_MAX = 200 * 1024;
+constexpr int CR_TALL_THREADS = 1024;
+constexpr int CR_TALL_COLS = 296, CR_TALL_ROWS = 4096;   // domains whose columns k_cr_tall takes
 struct CrLevels {
     int K;                              // levels
     int tail;                           // first level (>= 1) that one warp handles
@@ -294,16 +296,17 @@ struct CrLevels {
 struct SolveArgs {
     float4* st;
     CrLevels x, y;
+    int bands;                          // column CTAs of k_cr
     float* scratch;                     // the levels in global memory where shared memory does not hold them
 };
 
-// ROW: one row (level 0 kept with the levels); else CR_COLS columns.  lv: the levels, element i of
+// ROW: one row (level 0 kept with the levels, W = 1); else W columns.  lv: the levels, element i of
 // column c of level k at lv[(off_k + i) * W + c]; st0: the level-0 values in the state, d0 floats apart;
 // sys: the row, or this thread's column; ns: the number of columns (the columns' coefficient stride).
-template <bool ROW>
+template <bool ROW, int W, int THREADS>
 __device__ __forceinline__ void cr_solve(const CrLevels& L, float* __restrict__ lv, float* st0, size_t d0, int sys, int ns,
                                          bool live) {
-    constexpr int W = ROW ? 1 : CR_COLS, T = CR_THREADS / W;
+    constexpr int T = THREADS / W;
     const int c = int(threadIdx.x) % W, t = int(threadIdx.x) / W;
     const int n = L.len[0];
     lv += c;
@@ -408,17 +411,32 @@ template <bool SMEM_X, bool SMEM_Y>
 __global__ void __launch_bounds__(CR_THREADS) k_cr(SolveArgs a, SimConsts c) {
     extern __shared__ float cr_sm[];
     // columns first: a column CTA has four systems and the strided reads
-    const int rows = c.ny, bands = (c.nx + CR_COLS - 1) / CR_COLS, b = int(blockIdx.x) - bands;
+    const int rows = c.ny, bands = a.bands, b = int(blockIdx.x) - bands;
     if (b >= 0) {
         float* lv = SMEM_X ? cr_sm : a.scratch + size_t(b) * a.x.total;
-        cr_solve<true>(a.x, lv, reinterpret_cast<float*>(a.st + size_t(b + 2) * c.NX + 2) + 1, 4, b, 0, true);
+        cr_solve<true, 1, CR_THREADS>(a.x, lv, reinterpret_cast<float*>(a.st + size_t(b + 2) * c.NX + 2) + 1, 4, b, 0, true);
     } else {
         const int band = blockIdx.x, col = band * CR_COLS + int(threadIdx.x) % CR_COLS;
         float* lv = SMEM_Y ? cr_sm
                            : a.scratch + (SMEM_X ? 0 : size_t(rows) * a.x.total) + size_t(band) * a.y.total * CR_COLS;
-        cr_solve<false>(a.y, lv, reinterpret_cast<float*>(a.st + size_t(2) * c.NX + 2 + col) + 2, size_t(4) * c.NX, col, c.nx,
+        cr_solve<false, CR_COLS, CR_THREADS>(a.y, lv, reinterpret_cast<float*>(a.st + size_t(2) * c.NX + 2 + col) + 2, size_t(4) * c.NX, col, c.nx,
                         col < c.nx);
     }
+}
+
+// Few tall columns: a CTA of 1024 threads per column, in a launch of its own before the rows'.  What bounds
+// tall columns is the serial sweep of a level by the 64 threads that a column has in k_cr, and beside it the
+// rows' CTAs, one or two an SM, since a launch's CTAs all take the shared memory that four columns' levels
+// need.  Level 0 comes 4 bytes a 32-byte sector, so columns that fill the GPU are better off in fours.
+// Event times of the solves, k_cr -> both launches: 8 x 4096 cells 69 -> 45 us, 64 x 8192 509 -> 141, 148 x
+// 12000 937 -> 244, 8 x 32768 636 -> 269, 296 x 4096 154 -> 130; below 4096 rows it is the other way: 64 x 1000
+// 31 -> 35.  (A launch per level and direction took longer than k_cr except on such columns: 2 x 32768 cells
+// 697 us a step, 1391 in k_cr, 569 here.)
+__global__ void __launch_bounds__(CR_TALL_THREADS) k_cr_tall(SolveArgs a, SimConsts c) {
+    extern __shared__ float cr_sm[];
+    const int col = blockIdx.x;
+    cr_solve<false, 1, CR_TALL_THREADS>(a.y, cr_sm, reinterpret_cast<float*>(a.st + size_t(2) * c.NX + 2 + col) + 2,
+                                        size_t(4) * c.NX, col, c.nx, true);
 }
 
 // ---- Boundaries (compute.hlsl:985-1309) --------------------------------------------------
@@ -709,7 +727,8 @@ public:
     float4 *ACBx = nullptr, *ACBy = nullptr;                        // substitution coefficients of every level
     SolveArgs solve{};
     bool smem_x = true, smem_y = true;
-    size_t smem_cr = 0;
+    size_t smem_cr = 0, smem_tall = 0;
+    bool tall = false;                                              // k_cr_tall takes the columns
     bool planned = false;                                           // the four sides run as one launch
     Rect regions[BND_REGIONS] = {};
     int2* bitems = nullptr;
@@ -839,7 +858,9 @@ public:
 
     // Level tables of the cyclic reduction and, once, the room for them.
     int init_solve() {
-        auto levels = [](const std::vector<int>& len, bool rows, int systems) {
+        tall = hs.nx <= CR_TALL_COLS && hs.ny >= CR_TALL_ROWS;
+        const int cols = tall ? 1 : CR_COLS;
+        auto levels = [&](const std::vector<int>& len, bool rows, int systems) {
             CrLevels L{};
             L.K = int(len.size());
             L.tail = L.K;
@@ -852,7 +873,7 @@ public:
                 L.soff[k] = so;
                 if (k > 0) ko += size_t(len[k]) * systems;
                 so += size_t((len[k] + 1) / 2) * systems;
-                if (k > 0 && L.tail == L.K && len[k] * (rows ? 1 : CR_COLS) <= 32) L.tail = k;
+                if (k > 0 && L.tail == L.K && len[k] * (rows ? 1 : cols) <= 32) L.tail = k;
             }
             return std::make_pair(L, std::make_pair(ko, so));
         };
@@ -865,16 +886,18 @@ public:
         if (int e = dalloc(ACBy, ly.second.second)) return e;
         solve.x.k12 = K12x; solve.x.acb = ACBx;
         solve.y.k12 = K12y; solve.y.acb = ACBy;
-        const size_t bx = sizeof(float) * size_t(solve.x.total), by = sizeof(float) * size_t(solve.y.total) * CR_COLS;
+        const size_t bx = sizeof(float) * size_t(solve.x.total), by = sizeof(float) * size_t(solve.y.total) * cols;
         smem_x = bx <= CR_SMEM_MAX;
         smem_y = by <= CR_SMEM_MAX;
-        smem_cr = std::max(smem_x ? bx : 0, smem_y ? by : 0);
+        smem_tall = tall ? by : 0;
+        smem_cr = std::max(smem_x ? bx : 0, smem_y && !tall ? by : 0);
+        solve.bands = tall ? 0 : (hs.nx + CR_COLS - 1) / CR_COLS;
         const size_t scratch = (smem_x ? 0 : size_t(hs.ny) * solve.x.total) +
-                               (smem_y ? 0 : size_t((hs.nx + CR_COLS - 1) / CR_COLS) * CR_COLS * solve.y.total);
+                               (smem_y ? 0 : size_t(solve.bands) * CR_COLS * solve.y.total);
         if (scratch)
             if (int e = dalloc(solve.scratch, scratch)) return e;
         // the limit is the function's, not this engine's: set once to the most any engine asks for
-        for (auto* k : {k_cr<true, true>, k_cr<true, false>, k_cr<false, true>, k_cr<false, false>})
+        for (auto* k : {k_cr<true, true>, k_cr<true, false>, k_cr<false, true>, k_cr<false, false>, k_cr_tall})
             CEL_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(CR_SMEM_MAX)));
         // the allocations' clears ran on the legacy stream, which the engine's stream does not wait for
         CEL_CUDA_TRY(cudaDeviceSynchronize());
@@ -1123,7 +1146,8 @@ public:
             TimedLaunch tl(&tm, stream, "plain_cr");
             auto* k = smem_x ? (smem_y ? k_cr<true, true> : k_cr<true, false>) : (smem_y ? k_cr<false, true> : k_cr<false, false>);
             solve.st = new_state;
-            k<<<hs.ny + (hs.nx + CR_COLS - 1) / CR_COLS, CR_THREADS, smem_cr, stream>>>(solve, c);
+            if (tall) k_cr_tall<<<hs.nx, CR_TALL_THREADS, smem_tall, stream>>>(solve, c);
+            k<<<hs.ny + solve.bands, CR_THREADS, smem_cr, stream>>>(solve, c);
         }
         boundaries(new_state);
         CEL_CUDA_TRY(cudaGetLastError());
