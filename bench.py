@@ -500,7 +500,7 @@ def main():
                            cells * 4 * (46 + (9 if args.form == "mixed" else 0)) / 1e9),
                        "parallelism": f"ensemble sharded by domain over {world} GPU(s)",
                        "lanes": lanes,
-                       "tuning": {"column_band_width": batch.tuning[0], "strip_height": batch.tuning[1],
+                       "tuning": {"column_band_width": batch.tuning[0], "strip_height": batch.strip_height,
                                   "stencil_rows_per_step": batch.stencil_rows,
                                   "stencil_threads_per_strip": batch.stencil_width,
                                   "autotuned": tuned is not None,

@@ -249,7 +249,7 @@ class Batch:
 
     def set_tuning(self, band_width: int = 0, strip_height: int = 0, chunks: int = 0):
         """Column-solver band width (1/8/16/32), stencil strip height and the column solver's chunks
-        per column (0 keeps the current value)."""
+        per column (0 keeps the current value; the height is chosen by the batch's size until one is given)."""
         check(lib().cel_batch_set_tuning(self.h, band_width, strip_height, chunks))
 
     @property
@@ -259,7 +259,7 @@ class Batch:
 
     @property
     def tuning(self) -> tuple:
-        """(column band width, strip height)."""
+        """(column band width, selected strip height: 64 while the batch's size chooses it)."""
         tx, ty, rp = C.c_int(), C.c_int(), C.c_int()
         check(lib().cel_batch_get_tuning(self.h, C.byref(tx), C.byref(ty), C.byref(rp)))
         return tx.value, ty.value
@@ -277,6 +277,11 @@ class Batch:
     @property
     def stencil_width(self) -> int:
         return int(lib().cel_batch_stencil_width(self.h))
+
+    @property
+    def strip_height(self) -> int:
+        """Rows of the tallest stencil strip that runs."""
+        return int(lib().cel_batch_strip_height(self.h))
 
     def set_stencil_width(self, threads: int):
         """Threads per stencil CTA (128 or 96; 96 with two rows per step)."""

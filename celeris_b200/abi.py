@@ -194,6 +194,7 @@ def _declare(L: C.CDLL) -> None:
         "cel_batch_set_stencil_rows": (i, [vp, i]),
         "cel_batch_set_stencil_width": (i, [vp, i]),
         "cel_batch_stencil_width": (i, [vp]),
+        "cel_batch_strip_height": (i, [vp]),
         "cel_batch_autotune": (i, [vp, i, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_double)]),
         "cel_batch_get_state": (i, [vp, i, fp]),
         "cel_batch_get_state_parts": (i, [vp, i, fp, fp]),
@@ -244,6 +245,6 @@ EXPORTED = [
     "cel_batch_stats", "cel_batch_stats_current", "cel_batch_get_state", "cel_batch_get_state_parts", "cel_batch_set_state", "cel_batch_get_aux",
     "cel_batch_use_graph", "cel_batch_cells", "cel_batch_set_timestep", "cel_batch_launches_per_step", "cel_set_tuning", "cel_batch_set_tuning",
     "cel_batch_get_tuning", "cel_batch_col_chunks", "cel_batch_set_stencil_rows", "cel_batch_set_stencil_width", "cel_batch_stencil_width",
-    "cel_batch_autotune",
+    "cel_batch_strip_height", "cel_batch_autotune",
     "cel_batch_kernel_timing", "cel_engine_kernel_timing", "cel_kernel_times", "cel_byte_model", "cel_selftest_reciprocal", "cel_stats_noalloc",
 ]

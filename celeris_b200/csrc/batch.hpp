@@ -52,6 +52,8 @@ int lane_get_tuning(const cel_lane* b, int* tx, int* ty, int* rps);
 int lane_set_stencil_rows(cel_lane* b, int rps, std::string& err);
 int lane_set_stencil_width(cel_lane* b, int threads, std::string& err);
 int lane_stencil_width(const cel_lane* b);
+int lane_strip_height(const cel_lane* b);   // rows of the tallest stencil strip that runs
+int lane_split_height(const cel_lane* b, int rps, int mw);   // ... that the split rule takes for this variant
 // column band width, strip height, stencil rows per step, stencil width, column solver threads in one call
 int lane_configure(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::string& err);
 int lane_col_threads(const cel_lane* b);
@@ -86,6 +88,7 @@ int batch_col_chunks(const cel_batch* b);
 int batch_set_stencil_rows(cel_batch* b, int rps, std::string& err);
 int batch_set_stencil_width(cel_batch* b, int threads, std::string& err);
 int batch_stencil_width(const cel_batch* b);
+int batch_strip_height(const cel_batch* b);
 int batch_autotune(cel_batch* b, int steps, int* tx, int* ty, double* best_ms, std::string& err);
 void batch_kernel_timing(cel_batch* b, bool enable);
 // per-kernel totals summed over the lanes (synchronizes the pending timer events)

@@ -411,6 +411,7 @@ int cel_batch_set_stencil_width(cel_batch* b, int threads) {
     CEL_GUARD_BEGIN BRET(cel::batch_set_stencil_width(b, threads, err)); CEL_GUARD_END
 }
 int cel_batch_stencil_width(const cel_batch* b) { return b ? cel::batch_stencil_width(b) : 0; }
+int cel_batch_strip_height(const cel_batch* b) { return b ? cel::batch_strip_height(b) : 0; }
 int cel_batch_set_stencil_rows(cel_batch* b, int rows_per_step) {
     BAT(b);
     CEL_GUARD_BEGIN BRET(cel::batch_set_stencil_rows(b, rows_per_step, err)); CEL_GUARD_END

@@ -182,7 +182,7 @@ __device__ void stats_reduce(double* acc, bool cnt_block, bool cnt_all, float h,
 constexpr int MARCH_MIN_CTAS = CEL_MARCH_MIN_CTAS;
 constexpr int MW = 128;          // threads = columns with faces per row
 constexpr int MO = MW - 2;       // output columns per strip
-constexpr int MH_DEFAULT = 64;   // rows per strip unless tuned (each work item carries its height)
+constexpr int MH_DEFAULT = 64;   // the most rows of a strip whose height strip_split chooses
 constexpr int RING = 7;          // state / bottom rows resident in shared memory (PREFETCH + 5)
 constexpr int RBOX = 136;        // TMA box width in floats (covers columns x0-2 .. x0+127)
 constexpr int RSTR = 160;        // ring row stride in floats (640 B, a multiple of 128 B)
@@ -2850,7 +2850,9 @@ struct cel_lane {
     int cnt = 512;                      // column solver threads per CTA (chunks per column = cnt / cw)
     int col_cl = 0;                     // cluster column solver: CTAs per cluster (0: not in use)
     bool col_tt = false;                // tile-transposed column solver (band width 16, "1 chunk")
-    int mh = cel::MH_DEFAULT;           // stencil strip height (rows per CTA work item)
+    int mh = cel::MH_DEFAULT;           // the selected stencil strip height (rows per CTA work item)
+    bool mh_auto = true;                // ... by strip_split, until it is selected (mh is MH_DEFAULT then)
+    int strip = 0;                      // rows of the tallest strip that runs
     int rows_per_step = 2;              // stencil rows per thread step: 1 (k_march) or 2 (k_march2)
     int mw = 128;                       // stencil CTA width in threads (k_march2: 128 or 96)
     bool mw_auto = true;                // ... by strip_split, until it is selected
@@ -3248,8 +3250,8 @@ cudaError_t allow_max_dynamic_smem(const void* kernel) {
     return e;
 }
 
-// The split of a batch's stencil: a strip height of at most mh_max rows, lower where taller strips would
-// leave SMs idle, and, with mw 0, the strip width (128 or 96 threads).  A strip is a serial chain of row
+// The split of a batch's stencil: with mh 0 a strip height of at most MH_DEFAULT rows, lower where taller
+// strips would leave SMs idle, and with mw 0 the strip width (128 or 96 threads).  A strip is a serial chain of row
 // steps, so a batch with fewer strips than CTA slots takes as long as one strip, and one with a few
 // strips more than a whole number of waves takes a wave more.  The cost of a split is modelled as
 //   sum over waves of (row steps of a strip + PRO) x step(CTAs per SM in that wave),
@@ -3262,17 +3264,18 @@ cudaError_t allow_max_dynamic_smem(const void* kernel) {
 // threads), 40 members of 128..512 a side 517 -> 475 (40); 16 M cells keep 64 rows (128 threads 1338,
 // 96 1346; 32 rows 1368).  Splits change no cell's arithmetic; every lane takes the split of the whole
 // batch, so the statistics do not depend on the lanes either.
-int strip_split(const cel_lane* b, int rps, int& mw, int mh_max) {
+int strip_split(const cel_lane* b, int rps, int& mw, int mh) {
     constexpr int H_MIN = 4;
     constexpr double PRO = 2.5;
-    int best = mh_max, best_w = mw ? mw : MW;
+    const int h_min = mh ? mh : H_MIN, h_max = mh ? mh : MH_DEFAULT;
+    int best = h_max, best_w = mw ? mw : MW;
     double best_t = 1e300;
     for (int w : {128, 96}) {
         if (mw && w != mw) continue;
         const int mo = w - 2, slots = rps == 1 ? MARCH_MIN_CTAS : march2_min_ctas(w);
         const double base_us = rps == 1 ? 0.9 : 1.0, rate_us = rps == 1 ? 0.54 : w == 128 ? 0.8 : 0.64;
         auto step = [&](double n) { return n > 0 ? base_us + n * rate_us : 0.0; };
-        for (int h = std::min(H_MIN, mh_max);; h = std::min(h + 2, mh_max)) {
+        for (int h = h_min;; h = std::min(h + 2, h_max)) {
             long long strips = 0;
             for (const auto& m : b->batch_sizes) strips += (long long)((m.first + mo - 1) / mo) * ((m.second + h - 1) / h);
             const double per_sm = std::ceil(strips / double(b->sms)), whole = std::floor(per_sm / slots);
@@ -3282,14 +3285,14 @@ int strip_split(const cel_lane* b, int rps, int& mw, int mh_max) {
                 best = h;
                 best_w = w;
             }
-            if (h == mh_max) break;
+            if (h == h_max) break;
         }
     }
     mw = best_w;
     return best;
 }
 
-// mw 0: the stencil width by strip_split.
+// mh 0, mw 0: the strip height, the stencil width by strip_split.
 int configure_work(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::string& err) {
     // 32-column bands with 32, 64 or 128 chunks per column (nt = chunks x 32 = 1024, 2048, 4096):
     // the cluster solver, 8 chunks per CTA and nt / 256 CTAs per cluster
@@ -3329,18 +3332,21 @@ int configure_work(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::st
     if (rps == 1) mw = MW;   // the one-row stencil has one width
     b->rows_per_step = rps;
     if (cw != 1 && cw != 8 && cw != 16 && cw != 32) { err = "column band width must be 1, 8, 16 or 32"; return CEL_ERR_ARG; }
-    if (mh < 8 || mh > 1024) { err = "strip height must be in [8, 1024]"; return CEL_ERR_ARG; }
+    if (mh != 0 && (mh < 8 || mh > 1024)) { err = "strip height must be in [8, 1024]"; return CEL_ERR_ARG; }
     const size_t smem_cols = tt ? sizeof(float) * size_t(TT_CW) * size_t((b->max_ny + 3) & ~3)
                              : (cw == 1 || cl > 0) ? 0 : sizeof(float) * size_t(b->max_ny) * cw;
     if (smem_cols + COLS_STATIC_SMEM > 227 * 1024) { err = "column band too wide for the tallest member (shared memory)"; return CEL_ERR_ARG; }
     std::vector<int4> mt;
     std::vector<int2> bd, mr;
-    const bool mw_auto = mw == 0;
+    const bool mw_auto = mw == 0, mh_auto = mh == 0;
     const int sh = strip_split(b, rps, mw, mh), mo = mw - 2;   // strip height, output columns per strip
+    int strip = 0;
     for (int i = 0; i < int(b->mem.size()); ++i) {
         const HostSetup& hs = b->mem[i].hs;
-        // a member's strips as equal as whole steps allow
-        const int nb = (hs.ny + sh - 1) / sh, hm = std::min(sh, ((hs.ny + nb - 1) / nb + rps - 1) / rps * rps);
+        // unless their height is selected, a member's strips are as equal as whole steps allow
+        const int nb = (hs.ny + sh - 1) / sh;
+        const int hm = mh_auto ? std::min(sh, ((hs.ny + nb - 1) / nb + rps - 1) / rps * rps) : sh;
+        strip = std::max(strip, hm);
         const int first = int(mt.size());
         for (int y0 = 2; y0 < hs.ny + 2; y0 += hm)
             for (int x0 = 2; x0 < hs.nx + 2; x0 += mo) mt.push_back(make_int4(i, x0, y0, hm));
@@ -3385,7 +3391,9 @@ int configure_work(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::st
     b->nbands = int(bd.size());
     b->cw = cw;
     b->cnt = nt;
-    b->mh = mh;
+    b->mh = mh_auto ? MH_DEFAULT : mh;
+    b->mh_auto = mh_auto;
+    b->strip = strip;
     b->mw = mw;
     b->mw_auto = mw_auto;
     b->smem_cols = smem_cols;
@@ -3737,9 +3745,9 @@ cel_lane* lane_create(int n, const cel_params* const* params, const float* const
         const int wpc = b->rows_threads / 32;
         b->grid_rows = std::max(1, std::min((b->nrows + wpc - 1) / wpc, b->sms * std::max(occ, 1)));
     }
-    {   // column bands of 16 columns (8 for tall domains: shared-memory capacity), strips of 64 rows
+    {   // column bands of 16 columns (8 for tall domains: shared-memory capacity), strips by strip_split
         const int cw = (size_t(max_ny) * 16 * sizeof(float) + COLS_STATIC_SMEM <= 227 * 1024) ? 16 : 8;
-        if (configure_work(b.get(), cw, MH_DEFAULT, b->rows_per_step, 0, NTC_DEFAULT, err)) return nullptr;
+        if (configure_work(b.get(), cw, 0, b->rows_per_step, 0, NTC_DEFAULT, err)) return nullptr;
     }
     b->sch.reset(*params[0]);
     cudaMemcpy(b->dt_table, b->dt_host, sizeof(float) * n, cudaMemcpyHostToDevice);
@@ -4049,7 +4057,7 @@ int lane_set_tuning(cel_lane* b, int tx, int ty, int pcr, std::string& err) {
     // swept serially), so the CTA has pcr x band width threads; 0 keeps the threads per CTA
     const int cw = tx > 0 ? tx : b->cw;
     const int nt = (pcr > 0 && cw > 1) ? pcr * cw : b->cnt;
-    return configure_work(b, cw, ty > 0 ? ty : b->mh, b->rows_per_step, b->mw_auto ? 0 : b->mw, nt, err);
+    return configure_work(b, cw, ty > 0 ? ty : b->mh_auto ? 0 : b->mh, b->rows_per_step, b->mw_auto ? 0 : b->mw, nt, err);
 }
 
 int lane_get_tuning(const cel_lane* b, int* tx, int* ty, int* rps) {
@@ -4063,7 +4071,7 @@ int lane_col_chunks(const cel_lane* b) { return b->cw > 1 ? b->cnt / b->cw : 1; 
 
 int lane_set_stencil_rows(cel_lane* b, int rps, std::string& err) {
     // two rows per step start from 128-thread strips until a width is chosen (lane_set_stencil_width)
-    if (int e = configure_work(b, b->cw, b->mh, rps, rps == 2 && b->rows_chosen ? b->mw : MW, b->cnt, err)) return e;
+    if (int e = configure_work(b, b->cw, b->mh_auto ? 0 : b->mh, rps, rps == 2 && b->rows_chosen ? b->mw : MW, b->cnt, err)) return e;
     b->rows_chosen = true;
     return CEL_OK;
 }
@@ -4073,10 +4081,12 @@ int lane_set_stencil_width(cel_lane* b, int threads, std::string& err) {
         err = "the one-row stencil runs 128-thread strips; select two rows per step first";
         return CEL_ERR_ARG;
     }
-    return configure_work(b, b->cw, b->mh, b->rows_per_step, threads, b->cnt, err);
+    return configure_work(b, b->cw, b->mh_auto ? 0 : b->mh, b->rows_per_step, threads, b->cnt, err);
 }
 
 int lane_stencil_width(const cel_lane* b) { return b->mw; }
+int lane_strip_height(const cel_lane* b) { return b->strip; }
+int lane_split_height(const cel_lane* b, int rps, int mw) { return strip_split(b, rps, mw, 0); }
 
 cudaStream_t lane_stream(const cel_lane* b) { return b->stream; }
 int lane_members(const cel_lane* b) { return int(b->mem.size()); }

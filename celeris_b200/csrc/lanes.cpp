@@ -279,10 +279,16 @@ int batch_set_stencil_width(cel_batch* b, int threads, std::string& err) {
 
 int batch_stencil_width(const cel_batch* b) { return lane_stencil_width(b->lanes[0]); }
 
+int batch_strip_height(const cel_batch* b) {
+    int h = 0;
+    for (const cel_lane* l : b->lanes) h = std::max(h, lane_strip_height(l));
+    return h;
+}
+
 // Times `steps` physical steps of the whole batch (all lanes side by side) for each candidate, in
 // the launch mode the batch is set to, two rounds in turn, and keeps the fastest by its better
 // round.  The stencil and the solvers are separate kernels, so the search runs in two stages: the
-// stencil (rows per step and width x strip height) with the default solvers, then the column solver
+// stencil (rows per step and width x strip height, by the split rule or fixed) with the default solvers, then the column solver
 // (band width x chunks per column, i.e. the switch point from the carry scan to serial sweeps, and
 // the cluster solver where the tallest member fits its chunks) with the chosen stencil.  Every lane takes the same candidate and the same steps, so the members stay
 // in step with one another.
@@ -328,7 +334,8 @@ int batch_autotune(cel_batch* b, int steps, int* tx, int* ty, double* best_ms, s
     std::vector<Cand> stencil;
     const int variants[3][2] = {{1, 128}, {2, 128}, {2, 96}};   // stencil rows per step, stencil width
     for (const auto& v : variants)
-        for (int mh : {32, 64, 128}) stencil.push_back({cw0, mh, v[0], v[1], 512});
+        for (int mh : {0, 32, 64, 128})   // (0: by the split rule)
+            if (mh != lane_split_height(b->lanes[0], v[0], v[1])) stencil.push_back({cw0, mh, v[0], v[1], 512});
     double ms = 0.0;
     const int ks = search(stencil, ms);
     std::vector<Cand> solver;
@@ -352,7 +359,7 @@ int batch_autotune(cel_batch* b, int steps, int* tx, int* ty, double* best_ms, s
     if (rc) return rc;
     if ((rc = configure(solver[size_t(kb)]))) return rc;
     if (tx) *tx = solver[size_t(kb)].cw;
-    if (ty) *ty = solver[size_t(kb)].mh;
+    if (ty) batch_get_tuning(b, nullptr, ty, nullptr);
     if (best_ms) *best_ms = ms;
     return CEL_OK;
 }

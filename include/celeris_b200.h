@@ -275,8 +275,8 @@ int cel_batch_launches_per_step(const cel_batch* b);
 /* ---- tuning and measurement ------------------------------------------------------------- */
 /* Fused forms.  tile_x: column-solver band width (8, 16 or 32 columns per CTA, chunked scans; or 1:
  * one thread per column, serial sweeps, forward values kept in the right-hand-side plane); tile_y: stencil
- * strip height (the most rows a CTA marches, 8..1024; strips are split shorter where the batch has too few
- * of them to fill the GPU); 0 keeps the current value.  pcr_switch: chunks per
+ * strip height (rows a CTA marches, 8..1024; until one is selected, at most 64 and fewer where the batch has
+ * too few strips to fill the GPU, and cel_batch_get_tuning gives 64); 0 keeps the current value.  pcr_switch: chunks per
  * column of the column solver, i.e. where it switches from the parallel stage to serial sweeps.  The
  * solves factor each system once (M = LU, engine.cpp:2612-2887 coefficients); the L and U sweeps of
  * a column are split into that many chunks, each swept serially by one thread (Thomas), and the
@@ -299,9 +299,12 @@ int cel_batch_set_stencil_rows(cel_batch* b, int rows_per_step);
  * only).  Narrower strips waste fewer lanes on members whose width is not a multiple of 126. */
 int cel_batch_set_stencil_width(cel_batch* b, int threads);
 int cel_batch_stencil_width(const cel_batch* b);
+/* Rows of the tallest stencil strip that runs: the selected height, or the one that the batch's size chose. */
+int cel_batch_strip_height(const cel_batch* b);
 /* Times `steps` physical steps for each candidate (band width x strip height x stencil rows per
- * step x stencil width) and keeps the fastest; writes the choice and its ms per step.  The
- * members advance by every timed step. */
+ * step x stencil width) and keeps the fastest; writes the choice, as cel_batch_get_tuning gives it, and its
+ * ms per step.  The heights tried are 32, 64, 128 and the one chosen by the batch's size, which then stays
+ * chosen so.  The members advance by every timed step. */
 int cel_batch_autotune(cel_batch* b, int steps, int* tile_x, int* tile_y, double* ms_per_step);
 /* Per-kernel CUDA-event timing on the launching stream (off by default). */
 int cel_batch_kernel_timing(cel_batch* b, int enable);
