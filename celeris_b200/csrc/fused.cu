@@ -2856,7 +2856,6 @@ struct cel_lane {
     int rows_per_step = 2;              // stencil rows per thread step: 1 (k_march) or 2 (k_march2)
     int mw = 128;                       // stencil CTA width in threads (k_march2: 128 or 96)
     bool mw_auto = true;                // ... by strip_split, until it is selected
-    bool rows_chosen = false;           // the caller selected the stencil variant (lane_set_stencil_rows)
     std::vector<std::pair<int, int>> batch_sizes;   // (nx, ny) of every member of the batch, all lanes
     int max_nx = 0, max_ny = 0;
     bool any_log = false;               // some member has <logData> doLog set
@@ -4070,14 +4069,13 @@ int lane_get_tuning(const cel_lane* b, int* tx, int* ty, int* rps) {
 int lane_col_chunks(const cel_lane* b) { return b->cw > 1 ? b->cnt / b->cw : 1; }
 
 int lane_set_stencil_rows(cel_lane* b, int rps, std::string& err) {
-    // two rows per step start from 128-thread strips until a width is chosen (lane_set_stencil_width)
-    if (int e = configure_work(b, b->cw, b->mh_auto ? 0 : b->mh, rps, rps == 2 && b->rows_chosen ? b->mw : MW, b->cnt, err)) return e;
-    b->rows_chosen = true;
-    return CEL_OK;
+    // a selected width stays; else selecting a variant selects 128 threads with it
+    const int mw = rps == 2 && b->rows_per_step == 2 && !b->mw_auto ? b->mw : MW;
+    return configure_work(b, b->cw, b->mh_auto ? 0 : b->mh, rps, mw, b->cnt, err);
 }
 
 int lane_set_stencil_width(cel_lane* b, int threads, std::string& err) {
-    if ((b->rows_per_step != 2 || !b->rows_chosen) && threads != MW) {
+    if (b->rows_per_step != 2 && threads != MW) {
         err = "the one-row stencil runs 128-thread strips; select two rows per step first";
         return CEL_ERR_ARG;
     }
@@ -4092,9 +4090,7 @@ cudaStream_t lane_stream(const cel_lane* b) { return b->stream; }
 int lane_members(const cel_lane* b) { return int(b->mem.size()); }
 int lane_max_ny(const cel_lane* b) { return b->max_ny; }
 int lane_configure(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::string& err) {
-    if (int e = configure_work(b, cw, mh, rps, mw, nt, err)) return e;
-    b->rows_chosen = true;
-    return CEL_OK;
+    return configure_work(b, cw, mh, rps, mw, nt, err);
 }
 int lane_col_threads(const cel_lane* b) { return b->cnt; }
 

@@ -293,7 +293,9 @@ int cel_batch_get_tuning(const cel_batch* b, int* tile_x, int* tile_y, int* rows
 /* The column solver's chunks per column (the pcr_switch above; 1 with tile_x = 1: one thread per column). */
 int cel_batch_col_chunks(const cel_batch* b);
 /* Stencil variant: 1 = one row per thread step; 2 = two rows per step as pairs, with the paired
- * single-precision instructions of sm_100 (f32x2).  Until it is selected, two rows, at 128 or 96 threads by the members' sizes. */
+ * single-precision instructions of sm_100 (f32x2).  A new batch runs two rows, at 128 or 96 threads
+ * by its members' sizes until a variant or a width is selected; selecting a variant selects 128 threads
+ * with it, unless two rows run already at a selected width. */
 int cel_batch_set_stencil_rows(cel_batch* b, int rows_per_step);
 /* Threads per stencil CTA, i.e. strip width + 2 halo columns: 128 or 96 (96 with two rows per step
  * only).  Narrower strips waste fewer lanes on members whose width is not a multiple of 126. */
