@@ -24,7 +24,7 @@ __host__ __device__
 inline int corner_side(int corner, int q) {
     return q == 0 ? (corner == 1 ? 0 : corner == 3 ? 3 : 1) : (corner == 0 ? 0 : corner == 1 ? 3 : 2);
 }
-// A corner is one CTA's work: larger ones (two very wide sponges) are left to one launch per side.
+// The plain form takes a corner in one CTA; with larger ones (two very wide sponges) each side keeps its launch.
 constexpr int BND_CORNER_MAX = 16384;
 
 // How a corner may be cut into pieces that take its two sides independently: a wall reads texels along its

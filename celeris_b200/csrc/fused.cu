@@ -53,7 +53,8 @@ constexpr int TX = 32, TY = 16;
 // 32-column bands and 9.67 with 16, against 10.34 Gcell-steps/s; a CTA's barriers and carry scans
 // then stall the whole SM.
 constexpr int NTC_DEFAULT = 512;
-// column solver CTAs per SM the build targets at 512 threads: 2 (64 registers, no spills); 1 lets
+// column solver CTAs per SM the build targets at 512 threads: 2 (64 registers; four of the twelve instances
+// spill 4 or 8 bytes a thread, the single-precision one of the default band among them); 1 lets
 // the compiler take about 100 registers and run one CTA per SM, 3 spills (measured on C4: 8.9 / 10.3
 // / 9.2 Gcell-steps/s).  256-thread CTAs target twice as many, at the same 64 registers.
 #ifndef CEL_COLS_MIN_CTAS
@@ -756,15 +757,17 @@ __global__ void __launch_bounds__(MW, MARCH_MIN_CTAS) k_march(const MemberDev* _
 // reads it instead of three levels (60): compensated form 112 -> 104 bytes a cell in the predictor,
 // 136 -> 88 in the corrector.  28 members, 16 M cells: 286 -> 253 us a launch on average, ms per step
 // 1.482 -> 1.374.  What the correctors add up is rounded once more than before (the combination, relative
-// 2^-24), as the rates themselves were; the states' distance from 64 bits is unchanged.
+// 2^-24), as the rates themselves were.  The states' distance from 64 bits moves by a few percent either way
+// with the inputs (512 x 64 flume, 200 steps, ten sets: w, hu, hv 0.998, 0.996 and 1.007 of what it was, on average).
 // ---------------------------------------------------------------------------------------------
 // CTAs per SM the paired-row stencil is built for: 4 of 128 threads or 5 of 96 (16 and 15 warps at 128
 // registers).  Its warps wait on each other's arithmetic more than on memory (issue slots were 59 % used
 // with 12 warps of 168 registers an SM, 66 % with 16, tail included), so warps count: 2048 x 2048 cells
 // 165 -> 138 us a launch, 28 members 1374 -> 1338 us a step.  Two changes made room: the statistics add up
 // in FP64 (one register pair a sum instead of two compensated pairs), and a single barrier a step, which
-// lets the warps of a CTA drift through Pass3 of one step and the faces of the next.  With two barriers
-// and compensated sums the same bound spilled 188 bytes a thread and the step took 1418 us.
+// lets the warps of a CTA drift through Pass3 of one step and the faces of the next.  At this bound the
+// predictors' and Euler's instances spill 16 to 48 bytes a thread and the correctors' none; with two barriers
+// and compensated sums it was 188 bytes, and the step took 1418 us.
 constexpr int march2_min_ctas(int w) { return w == 128 ? 4 : 5; }
 constexpr int PRING = 6;
 template <int TW>
@@ -2327,7 +2330,7 @@ __device__ __forceinline__ void sponge_apply_d(double gam, double sl, float& w, 
 
 // A sponge strip is a few loads, an FP64 scaling and the stores a cell; the wave-makers' FP64 functions set
 // the registers.  With CTAs of 256 threads, four cells each, two an SM, the loads in flight bound it.  128
-// threads with two cells each, five CTAs an SM at 96 registers (112 B spilled), took the 2048 x 2048 coast's
+// threads with two cells each, five CTAs an SM at 96 registers (88 B spilled), took the 2048 x 2048 coast's
 // launch from 26.6 to 22.5 us, 40 members' from 20.7 to 16.4, 8 members' of 256 x 256 from 12.1 to 10.0.
 // Six an SM spill 464 B (8 members 95.3 us a step for 94.2), four are too few (coast 24.6 us).
 constexpr int BND_T = 128;
@@ -2768,8 +2771,6 @@ __global__ void __launch_bounds__(ADV_STRIPS * STATS_N) k_advance_time(const Mem
     }
 }
 
-// Final Pass1 aux update of the current state (txAuxiliary2 -> reported txAuxiliary1 values are
-// what the device keeps; this kernel is not needed for them).
 }  // namespace
 
 // ---------------------------------------------------------------------------------------------
@@ -3232,8 +3233,6 @@ void byte_model(int form, int N, double& stencil, double& step) {
     step = (st_pred + tri) + N * (st_corr + tri);
 }
 
-// (Re)builds the stencil strips (height mh) and the column bands (width cw) of a batch, sizes the
-// column solver's shared memory and grids, and drops captured graphs (they hold the old lists).
 // Lets `kernel` take as much dynamic shared memory as the device allows beside its static shared
 // memory.  The limit is an attribute of the function for the whole process, so setting it to one
 // batch's need would refuse the larger launches of another live batch; the launches themselves
@@ -3291,7 +3290,9 @@ int strip_split(const cel_lane* b, int rps, int& mw, int mh) {
     return best;
 }
 
-// mh 0, mw 0: the strip height, the stencil width by strip_split.
+// (Re)builds the stencil strips (height mh, or 0: by strip_split; width mw, or 0: likewise) and the column
+// bands (width cw) of a batch, sizes the column solver's shared memory and grids, and drops captured graphs
+// (they hold the old lists).
 int configure_work(cel_lane* b, int cw, int mh, int rps, int mw, int nt, std::string& err) {
     // 32-column bands with 32, 64 or 128 chunks per column (nt = chunks x 32 = 1024, 2048, 4096):
     // the cluster solver, 8 chunks per CTA and nt / 256 CTAs per cluster

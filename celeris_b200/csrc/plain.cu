@@ -1,6 +1,6 @@
-// Plain FP32 form: one CUDA kernel per reference pass and one per cyclic-reduction level,
-// over float4 "textures" with the reference's ghost layout.  This is the straightforward GPU
-// restatement of timestep()/resetTimestep() (engine.cpp:849-1756) and of the compute.hlsl
+// Plain FP32 form over float4 "textures" with the reference's ghost layout: one kernel for Pass1 to Pass3, one for
+// every level of both directions' cyclic reduction, one for the four boundary sides and one for GetStats.  This is
+// the GPU restatement of timestep()/resetTimestep() (engine.cpp:849-1756) and of the compute.hlsl
 // pixel shaders; it is compiled with -fmad=false so its arithmetic follows the FP32
 // transcription operation by operation.  One domain per launch set.
 #define CEL_EXACT_FP32 1

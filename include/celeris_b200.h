@@ -319,8 +319,10 @@ int cel_kernel_times(void* handle, int is_batch, char (*names)[64], double* tota
  * one Newton-Raphson step), computed on the current device; x and out are host arrays of n floats.
  * It allocates device memory for the call. */
 int cel_selftest_reciprocal(const float* x, float* out, int n);
-/* Algorithmic HBM bytes per cell for one pass of the dominant kernel and for a whole
- * physical step (the roofline byte model recorded in code). */
+/* Algorithmic HBM bytes per cell for a predictor pass of the paired-row stencil and for a whole physical step, of
+ * a step whose every pass keeps its rates.  With correctors the kernels move less: a predictor hands them one
+ * combination of its rates, which saves 8 bytes in its own pass and 48 in each corrector's (mixed form, one
+ * corrector: 320 bytes a step where this gives 376). */
 int cel_byte_model(int form, int correction_steps, double* stencil_bytes_per_cell_pass,
                    double* step_bytes_per_cell);
 
